@@ -11,9 +11,7 @@
 //             forward convolution of the output gradient with the
 //             tap-flipped, transposed weights;
 //   wgrad     dW[co][tap][ci] += sum_p dOut[p][co] in[p + tap][ci]
-//             M = Cout, N = Cin, K = pixels, split over pixel chunks.
-// Shared-memory tiles are filled with cp.async (zero fill for the padding)
-// through an XOR swizzle that keeps ldmatrix conflict-free.
+//             M = taps x Cin, N = Cout, K = pixels, split over CTAs.
 #include <cstdint>
 #include <cstdlib>
 #include <initializer_list>
@@ -52,11 +50,6 @@ __device__ __forceinline__ void cpAsyncWait() {
 
 __device__ __forceinline__ void ldmatrixX4(uint32_t& r0, uint32_t& r1, uint32_t& r2, uint32_t& r3, const void* p) {
     asm volatile("ldmatrix.sync.aligned.m8n8.x4.shared.b16 {%0, %1, %2, %3}, [%4];\n"
-                 : "=r"(r0), "=r"(r1), "=r"(r2), "=r"(r3)
-                 : "r"(smemAddr(p)));
-}
-__device__ __forceinline__ void ldmatrixX4T(uint32_t& r0, uint32_t& r1, uint32_t& r2, uint32_t& r3, const void* p) {
-    asm volatile("ldmatrix.sync.aligned.m8n8.x4.trans.shared.b16 {%0, %1, %2, %3}, [%4];\n"
                  : "=r"(r0), "=r"(r1), "=r"(r2), "=r"(r3)
                  : "r"(smemAddr(p)));
 }
@@ -1336,117 +1329,168 @@ size_t haloSmemBytes(uint32_t cout, uint32_t chunks, bool staged, uint32_t ring,
 }
 
 // -------------------------------------------------------------- wgrad ----
+// dW[co][tap][ci] += sum_p dOut[p][co] in[p + tap][ci] on the tensor cores:
+// K = pixels, so both operands are read "MN-major" straight from NHWC tiles
+// (the channels of a pixel are contiguous, the pixels are the K index).
+//   A (M = 128)  four horizontal taps x 32 input channels: rows of 64 bytes
+//                (32 channels, 64-byte swizzle), the next tap's block one pixel
+//                further (leading byte offset 64), so one MMA covers dx = 0, 1,
+//                2 of a vertical tap; the fourth block is the price of M = 128
+//                and its rows are not read back;
+//   B (N = coB)  the output gradient's channels in blocks of 32.
+// A persistent CTA owns `cpc` blocks of 32 input channels and up to 160 output
+// channels (3 x cpc x coB <= 512 accumulator columns, one set per vertical tap)
+// and walks 16 x 16 pixel tiles: per tile one box {32 channels, 18, 18} per
+// input block and one {32 channels, 16, 16} per output block, zero filled
+// outside the image, then 16 K steps x 3 vertical taps of straight-line MMAs
+// per input block.  The sums stay in tensor memory over all of a CTA's tiles
+// (at most a few hundred K steps, like a chunk of a split-K sum) and are added
+// to dW once, 32 consecutive input channels per warp instruction.
+// Bound: shared-memory operand reads at 32 output channels (4 KB of A per MMA),
+// a fixed ~20 us of set-up and read-out at the deep levels.  Measured over the
+// 19 layers of a 16 x 256^2 training step: 689 us; an mma.sync kernel that read
+// every input pixel once per tap took 4218 us.  Error against 64 bits on those
+// gradients: 2e-7 to 1.2e-5 (tensor-core sums truncate, so it grows with a
+// CTA's K steps), below the former kernel's on every layer.
 struct WgradArgs {
-    const __nv_bfloat16* in;    // [M][ldi], channels [0, cin)
-    const __nv_bfloat16* dout;  // [M][ldd], channels [0, cout)
-    float* dw;                  // [cout][9][cin], accumulated
-    uint32_t n, h, w_, cin, ldi, cout, ldd, M;
-    uint32_t chunk;             // pixels per block (multiple of 32)
+    float* dw;  // [cout][9][cin], accumulated
+    uint32_t cin, cout, tilesX, tilesY, numTiles;
+    uint32_t chunks, cpc, ciGroups;  // 32-channel input blocks: in all, per CTA; groups of them
+    uint32_t coB, coChunks;          // output channels per CTA and their 32-channel blocks
+    uint32_t stages, cols;
 };
+constexpr uint32_t kWgTile = 16u;                                   // tile edge in pixels
+constexpr uint32_t kWgHalo = kWgTile + 2u;
+constexpr uint32_t kWgInBytes = kWgHalo * kWgHalo * 64u;            // one input box
+constexpr uint32_t kWgInSlot = (kWgInBytes + 64u + 1023u) & ~1023u;  // + the fourth tap's last pixel
+constexpr uint32_t kWgOutSlot = kWgTile * kWgTile * 64u;
+constexpr uint32_t kWgStagesMax = 4u;
+constexpr uint32_t kWgBarBytes = 128u;
+constexpr uint32_t kWgCoMax = 160u;
 
-constexpr int kWB = 64;  // co and ci per block
+__global__ void __launch_bounds__(128, 1)
+    k_conv3x3_wgrad(const __grid_constant__ CUtensorMap mapIn, const __grid_constant__ CUtensorMap mapOut,
+                    WgradArgs a) {
+    extern __shared__ unsigned char dsm[];
+    const uint32_t raw = smemAddr(dsm);
+    unsigned char* sm = dsm + (((raw + 1023u) & ~1023u) - raw);
+    const uint32_t tid = threadIdx.x, warp = tid >> 5, lane = tid & 31u;
+    const uint32_t coBlock = blockIdx.y / a.ciGroups, chunk0 = (blockIdx.y - coBlock * a.ciGroups) * a.cpc;
+    const uint32_t co0 = coBlock * a.coB, nc = min(a.cpc, a.chunks - chunk0);
+    const uint32_t stageBytes = a.cpc * kWgInSlot + a.coChunks * kWgOutSlot;
+    uint64_t* bars = reinterpret_cast<uint64_t*>(sm + a.stages * stageBytes);
+    const uint32_t fullBar = smemAddr(bars), emptyBar = fullBar + 8u * kWgStagesMax;
+    const uint32_t doneBar = emptyBar + 8u * kWgStagesMax;
+    uint32_t* tslot = reinterpret_cast<uint32_t*>(bars + 2u * kWgStagesMax + 1u);
+    int* abortFlag = reinterpret_cast<int*>(tslot + 1);
 
-// Byte offset of 16-byte chunk `seg` (0..7) of row `r` in a 128-byte-row tile.
-__device__ __forceinline__ uint32_t swz128(uint32_t r, uint32_t seg) { return r * 128u + ((seg ^ (r & 7u)) << 4); }
-
-__global__ void __launch_bounds__(128) k_conv3x3_wgrad(WgradArgs a) {
-    __shared__ __align__(128) unsigned char sA[2][32 * 128];  // [pixel][64 co]
-    __shared__ __align__(128) unsigned char sB[2][32 * 128];  // [pixel][64 ci]
-    const uint32_t tid = threadIdx.x, lane = tid & 31u, warp = tid >> 5;
-    const uint32_t tap = blockIdx.z;
-    const uint32_t ciTiles = (a.cin + kWB - 1) / kWB;
-    const uint32_t co0 = (blockIdx.y / ciTiles) * kWB, ci0 = (blockIdx.y % ciTiles) * kWB;
-    const uint32_t p0 = blockIdx.x * a.chunk, p1 = min(p0 + a.chunk, a.M);
-    const int dy = (int)(tap / 3u) - 1, dx = (int)(tap % 3u) - 1;
-    const uint32_t HW = a.h * a.w_;
-    const uint32_t wm = warp >> 1, wn = warp & 1u;  // 2 x 2 warps of 32 co x 32 ci
-
-    auto loadStage = [&](uint32_t pb, int stage) {
-        // 32 pixels x 8 chunks for each operand: 2 + 2 chunks per thread.
-#pragma unroll
-        for (uint32_t k = 0; k < 2; ++k) {
-            uint32_t i = tid + k * 128u, row = i >> 3, seg = i & 7u;
-            uint32_t p = pb + row;
-            bool pv = p < p1;
-            bool v = pv && co0 + seg * 8u < a.cout;
-            const __nv_bfloat16* src = a.dout + (size_t)p * a.ldd + co0 + seg * 8u;
-            cpAsync16(&sA[stage][swz128(row, seg)], v ? src : a.dout, v ? 16u : 0u);
-            bool vb = false;
-            const __nv_bfloat16* bsrc = a.in;
-            if (pv && ci0 + seg * 8u < a.cin) {
-                uint32_t img = p / HW, rem = p - img * HW;
-                int yy = (int)(rem / a.w_) + dy, xx = (int)(rem % a.w_) + dx;
-                if (yy >= 0 && yy < (int)a.h && xx >= 0 && xx < (int)a.w_) {
-                    vb = true;
-                    bsrc = a.in + ((size_t)(img * a.h + (uint32_t)yy) * a.w_ + (uint32_t)xx) * a.ldi + ci0 + seg * 8u;
-                }
-            }
-            cpAsync16(&sB[stage][swz128(row, seg)], bsrc, vb ? 16u : 0u);
-        }
-    };
-
-    float acc[2][4][4];
-#pragma unroll
-    for (int i = 0; i < 2; ++i)
-#pragma unroll
-        for (int j = 0; j < 4; ++j)
-#pragma unroll
-            for (int k = 0; k < 4; ++k) acc[i][j][k] = 0.0f;
-
-    const uint32_t steps = (p1 > p0) ? (p1 - p0 + 31u) / 32u : 0u;
-    if (steps > 0) loadStage(p0, 0);
-    cpAsyncCommit();
-    for (uint32_t s = 0; s < steps; ++s) {
-        if (s + 1 < steps) loadStage(p0 + (s + 1) * 32u, (int)((s + 1) & 1u));
-        cpAsyncCommit();
-        cpAsyncWait<1>();
-        __syncthreads();
-        const int st = (int)(s & 1u);
-#pragma unroll
-        for (uint32_t kk = 0; kk < 2; ++kk) {  // 16 pixels each
-            uint32_t af[2][4];
-#pragma unroll
-            for (uint32_t mt = 0; mt < 2; ++mt) {
-                // A (co x p) from sA[p][co] through transposed 8x8 loads:
-                // matrices (co 0-7, p 0-7), (co 8-15, p 0-7), (co 0-7, p 8-15), (co 8-15, p 8-15).
-                uint32_t id = lane >> 3;
-                uint32_t prow = kk * 16u + ((id >> 1) << 3) + (lane & 7u);
-                uint32_t seg = (wm * 32u + mt * 16u) / 8u + (id & 1u);
-                ldmatrixX4T(af[mt][0], af[mt][1], af[mt][2], af[mt][3], &sA[st][swz128(prow, seg)]);
-            }
-#pragma unroll
-            for (uint32_t np = 0; np < 2; ++np) {
-                // B (p x ci): matrices (p 0-7, ci 0-7), (p 8-15, ci 0-7), (p 0-7, ci 8-15), (p 8-15, ci 8-15).
-                uint32_t id = lane >> 3;
-                uint32_t prow = kk * 16u + ((id & 1u) << 3) + (lane & 7u);
-                uint32_t seg = (wn * 32u + np * 16u) / 8u + (id >> 1);
-                uint32_t b0, b1, b2, b3;
-                ldmatrixX4T(b0, b1, b2, b3, &sB[st][swz128(prow, seg)]);
-#pragma unroll
-                for (uint32_t mt = 0; mt < 2; ++mt) {
-                    mmaBf16(acc[mt][2 * np], af[mt], b0, b1);
-                    mmaBf16(acc[mt][2 * np + 1], af[mt], b2, b3);
-                }
-            }
-        }
-        __syncthreads();
+    if (warp == 0) {
+        asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;\n" ::"r"(smemAddr(tslot)),
+                     "r"(a.cols));
+        asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;\n" ::);
     }
-    cpAsyncWait<0>();
+    if (tid == 0) {
+        for (uint32_t s = 0; s < a.stages; ++s) {
+            mbarInit(fullBar + 8u * s, 1);
+            mbarInit(emptyBar + 8u * s, 1);
+        }
+        mbarInit(doneBar, 1);
+        *abortFlag = 0;
+        asm volatile("fence.mbarrier_init.release.cluster;\n" ::: "memory");
+        asm volatile("prefetch.tensormap [%0];\n" ::"l"(&mapIn) : "memory");
+        asm volatile("prefetch.tensormap [%0];\n" ::"l"(&mapOut) : "memory");
+    }
+    __syncthreads();
+    asm volatile("tcgen05.fence::after_thread_sync;\n" ::: "memory");
+    const uint32_t taddr = *tslot;
+    volatile int* abortV = abortFlag;
+
+    if (tid == 0) {  // TMA producer
+        const uint32_t txBytes = nc * kWgInBytes + a.coChunks * kWgOutSlot;
+        RingPos pos{0u, 0u};
+        uint32_t g = 0;
+        for (uint32_t tile = blockIdx.x; tile < a.numTiles && !*abortV; tile += gridDim.x, ++g, pos.advance(a.stages)) {
+            if (g >= a.stages && !mbarWait(emptyBar + 8u * pos.slot, pos.phase ^ 1u)) {
+                *abortV = 1;
+                break;
+            }
+            const uint32_t tx = tile % a.tilesX, rest = tile / a.tilesX, ty = rest % a.tilesY, img = rest / a.tilesY;
+            const int x0 = (int)(tx * kWgTile), y0 = (int)(ty * kWgTile);
+            const uint32_t full = fullBar + 8u * pos.slot, base = smemAddr(sm + pos.slot * stageBytes);
+            mbarExpectTx(full, txBytes);
+            for (uint32_t c = 0; c < nc; ++c)
+                tmaLoad4(base + c * kWgInSlot, &mapIn, (int)((chunk0 + c) * 32u), x0 - 1, y0 - 1, (int)img, full);
+            for (uint32_t j = 0; j < a.coChunks; ++j)
+                tmaLoad4(base + a.cpc * kWgInSlot + j * kWgOutSlot, &mapOut, (int)(co0 + j * 32u), x0, y0, (int)img,
+                         full);
+        }
+    } else if (tid == 32) {  // MMA issuer
+        // kind::f16: D f32, A and B bf16, both MN-major, N = coB, M = 128.
+        const uint32_t idesc = (1u << 4) | (1u << 7) | (1u << 10) | (1u << 15) | (1u << 16) | ((a.coB >> 3) << 17) |
+                               ((128u >> 4) << 24);
+        // 8 pixels x 64 bytes between K groups (stride byte offset 512), version 1, 64-byte swizzle.
+        const uint32_t hi = (512u >> 4) | (1u << 14) | (4u << 29);
+        const uint32_t aLbo = (64u >> 4) << 16, bLbo = (kWgOutSlot >> 4) << 16;
+        RingPos pos{0u, 0u};
+        uint32_t acc = 0u;
+        bool ok = true;
+        for (uint32_t tile = blockIdx.x; tile < a.numTiles; tile += gridDim.x, pos.advance(a.stages)) {
+            if (*abortV || !mbarWait(fullBar + 8u * pos.slot, pos.phase)) {
+                ok = false;
+                break;
+            }
+            asm volatile("tcgen05.fence::after_thread_sync;\n" ::: "memory");
+            const uint32_t base = smemAddr(sm + pos.slot * stageBytes);
+            const uint32_t bLo = (((base + a.cpc * kWgInSlot) & 0x3FFFFu) >> 4) | bLbo;
+            for (uint32_t c = 0; c < nc; ++c) {
+                const uint32_t aLo = (((base + c * kWgInSlot) & 0x3FFFFu) >> 4) | aLbo;
+                const uint32_t d = taddr + 3u * c * a.coB;
 #pragma unroll
-    for (uint32_t mt = 0; mt < 2; ++mt)
+                for (uint32_t r = 0; r < kWgTile; ++r)
 #pragma unroll
-        for (uint32_t half = 0; half < 2; ++half) {
-            uint32_t co = co0 + wm * 32u + mt * 16u + (lane >> 2) + half * 8u;
-            if (co >= a.cout) continue;
+                    for (uint32_t dy = 0; dy < 3u; ++dy)
+                        mmaF16(d + dy * a.coB, aLo + (r + dy) * (kWgHalo * 64u / 16u), bLo + r * (kWgTile * 64u / 16u),
+                               hi, idesc, r ? 1u : acc);
+            }
+            acc = 1u;
+            umaCommit(emptyBar + 8u * pos.slot);
+        }
+        if (ok) umaCommit(doneBar);
+        else *abortV = 1;
+    }
+    __syncwarp();
+    // Lanes of warp q hold rows 32 q..: horizontal tap q, input channel = lane.
+    if (!mbarWait(doneBar, 0u)) *abortV = 1;
+    asm volatile("tcgen05.fence::after_thread_sync;\n" ::: "memory");
+    if (!*abortV && warp < 3u) {
+        for (uint32_t c = 0; c < nc; ++c) {
+            const uint32_t ci = (chunk0 + c) * 32u + lane;
+            for (uint32_t dy = 0; dy < 3u; ++dy) {
+                for (uint32_t k0 = 0; k0 < a.coB; k0 += 16u) {
+                    uint32_t rr[16];
+                    asm volatile(
+                        "tcgen05.ld.sync.aligned.32x32b.x16.b32 {%0, %1, %2, %3, %4, %5, %6, %7, %8, %9, %10, %11, "
+                        "%12, %13, %14, %15}, [%16];\n"
+                        : "=r"(rr[0]), "=r"(rr[1]), "=r"(rr[2]), "=r"(rr[3]), "=r"(rr[4]), "=r"(rr[5]), "=r"(rr[6]),
+                          "=r"(rr[7]), "=r"(rr[8]), "=r"(rr[9]), "=r"(rr[10]), "=r"(rr[11]), "=r"(rr[12]),
+                          "=r"(rr[13]), "=r"(rr[14]), "=r"(rr[15])
+                        : "r"(taddr + ((warp * 32u) << 16) + (3u * c + dy) * a.coB + k0));
+                    asm volatile("tcgen05.wait::ld.sync.aligned;\n" ::: "memory");
 #pragma unroll
-            for (uint32_t nt = 0; nt < 4; ++nt) {
-                uint32_t ci = ci0 + wn * 32u + nt * 8u + (lane & 3u) * 2u;
-                if (ci >= a.cin) continue;
-                float* dst = a.dw + ((size_t)co * 9u + tap) * a.cin + ci;
-                atomicAdd(dst, acc[mt][nt][half * 2 + 0]);
-                atomicAdd(dst + 1, acc[mt][nt][half * 2 + 1]);
+                    for (uint32_t k = 0; k < 16; ++k) {
+                        const uint32_t co = co0 + k0 + k;
+                        if (ci < a.cin && co < a.cout)
+                            atomicAdd(a.dw + ((size_t)co * 9u + dy * 3u + warp) * a.cin + ci, __uint_as_float(rr[k]));
+                    }
+                }
             }
         }
+    }
+    asm volatile("tcgen05.fence::before_thread_sync;\n" ::: "memory");
+    __syncthreads();
+    if (*abortV && tid == 0) atomicExch(&g_unetError, 4);
+    asm volatile("tcgen05.fence::after_thread_sync;\n" ::: "memory");
+    if (warp == 0) asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;\n" ::"r"(taddr), "r"(a.cols));
 }
 
 // ------------------------------------------------------- elementwise ----
@@ -1598,16 +1642,51 @@ __device__ __forceinline__ void st8(__nv_bfloat16* p, const float (&f)[8]) {
     *reinterpret_cast<uint4*>(p) = make_uint4(w[0], w[1], w[2], w[3]);
 }
 
-__global__ void k_relu_backward8(const __nv_bfloat16* out, uint32_t ldo, const __nv_bfloat16* dout, uint32_t ldd,
-                                 __nv_bfloat16* dpre, uint32_t ldp, uint32_t groups, uint32_t total) {
-    for (uint32_t i = blockIdx.x * blockDim.x + threadIdx.x; i < total; i += gstride()) {
-        const uint32_t p = i / groups, k = (i - p * groups) * 8u;
-        float o[8], d[8];
-        ld8(out + (size_t)p * ldo + k, o);
-        ld8(dout + (size_t)p * ldd + k, d);
+// The ReLU gradient (kRelu: dpre = dout where out > 0) and/or the bias gradient
+// (kBias: db[c] += the sum of dpre, or of dout itself without kRelu) over
+// groups of 8 channels.  A thread keeps one channel group, so its eight sums
+// stay in registers over its pixels; the block adds its partial sums in shared
+// memory and issues one atomic per channel.  Memory-bound: each operand is
+// read once, whole 64-byte runs of a pixel by neighbouring threads (32
+// channels of 2^20 pixels with both gradients: 36 us, 5.6 TB/s).  Over a
+// 16 x 256^2 training step 341 us; the separate passes with one channel per
+// thread took 236 + 719 us.
+constexpr uint32_t kRbThreads = 256u;
+template <bool kRelu, bool kBias>
+__global__ void __launch_bounds__(256) k_relu_bias8(const __nv_bfloat16* out, uint32_t ldo, const __nv_bfloat16* dout,
+                                                    uint32_t ldd, __nv_bfloat16* dpre, uint32_t ldp, uint32_t groups,
+                                                    uint32_t M, float* db) {
+    const uint32_t lanes = kRbThreads / groups, lane = threadIdx.x / groups;
+    const uint32_t g = threadIdx.x - lane * groups, k = g * 8u;
+    float s[8] = {0.0f, 0.0f, 0.0f, 0.0f, 0.0f, 0.0f, 0.0f, 0.0f};
+    if (lane < lanes) {
+        const uint64_t step = (uint64_t)gridDim.x * lanes;
+#pragma unroll 4
+        for (uint64_t p = (uint64_t)blockIdx.x * lanes + lane; p < M; p += step) {
+            float d[8];
+            ld8(dout + (size_t)p * ldd + k, d);
+            if (kRelu) {
+                float o[8];
+                ld8(out + (size_t)p * ldo + k, o);
 #pragma unroll
-        for (int j = 0; j < 8; ++j) d[j] = o[j] > 0.0f ? d[j] : 0.0f;
-        st8(dpre + (size_t)p * ldp + k, d);
+                for (int j = 0; j < 8; ++j) d[j] = o[j] > 0.0f ? d[j] : 0.0f;
+                st8(dpre + (size_t)p * ldp + k, d);
+            }
+            if (kBias) {
+#pragma unroll
+                for (int j = 0; j < 8; ++j) s[j] += d[j];
+            }
+        }
+    }
+    if (!kBias) return;
+    __shared__ float part[kRbThreads][9];
+#pragma unroll
+    for (int j = 0; j < 8; ++j) part[threadIdx.x][j] = s[j];
+    __syncthreads();
+    for (uint32_t c = threadIdx.x; c < groups * 8u; c += kRbThreads) {
+        float t = 0.0f;
+        for (uint32_t l = 0; l < lanes; ++l) t += part[l * groups + (c >> 3)][c & 7u];
+        atomicAdd(&db[c], t);
     }
 }
 
@@ -1858,6 +1937,22 @@ inline bool vec8(std::initializer_list<uint32_t> counts, std::initializer_list<c
     for (const void* q : ptrs)
         if (reinterpret_cast<uintptr_t>(q) % 16u) return false;
     return total > 0 && total < (1ull << 31);
+}
+
+// k_relu_bias8 over `pixels` pixels of `c` channels: up to six resident blocks
+// per SM, at least eight pixels per thread.
+template <bool kRelu, bool kBias>
+int launchReluBias(const void* out, uint32_t ldo, const void* dout, uint32_t ldd, void* dpre, uint32_t ldp, uint32_t c,
+                   uint32_t pixels, float* db, void* stream) {
+    if (deviceProp().multiProcessorCount == 0) ensureDevice();
+    const uint32_t groups = c / 8u, perBlock = kRbThreads / groups * 8u;
+    const uint32_t blocks = (uint32_t)(((uint64_t)pixels + perBlock - 1u) / perBlock);
+    const uint32_t grid = std::min(blocks, (uint32_t)deviceProp().multiProcessorCount * 6u);
+    k_relu_bias8<kRelu, kBias><<<grid, kRbThreads, 0, static_cast<cudaStream_t>(stream)>>>(
+        static_cast<const __nv_bfloat16*>(out), ldo, static_cast<const __nv_bfloat16*>(dout), ldd,
+        static_cast<__nv_bfloat16*>(dpre), ldp, groups, pixels, db);
+    DK_CUDA(cudaGetLastError(), "relu / bias gradient launch");
+    return DK_OK;
 }
 
 // 3: halo-row TMA + tcgen05 convolution where the layer fits it, else the
@@ -2128,6 +2223,65 @@ int launchConvTma(const ConvArgs& c, cudaStream_t st, bool rowTap) {
     return DK_OK;
 }
 
+// The weight gradient's launch: input blocks per CTA from the accumulator
+// columns (3 x coB per block of 32 channels) and two pipeline stages of shared
+// memory, fewer where the pixel tiles alone would leave SMs idle.
+int launchWgrad(const __nv_bfloat16* in, uint32_t ldi, const __nv_bfloat16* dout, uint32_t ldd, uint32_t n, uint32_t h,
+                uint32_t w, uint32_t cin, uint32_t cout, float* dw, cudaStream_t st) {
+    EncodeTiledFn enc = encodeTiled();
+    if (!enc) return fail(DK_ERROR_COMMAND_FAILED, "cuTensorMapEncodeTiled is not available");
+    if (deviceProp().multiProcessorCount == 0) ensureDevice();
+    const uint32_t sms = (uint32_t)deviceProp().multiProcessorCount;
+    const size_t budget = (size_t)deviceProp().sharedMemPerBlockOptin - 1024u - kWgBarBytes;
+    WgradArgs a;
+    a.dw = dw;
+    a.cin = cin;
+    a.cout = cout;
+    a.tilesX = (w + kWgTile - 1u) / kWgTile;
+    a.tilesY = (h + kWgTile - 1u) / kWgTile;
+    a.numTiles = a.tilesX * a.tilesY * n;
+    a.chunks = (cin + 31u) / 32u;
+    const uint32_t coBlocks = (cout + kWgCoMax - 1u) / kWgCoMax;
+    a.coB = ((cout + coBlocks - 1u) / coBlocks + 15u) / 16u * 16u;
+    a.coChunks = (a.coB + 31u) / 32u;
+    auto stageBytes = [&](uint32_t cpc) { return (size_t)cpc * kWgInSlot + (size_t)a.coChunks * kWgOutSlot; };
+    a.cpc = 1u;
+    while (a.cpc < a.chunks && 3u * a.coB * (a.cpc + 1u) <= 512u && 2u * stageBytes(a.cpc + 1u) <= budget) ++a.cpc;
+    while (a.cpc > 1u && (uint64_t)a.numTiles * coBlocks * ((a.chunks + a.cpc - 1u) / a.cpc) < sms) --a.cpc;
+    a.ciGroups = (a.chunks + a.cpc - 1u) / a.cpc;
+    a.cpc = (a.chunks + a.ciGroups - 1u) / a.ciGroups;
+    const uint32_t groups = coBlocks * a.ciGroups;
+    a.stages = 2u;
+    while (a.stages < kWgStagesMax && (a.stages + 1u) * stageBytes(a.cpc) <= budget) ++a.stages;
+    a.cols = 32u;
+    while (a.cols < 3u * a.cpc * a.coB) a.cols <<= 1;
+    alignas(64) CUtensorMap mapIn, mapOut;
+    cuuint32_t unit[4] = {1u, 1u, 1u, 1u};
+    auto encode = [&](CUtensorMap* map, const __nv_bfloat16* p, uint32_t ld, uint32_t c, uint32_t edge) {
+        cuuint64_t dims[4] = {c, w, h, n};
+        cuuint64_t strides[3] = {(cuuint64_t)ld * 2u, (cuuint64_t)w * ld * 2u, (cuuint64_t)h * w * ld * 2u};
+        cuuint32_t box[4] = {32u, edge, edge, 1u};
+        return enc(map, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 4, const_cast<__nv_bfloat16*>(p), dims, strides, box, unit,
+                   CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_64B, CU_TENSOR_MAP_L2_PROMOTION_L2_128B,
+                   CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
+    };
+    if (encode(&mapIn, in, ldi, cin, kWgHalo) != CUDA_SUCCESS)
+        return fail(DK_ERROR_INVALID_ARGUMENT, "activation tensor map rejected");
+    if (encode(&mapOut, dout, ldd, cout, kWgTile) != CUDA_SUCCESS)
+        return fail(DK_ERROR_INVALID_ARGUMENT, "gradient tensor map rejected");
+    const size_t smem = a.stages * stageBytes(a.cpc) + 1024u + kWgBarBytes;
+    static size_t configured = 0;
+    if (smem > configured) {
+        DK_CUDA(cudaFuncSetAttribute(k_conv3x3_wgrad, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem),
+                "conv3x3 wgrad shared memory");
+        configured = smem;
+    }
+    const uint32_t gx = std::min(a.numTiles, std::max(1u, sms / groups));
+    k_conv3x3_wgrad<<<dim3(gx, groups), 128, smem, st>>>(mapIn, mapOut, a);
+    DK_CUDA(cudaGetLastError(), "conv3x3 wgrad launch");
+    return DK_OK;
+}
+
 }  // namespace
 }  // namespace dk
 
@@ -2195,33 +2349,16 @@ int dk_unet_conv3x3_wgrad(const void* in, uint32_t ldi, const void* dout, uint32
     uint64_t M = (uint64_t)n * h * w;
     if (M == 0) return DK_OK;
     if (M >= (1ull << 31)) return dk::fail(DK_ERROR_INVALID_ARGUMENT, "dk_unet_conv3x3_wgrad: tensor too large");
-    uint32_t tiles = ((cout + 63u) / 64u) * ((cin + 63u) / 64u);
-    // Enough pixel chunks to fill the GPU several times over, 32-pixel aligned.
-    if (dk::deviceProp().multiProcessorCount == 0) dk::ensureDevice();
-    uint64_t target = (uint64_t)dk::deviceProp().multiProcessorCount * 8u;
-    uint64_t perTile = (target + 9u * tiles - 1) / (9u * tiles);
-    uint64_t chunk = (M + perTile - 1) / perTile;
-    chunk = ((chunk + 31u) / 32u) * 32u;
-    if (chunk < 256u) chunk = 256u;
-    dk::WgradArgs a{static_cast<const bf16*>(in), static_cast<const bf16*>(dout), dweight, n, h, w, cin, ldi, cout,
-                    ldd, (uint32_t)M, (uint32_t)chunk};
-    dim3 grid((uint32_t)((M + chunk - 1) / chunk), tiles, 9);
-    dk::k_conv3x3_wgrad<<<grid, 128, 0, static_cast<cudaStream_t>(stream)>>>(a);
-    DK_CUDA(cudaGetLastError(), "conv3x3 wgrad launch");
-    return DK_OK;
+    return dk::launchWgrad(static_cast<const bf16*>(in), ldi, static_cast<const bf16*>(dout), ldd, n, h, w, cin, cout,
+                           dweight, static_cast<cudaStream_t>(stream));
 }
 
 int dk_unet_relu_backward(const void* out, uint32_t ldo, const void* dout, uint32_t ldd, void* dpre, uint32_t ldp,
                           uint32_t c, uint32_t pixels, void* stream) {
     if (!out || !dout || !dpre || c % 2u) return dk::fail(DK_ERROR_INVALID_ARGUMENT, "dk_unet_relu_backward");
-    const uint64_t total8 = (uint64_t)pixels * (c / 8u);
-    if (dk::vec8({c, ldo, ldd, ldp}, {out, dout, dpre}, total8)) {
-        dk::k_relu_backward8<<<dk::gridFor(total8), 256, 0, static_cast<cudaStream_t>(stream)>>>(
-            static_cast<const bf16*>(out), ldo, static_cast<const bf16*>(dout), ldd, static_cast<bf16*>(dpre), ldp,
-            c / 8u, (uint32_t)total8);
-        DK_CUDA(cudaGetLastError(), "relu backward launch");
-        return DK_OK;
-    }
+    if (c / 8u <= dk::kRbThreads &&
+        dk::vec8({c, ldo, ldd, ldp}, {out, dout, dpre}, (uint64_t)pixels * (c / 8u)))
+        return dk::launchReluBias<true, false>(out, ldo, dout, ldd, dpre, ldp, c, pixels, nullptr, stream);
     dk::k_relu_backward<<<dk::gridFor((uint64_t)pixels * c / 2), 256, 0, static_cast<cudaStream_t>(stream)>>>(
         static_cast<const bf16*>(out), ldo, static_cast<const bf16*>(dout), ldd, static_cast<bf16*>(dpre), ldp, c,
         pixels);
@@ -2231,6 +2368,8 @@ int dk_unet_relu_backward(const void* out, uint32_t ldo, const void* dout, uint3
 
 int dk_unet_bias_grad(const void* dpre, uint32_t ld, uint32_t c, uint32_t pixels, float* dbias, void* stream) {
     if (!dpre || !dbias || c == 0 || c > 256u) return dk::fail(DK_ERROR_INVALID_ARGUMENT, "dk_unet_bias_grad");
+    if (dk::vec8({c, ld}, {dpre}, (uint64_t)pixels * (c / 8u)))
+        return dk::launchReluBias<false, true>(nullptr, 0, dpre, ld, nullptr, 0, c, pixels, dbias, stream);
     uint32_t lanes = 256u / c;
     uint64_t blocks = ((uint64_t)pixels + lanes * 64u - 1) / (lanes * 64u);
     int grid = (int)(blocks < 1 ? 1 : (blocks > 1024 ? 1024 : blocks));
@@ -2238,6 +2377,16 @@ int dk_unet_bias_grad(const void* dpre, uint32_t ld, uint32_t c, uint32_t pixels
                                                                           dbias);
     DK_CUDA(cudaGetLastError(), "bias grad launch");
     return DK_OK;
+}
+
+int dk_unet_relu_bias_backward(const void* out, uint32_t ldo, const void* dout, uint32_t ldd, void* dpre, uint32_t ldp,
+                               uint32_t c, uint32_t pixels, float* dbias, void* stream) {
+    if (!out || !dout || !dpre || !dbias || c == 0 || c % 2u || c > 256u)
+        return dk::fail(DK_ERROR_INVALID_ARGUMENT, "dk_unet_relu_bias_backward");
+    if (dk::vec8({c, ldo, ldd, ldp}, {out, dout, dpre}, (uint64_t)pixels * (c / 8u)))
+        return dk::launchReluBias<true, true>(out, ldo, dout, ldd, dpre, ldp, c, pixels, dbias, stream);
+    const int rc = dk_unet_relu_backward(out, ldo, dout, ldd, dpre, ldp, c, pixels, stream);
+    return rc != DK_OK ? rc : dk_unet_bias_grad(dpre, ldp, c, pixels, dbias, stream);
 }
 
 int dk_unet_avgpool2(const void* in, uint32_t ldi, void* out, uint32_t ldo, uint32_t coOff, uint32_t c, uint32_t n,

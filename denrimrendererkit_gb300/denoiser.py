@@ -268,14 +268,14 @@ class UNet:
         M = n * h * w
         if l.act:
             dpre, ldp = B["dpre"], l.cout
-            self._check(lib.dk_unet_relu_backward(_ptr(out, out_off), ldo, _ptr(gout, gout_off), ldg, _ptr(dpre), ldp,
-                                                  l.cout, M, st))
+            self._check(lib.dk_unet_relu_bias_backward(_ptr(out, out_off), ldo, _ptr(gout, gout_off), ldg, _ptr(dpre),
+                                                       ldp, l.cout, M, _ptr(l.gb), st))
             dsrc, dsrc_off, ldd = dpre, 0, ldp
         else:
             dsrc, dsrc_off, ldd = gout, gout_off, ldg
+            self._check(lib.dk_unet_bias_grad(_ptr(dsrc, dsrc_off), ldd, l.cout, M, _ptr(l.gb), st))
         self._check(lib.dk_unet_conv3x3_wgrad(_ptr(x, x_off), ldx, _ptr(dsrc, dsrc_off), ldd, n, h, w, l.cin, l.cout,
                                               _ptr(l.gw), st))
-        self._check(lib.dk_unet_bias_grad(_ptr(dsrc, dsrc_off), ldd, l.cout, M, _ptr(l.gb), st))
         if gin is not None:
             self._check(lib.dk_unet_conv3x3(_ptr(dsrc, dsrc_off), n, h, w, l.cout, ldd, _ptr(l.wflip), None, l.cin,
                                             _ptr(gin, gin_off), ldgi, 0, 0, gin_accumulate, st))

@@ -109,6 +109,7 @@ def load(build_if_missing: bool = False) -> C.CDLL:
             "dk_unet_conv3x3_wgrad": (i32, [P, u32, P, u32, u32, u32, u32, u32, u32, P, P]),
             "dk_unet_relu_backward": (i32, [P, u32, P, u32, P, u32, u32, u32, P]),
             "dk_unet_bias_grad": (i32, [P, u32, u32, u32, P, P]),
+            "dk_unet_relu_bias_backward": (i32, [P, u32, P, u32, P, u32, u32, u32, P, P]),
             "dk_unet_avgpool2": (i32, [P, u32, P, u32, u32, u32, u32, u32, u32, P]),
             "dk_unet_avgpool2_backward": (i32, [P, u32, P, u32, u32, u32, u32, u32, i32, P]),
             "dk_unet_upsample2": (i32, [P, u32, P, u32, u32, u32, u32, u32, u32, P]),

@@ -544,6 +544,10 @@ int dk_unet_relu_backward(const void* out, uint32_t ldo, const void* dout, uint3
                           uint32_t c, uint32_t pixels, void* stream);
 /* dbias[c] += sum_p dpre[p][c] (c <= 256). */
 int dk_unet_bias_grad(const void* dpre, uint32_t ld, uint32_t c, uint32_t pixels, float* dbias, void* stream);
+/* dk_unet_relu_backward followed by dk_unet_bias_grad of its result (c <= 256),
+ * in one pass over the tensors where they are 16-byte aligned. */
+int dk_unet_relu_bias_backward(const void* out, uint32_t ldo, const void* dout, uint32_t ldd, void* dpre, uint32_t ldp,
+                               uint32_t c, uint32_t pixels, float* dbias, void* stream);
 /* dk_unet_conv3x3 (no accumulation) followed by dk_unet_avgpool2 of the
  * channels it wrote: pool[q][c] (channel stride pool_ld, offset 0) = the 2x2
  * average of out's channels co_off .. co_off + cout; h and w even.  The same
