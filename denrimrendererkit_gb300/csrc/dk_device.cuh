@@ -215,9 +215,11 @@ __device__ __forceinline__ int wideVisit(const DevScene& S, uint32_t node, float
 // Closest hit.  Returns argmin over (t, reference leaf slot): the reference's
 // strict `t < closest.t` under left-first DFS picks, among equal t, the
 // triangle that comes first in its primitiveIndices order, which is the slot.
-__device__ HitRec traceClosest(const DevScene& S, float3 o, float3 d) {
+// `tmax` bounds the query: a hit beyond it is not looked for (tri stays kNoHit
+// and t the bound); one below it is the unbounded query's answer.
+__device__ HitRec traceClosest(const DevScene& S, float3 o, float3 d, float tmax = INFINITY) {
     HitRec best;
-    best.t = INFINITY;
+    best.t = tmax;
     best.tri = kNoHit;
     best.u = 0.0f;
     best.v = 0.0f;

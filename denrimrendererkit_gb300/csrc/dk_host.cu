@@ -883,7 +883,7 @@ static int renderPreview(Session* s, uint32_t tx, uint32_t ty, uint32_t tw, uint
     if (rc != DK_OK) return rc;
     DK_CUDA(cudaEventRecord(e0, s->stream), "cudaEventRecord");
     DK_CUDA(dk::launchPreview(s->scene, P, s->accum, s->scene.mat_count, s->opaqueMask,
-                              st.quality == DK_QUALITY_INTERACTIVE, s->grids.extend, s->stream),
+                              st.quality == DK_QUALITY_INTERACTIVE, s->stream),
             "preview launch");
     DK_CUDA(cudaEventRecord(e1, s->stream), "cudaEventRecord");
     DK_CUDA(cudaEventSynchronize(e1), "render");

@@ -207,6 +207,13 @@ __device__ __noinline__ HitRec traceSceneCounting(const DevScene& S, float3 o, f
     return r;
 }
 
+// The closest hit nearer than `tmax`; a record with t >= tmax is as good as a
+// miss.  Scenes with volumes and the 8-wide tree take the unbounded query.
+__device__ __noinline__ HitRec traceSceneWithin(const DevScene& S, float3 o, float3 d, float tmax) {
+    if (S.wide8 || S.volume_count) return traceSceneCounting(S, o, d);
+    return traceClosest(S, o, d, tmax);
+}
+
 // Subsurface walk helpers (PathTrace.metal:3490-3523).
 __device__ __forceinline__ float sampleSubsurfaceFreeFlight(float3 sigmaT, float ux, float uy) {
     float sigma = sigmaT.z;
@@ -1348,13 +1355,26 @@ __device__ __forceinline__ float smoothstepf(float e0, float e1, float x) {  // 
     return t * t * (3.0f - 2.0f * t);
 }
 
+// The preview kernels call one copy of the environment lookup: inlined at each
+// of its dozen uses it made them stall on instruction fetch (see k_preview).
+__device__ __noinline__ float3 sampleEnvironmentCall(const DevScene& S, float3 d) { return sampleEnvironment(S, d); }
+
+// The environment along the six axis directions sampleInteractiveDiffuse-
+// Environment blends: the same for every pixel, so a block samples them once.
+__device__ __forceinline__ void loadAxisEnvironment(const DevScene& S, float3* axis) {
+    if (threadIdx.x < 6u) {
+        const float s = (threadIdx.x & 1u) ? -1.0f : 1.0f;
+        const uint32_t a = threadIdx.x >> 1;
+        axis[threadIdx.x] = sampleEnvironmentCall(S, f3(a == 1u ? s : 0.0f, a == 0u ? s : 0.0f, a == 2u ? s : 0.0f));
+    }
+    __syncthreads();
+}
+
 // sampleInteractiveDiffuseEnvironment (:3805-3823)
-__device__ float3 interactiveDiffuseEnv(const DevScene& S, float3 n) {
-    float3 up = sampleEnvironment(S, f3(0.0f, 1.0f, 0.0f));
-    float3 down = sampleEnvironment(S, f3(0.0f, -1.0f, 0.0f));
-    float3 side = (sampleEnvironment(S, f3(1.0f, 0.0f, 0.0f)) + sampleEnvironment(S, f3(-1.0f, 0.0f, 0.0f)) +
-                   sampleEnvironment(S, f3(0.0f, 0.0f, 1.0f)) + sampleEnvironment(S, f3(0.0f, 0.0f, -1.0f))) *
-                  0.25f;
+__device__ float3 interactiveDiffuseEnv(const float3* axis, float3 n) {
+    float3 up = axis[0];
+    float3 down = axis[1];
+    float3 side = (axis[2] + axis[3] + axis[4] + axis[5]) * 0.25f;
     float upW = smoothstepf(-0.15f, 0.85f, n.y);
     float downW = smoothstepf(0.15f, -0.85f, n.y);
     float sideW = fmaxf(0.0f, 1.0f - upW - downW);
@@ -1368,38 +1388,42 @@ __device__ __forceinline__ float3 interactiveHemisphere(float3 d, float3 n) {
     return normalize(d);
 }
 
-// sampleInteractiveSpecularEnvironment (:3833-3880)
-__device__ float3 interactiveSpecularEnv(const DevScene& S, float3 r, float3 n, float roughness) {
+// sampleInteractiveSpecularEnvironment (:3833-3880); `diffuse` is
+// interactiveDiffuseEnv at the same normal.
+__device__ __noinline__ float3 interactiveSpecularEnv(const DevScene& S, float3 r, float3 n, float roughness, float3 diffuse) {
     r = interactiveHemisphere(normalize(r), n);
     roughness = clampf(roughness, 0.0f, 1.0f);
     float spread = roughness * roughness;
     float3 helper = fabsf(r.y) < 0.999f ? f3(0.0f, 1.0f, 0.0f) : f3(1.0f, 0.0f, 0.0f);
     float3 t = normalize(cross(helper, r));
     float3 b = cross(r, t);
-    float3 cone = sampleEnvironment(S, r) * 0.42f;
-    cone += sampleEnvironment(S, interactiveHemisphere(r + t * spread * 0.95f + n * spread * 0.18f, n)) * 0.145f;
-    cone += sampleEnvironment(S, interactiveHemisphere(r - t * spread * 0.95f + n * spread * 0.18f, n)) * 0.145f;
-    cone += sampleEnvironment(S, interactiveHemisphere(r + b * spread * 0.95f + n * spread * 0.18f, n)) * 0.145f;
-    cone += sampleEnvironment(S, interactiveHemisphere(r - b * spread * 0.95f + n * spread * 0.18f, n)) * 0.145f;
-    float3 diffuse = interactiveDiffuseEnv(S, n);
+    float3 cone = sampleEnvironmentCall(S, r) * 0.42f;
+    cone += sampleEnvironmentCall(S, interactiveHemisphere(r + t * spread * 0.95f + n * spread * 0.18f, n)) * 0.145f;
+    cone += sampleEnvironmentCall(S, interactiveHemisphere(r - t * spread * 0.95f + n * spread * 0.18f, n)) * 0.145f;
+    cone += sampleEnvironmentCall(S, interactiveHemisphere(r + b * spread * 0.95f + n * spread * 0.18f, n)) * 0.145f;
+    cone += sampleEnvironmentCall(S, interactiveHemisphere(r - b * spread * 0.95f + n * spread * 0.18f, n)) * 0.145f;
     return mix3(cone, diffuse, smoothstepf(0.62f, 0.95f, roughness));
 }
 
 // interactiveContactAmbientOcclusion (:4276-4360): four short probes around
 // the normal, each nearby occluder weighted by its opacity and proximity.
-__device__ float interactiveContactAO(const DevScene& S, MatTable mt, const Hit& h, const Material& m, float3 n) {
-    TangentFrame frame = makeTangentFrame(n, h.tangent, h.bitangent);
+// Called by every thread of the block (`hit`: this thread has a surface).
+__device__ __forceinline__ float interactiveContactAO(const DevScene& S, MatTable mt, bool hit, const Hit& h,
+                                                      const Material& m, float3 n) {
     constexpr float kRadius = 0.34f;
+    TangentFrame frame = makeTangentFrame(n, h.tangent, h.bitangent);
     const float3 local[4] = {f3(0.000f, 0.000f, 1.000f), f3(0.780f, 0.180f, 0.600f), f3(-0.420f, 0.720f, 0.552f),
                              f3(-0.620f, -0.520f, 0.587f)};
     float occlusion = 0.0f;
 #pragma unroll 1
     for (int k = 0; k < 4; ++k) {
+        __syncthreads();
+        if (!hit) continue;
         float3 l = normalize(local[k]);
         float3 dir = normalize(l.x * frame.tangent + l.y * frame.bitangent + l.z * n);
         Ray ray{h.position + n * 0.003f, dir};
         sdfCount(S.sdf_counters, kSdfShadowSceneQueries);
-        HitRec r = traceSceneCounting(S, ray.origin, ray.direction);
+        HitRec r = traceSceneWithin(S, ray.origin, ray.direction, kRadius);
         if (r.tri == kNoHit || !(r.t < kRadius)) continue;
         Hit oh = makeHitAny(S, ray, r);
         Material om = materialForHit(S, mt, oh);
@@ -1410,151 +1434,198 @@ __device__ float interactiveContactAO(const DevScene& S, MatTable mt, const Hit&
     return 1.0f - clampf((occlusion / 4.0f) * strength, 0.0f, 0.72f);
 }
 
+__device__ __forceinline__ void storePreview(const Accum& A, size_t pix, float4 beauty) {
+    A.sum[pix] = beauty;
+    A.comp[pix] = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+    A.resolved[pix] = D4{0.0, 0.0, 0.0, 0.0};
+    A.count[pix] = 1u;
+}
+
+// One thread per pixel, a warp per 8 x 4 pixels.  The kernel is bound by
+// instruction fetch: some 400 KB of code, of which every warp runs a large
+// part once, so warps at different places evict each other's instructions (a
+// version without barriers spent 31 of 36 cycles between a warp's issues
+// waiting for an instruction, whatever its occupancy).  Hence large blocks
+// whose warps go through the phases -- primary ray, each light, environment,
+// each occlusion probe -- together, with a barrier between phases, so that one
+// fetch serves 16 warps; threads without a hit go along with a neighbour's.
+// Interactive 1280 x 720 of the material scene, whole frame with its display
+// encoding: 7.56 ms as a grid-stride loop with everything inlined; 4.0 with the
+// axis directions of the environment sampled once per block and the occlusion
+// probes bounded by their radius; 2.7 with the environment lookup called;
+// 0.78 with the phases.  Blocks x minimum residency 128 x 4 / 256 x 2 / 512 x 1 /
+// 512 x 2 / 1024 x 1: 1.22 / 0.99 / 1.03 / 0.78 / 0.82 ms.
+#ifndef DK_PREVIEW_BLOCK
+#define DK_PREVIEW_BLOCK 512
+#endif
+#ifndef DK_PREVIEW_MIN_BLOCKS
+#define DK_PREVIEW_MIN_BLOCKS 2
+#endif
 template <bool kInteractive>
-__global__ void __launch_bounds__(128) k_preview(DevScene S, DevParams P, Accum A, MatTable mt, uint32_t opaqueMask) {
-    const uint32_t tileN = P.tile_w * P.tile_h;
+__global__ void __launch_bounds__(DK_PREVIEW_BLOCK, DK_PREVIEW_MIN_BLOCKS)
+    k_preview(const __grid_constant__ DevScene S, const __grid_constant__ DevParams P, Accum A, MatTable mt,
+              uint32_t opaqueMask) {
     const size_t plane = (size_t)P.width * P.height;
-    for (uint32_t i = globalId(); i < tileN; i += gridStride()) {
-        const uint32_t px = P.tile_x + i % P.tile_w, py = P.tile_y + i / P.tile_w;
-        const size_t pix = (size_t)py * P.width + px;
-        Ray ray = makeCameraRay(P.cam, P.width, P.height, px, py, 0.5f, 0.5f, 0.0f, 0.0f);
+    __shared__ float3 axisEnv[6];
+    if (kInteractive) loadAxisEnvironment(S, axisEnv);
+    const uint32_t lane = laneId(), warp = (blockIdx.x * DK_PREVIEW_BLOCK + threadIdx.x) >> 5;
+    const uint32_t tilesX = (P.tile_w + 7u) / 8u;
+    const uint32_t lx = (warp % tilesX) * 8u + (lane & 7u), ly = (warp / tilesX) * 4u + (lane >> 3);
+    const bool valid = lx < P.tile_w && ly < P.tile_h;
+    // Threads outside the tile, and later those whose ray missed, run the block's
+    // phases on a neighbour's pixel or hit and store nothing of them.
+    const uint32_t px = P.tile_x + min(lx, P.tile_w - 1u), py = P.tile_y + min(ly, P.tile_h - 1u);
+    const size_t pix = (size_t)py * P.width + px;
+    Ray ray = makeCameraRay(P.cam, P.width, P.height, px, py, 0.5f, 0.5f, 0.0f, 0.0f);
+    HitRec rec;
+    rec.tri = kNoHit;
+    if (valid) {
         sdfCount(S.sdf_counters, kSdfPrimarySceneQueries);
-        HitRec rec = traceSceneCounting(S, ray.origin, ray.direction);
-        float4 beauty;
-        if (rec.tri == kNoHit) {
-            float alpha = P.transparent_background ? 0.0f : 1.0f;
-            float3 color = mx(f3(P.bg[0], P.bg[1], P.bg[2]), f3(0.0f));
-            if (!P.transparent_background && P.shows_env_bg) color = sampleEnvironment(S, ray.direction);
-            beauty = make_float4(color.x, color.y, color.z, alpha);
-            A.aov[0 * plane + pix] = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
-            A.aov[1 * plane + pix] = make_float4(0.5f, 0.5f, 0.5f, 0.0f);
-            for (int k = 2; k < 6; ++k) A.aov[k * plane + pix] = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
-        } else {
-            Hit h = makeHitAny(S, ray, rec);
-            Material m = materialForHit(S, mt, h);
-            uint32_t nIdx = (uint32_t)m.parameters.w;
-            if (nIdx != 0u) h = applyNormalMap(S, h, nIdx, ray.direction);
-            uint32_t bIdx = (uint32_t)m.parameters.z;
-            if (bIdx != 0u) {  // applyBaseColorTexture
-                float4 t = sampleTexture(S, bIdx, h.uv, make_float4(1.0f, 1.0f, 1.0f, 1.0f));
-                m.baseColor = make_float4(ex::mul(m.baseColor.x, t.x), ex::mul(m.baseColor.y, t.y),
-                                          ex::mul(m.baseColor.z, t.z), ex::mul(m.baseColor.w, t.w));
-            }
-            const float3 n = ex::normalize(h.normal);
-            const float3 view = ex::normalize(-ray.direction);
-            float3 color;
-            float4 albedo;
-            if (!kInteractive) {  // :4824-4834
-                const float3 key = ex::normalize(f3(0.35f, 0.72f, 0.58f));
-                float lambert = fmaxf(ex::dot(n, key), 0.0f);
-                float facing = fmaxf(ex::dot(n, view), 0.0f);
-                float rim = ex::mul(powf(ex::sub(1.0f, facing), 2.0f), 0.08f);
-                float shade = ex::add(ex::add(0.32f, ex::mul(0.68f, lambert)), rim);
-                color = ex::add(ex::mul(mx(xyz(m.baseColor), f3(0.0f)), shade), mx(xyz(m.emission), f3(0.0f)));
-                beauty = make_float4(color.x, color.y, color.z,
-                                     P.transparent_background ? clampf(m.baseColor.w, 0.0f, 1.0f) : 1.0f);
-                albedo = m.baseColor;
-            } else {  // :4961-5133
-                const float roughness = clampf(m.parameters.x, 0.02f, 1.0f);
-                const float metallic = clampf(m.parameters.y, 0.0f, 1.0f);
-                const float opacity = clampf(m.baseColor.w, 0.0f, 1.0f);
-                const float3 base = mx(xyz(m.baseColor), f3(0.0f));
-                color = mx(xyz(m.emission), f3(0.0f));
-                ShadePoint sp;
-                makeShadePoint(sp, m, n, h.tangent, h.bitangent, view);
-                const uint32_t nl = min(S.light_count, 12u);
-#pragma unroll 1
-                for (uint32_t l = 0; l < nl; ++l) {
-                    const dk_light_record& L = S.lights[l];
-                    if (L.triangle_index >= S.tri_count || L.material_index >= S.mat_count) continue;
-                    const dk_triangle& lt = S.tris[L.triangle_index];
-                    float3 emission = mx(xyz(__ldg(reinterpret_cast<const float4*>(S.mats + L.material_index) + 1)),
-                                         f3(0.0f));
-                    if (maxComponent(emission) <= 0.0f || L.area <= 0.0f) continue;
-                    float3 lp = (f3(lt.v0.x, lt.v0.y, lt.v0.z) + f3(lt.v1.x, lt.v1.y, lt.v1.z) +
-                                 f3(lt.v2.x, lt.v2.y, lt.v2.z)) / 3.0f;
-                    float3 toL = lp - h.position;
-                    float d2 = fmaxf(dot(toL, toL), 1e-5f);
-                    float dist = sqrtf(d2);
-                    float3 ld = toL / dist;
-                    float cosS = fmaxf(dot(n, ld), 0.0f);
-                    float cosL = fmaxf(dot(f3(L.normal.x, L.normal.y, L.normal.z), -ld), 0.0f);
-                    if (cosS <= 0.0f || cosL <= 0.0f) continue;
-                    float3 T = f3(1.0f);
-                    float3 so = h.position + n * 0.001f;
-                    if (!S.volume_count) sdfCount(S.sdf_counters, kSdfShadowSceneQueries);
-                    bool occluded = S.volume_count ? shadowWalk(S, mt, so, ld, dist - 0.002f, T)
-                                                   : shadowLayers(S, mt, opaqueMask, so, ld, dist - 0.002f, T);
-                    if (occluded) continue;
-                    float3 brdf = evalBRDF(m, sp, ld);
-                    float ccGloss = materialClearcoat(m) * powf(1.0f - materialClearcoatRoughness(m), 2.0f);
-                    float glossW = clampf(metallic + ccGloss +
-                                              (1.0f - metallic) * powf(1.0f - roughness, 4.0f) *
-                                                  clampf(m.parameters2.x, 0.0f, 1.0f),
-                                          0.0f, 1.0f);
-                    float3 f0 = materialF0(m);
-                    float3 diffuseOnly = (1.0f - metallic) * base * mx(f3(0.0f), f3(1.0f) - f0) * 0.31830988618f;
-                    brdf = mix3(diffuseOnly, brdf, glossW);
-                    float G = cosS * cosL * L.area / d2;
-                    color += brdf * emission * G * T;
-                }
-                float3 envDiffuse = interactiveDiffuseEnv(S, n);
-                float3 refl = normalize(reflect(-view, n));
-                float3 baseRefl = interactiveSpecularEnv(S, refl, n, roughness);
-                float ccRough = materialClearcoatRoughness(m);
-                float3 ccRefl = interactiveSpecularEnv(S, refl, n, ccRough);
-                float nDotV = fmaxf(dot(n, view), 0.0f);
-                float3 fresnel = fresnelSchlickThinFilm(nDotV, materialF0(m), m);
-                float glossy = powf(1.0f - roughness, 4.0f);
-                float metalW = metallic * powf(1.0f - roughness, 2.0f);
-                float ccW = materialClearcoat(m) * powf(1.0f - ccRough, 3.0f);
-                float dielectricW = (1.0f - metallic) * glossy * clampf(m.parameters2.x, 0.0f, 1.0f);
-                float3 roughFresnel = mix3(fresnel, materialF0(m), smoothstepf(0.45f, 0.95f, roughness));
-                float3 ccFresnel = fresnelSchlickThinFilm(nDotV, materialClearcoatF0Color(m), m);
-                float horizon = 0.58f + 0.42f * clampf(n.y * 0.5f + 0.5f, 0.0f, 1.0f);
-                float contact = interactiveContactAO(S, mt, h, m, n);
-                float diffuseStrength = 0.58f * (1.0f - metallic) * (horizon * contact);
-                float baseReflStrength = metalW * 1.05f + dielectricW * 0.32f;
-                color += base * envDiffuse * diffuseStrength;
-                color += baseRefl * roughFresnel * baseReflStrength;
-                color += ccRefl * ccFresnel * ccW * 0.42f;
-                const float3 key = normalize(f3(-0.32f, 0.78f, 0.52f));
-                color += base * (1.0f - metallic) * fmaxf(dot(n, key), 0.0f) * 0.16f * contact;
-                float subsurface = materialSubsurface(m);
-                if (subsurface > 0.0f) {
-                    float wrap = powf(1.0f - nDotV, 2.0f);
-                    color += clamp3(xyz(m.subsurfaceColor), f3(0.0f), f3(0.999f)) * base * envDiffuse * subsurface *
-                             (0.12f + 0.22f * wrap) * contact;
-                }
-                float transmission = materialTransmission(m);
-                if (transmission > 0.0f) {
-                    float3 transmitted = sampleEnvironment(S, ray.direction);
-                    color = mix3(color, transmitted * materialTransmissionTint(m, 0.65f), transmission * 0.55f);
-                    color += baseRefl * fresnel * transmission * 0.35f;
-                }
-                color = clamp3(color, f3(0.0f), f3(fmaxf(P.clamp, 1.0f)));
-                beauty = make_float4(color.x, color.y, color.z, P.transparent_background ? opacity : 1.0f);
-                albedo = make_float4(base.x, base.y, base.z, opacity);
-            }
-            const float3 enc = ex::add(ex::mul(n, 0.5f), f3(0.5f));
-            const float mid = (float)(h.materialID + 1u), oid = (float)(h.objectID + 1u);
-            A.aov[0 * plane + pix] = make_float4(h.t, h.t, h.t, 1.0f);
-            A.aov[1 * plane + pix] = make_float4(enc.x, enc.y, enc.z, 1.0f);
-            A.aov[2 * plane + pix] = albedo;
-            A.aov[3 * plane + pix] = make_float4(mid, mid, mid, 1.0f);
-            A.aov[4 * plane + pix] = make_float4(oid, oid, oid, 1.0f);
-            float2 cur, prev;
-            if (projectToScreen(P.cam, h.position, P.width, P.height, cur) &&
-                projectToScreen(P.prev_cam, h.position, P.width, P.height, prev))
-                A.aov[5 * plane + pix] = make_float4(ex::sub(prev.x, cur.x), ex::sub(prev.y, cur.y), 0.0f, 1.0f);
-            else
-                A.aov[5 * plane + pix] = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
-        }
-        A.sum[pix] = beauty;
-        A.comp[pix] = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
-        A.resolved[pix] = D4{0.0, 0.0, 0.0, 0.0};
-        A.count[pix] = 1u;
+        rec = traceSceneCounting(S, ray.origin, ray.direction);
     }
+    const bool hit = rec.tri != kNoHit;
+    __shared__ uint32_t firstHit;
+    __shared__ HitRec sharedHit;
+    if (threadIdx.x == 0) firstHit = 0xffffffffu;
+    __syncthreads();
+    if (hit) atomicMin(&firstHit, threadIdx.x);
+    __syncthreads();
+    if (threadIdx.x == firstHit) sharedHit = rec;
+    __syncthreads();
+    if (valid && !hit) {
+        float alpha = P.transparent_background ? 0.0f : 1.0f;
+        float3 color = mx(f3(P.bg[0], P.bg[1], P.bg[2]), f3(0.0f));
+        if (!P.transparent_background && P.shows_env_bg) color = sampleEnvironmentCall(S, ray.direction);
+        A.aov[0 * plane + pix] = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+        A.aov[1 * plane + pix] = make_float4(0.5f, 0.5f, 0.5f, 0.0f);
+        for (int k = 2; k < 6; ++k) A.aov[k * plane + pix] = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+        storePreview(A, pix, make_float4(color.x, color.y, color.z, alpha));
+    }
+    if (firstHit == 0xffffffffu) return;
+    if (!hit) rec = sharedHit;
+
+    Hit h = makeHitAny(S, ray, rec);
+    Material m = materialForHit(S, mt, h);
+    float4 beauty, albedo;
+    float3 color;
+    uint32_t nIdx = (uint32_t)m.parameters.w;
+    if (nIdx != 0u) h = applyNormalMap(S, h, nIdx, ray.direction);
+    uint32_t bIdx = (uint32_t)m.parameters.z;
+    if (bIdx != 0u) {  // applyBaseColorTexture
+        float4 t = sampleTexture(S, bIdx, h.uv, make_float4(1.0f, 1.0f, 1.0f, 1.0f));
+        m.baseColor = make_float4(ex::mul(m.baseColor.x, t.x), ex::mul(m.baseColor.y, t.y),
+                                  ex::mul(m.baseColor.z, t.z), ex::mul(m.baseColor.w, t.w));
+    }
+    const float3 n = ex::normalize(h.normal);
+    const float3 view = ex::normalize(-ray.direction);
+    if constexpr (!kInteractive) {  // :4824-4834
+        const float3 key = ex::normalize(f3(0.35f, 0.72f, 0.58f));
+        float lambert = fmaxf(ex::dot(n, key), 0.0f);
+        float facing = fmaxf(ex::dot(n, view), 0.0f);
+        float rim = ex::mul(powf(ex::sub(1.0f, facing), 2.0f), 0.08f);
+        float shade = ex::add(ex::add(0.32f, ex::mul(0.68f, lambert)), rim);
+        color = ex::add(ex::mul(mx(xyz(m.baseColor), f3(0.0f)), shade), mx(xyz(m.emission), f3(0.0f)));
+        beauty = make_float4(color.x, color.y, color.z,
+                             P.transparent_background ? clampf(m.baseColor.w, 0.0f, 1.0f) : 1.0f);
+        albedo = m.baseColor;
+    } else {  // :4961-5133
+        const float roughness = clampf(m.parameters.x, 0.02f, 1.0f);
+        const float metallic = clampf(m.parameters.y, 0.0f, 1.0f);
+        const float opacity = clampf(m.baseColor.w, 0.0f, 1.0f);
+        const float3 base = mx(xyz(m.baseColor), f3(0.0f));
+        color = mx(xyz(m.emission), f3(0.0f));
+        ShadePoint sp;
+        makeShadePoint(sp, m, n, h.tangent, h.bitangent, view);
+        const uint32_t nl = min(S.light_count, 12u);
+#pragma unroll 1
+        for (uint32_t l = 0; l < nl; ++l) {
+            __syncthreads();
+            const dk_light_record& L = S.lights[l];
+            if (L.triangle_index >= S.tri_count || L.material_index >= S.mat_count) continue;
+            const dk_triangle& lt = S.tris[L.triangle_index];
+            float3 emission = mx(xyz(__ldg(reinterpret_cast<const float4*>(S.mats + L.material_index) + 1)), f3(0.0f));
+            if (!hit || maxComponent(emission) <= 0.0f || L.area <= 0.0f) continue;
+            float3 lp = (f3(lt.v0.x, lt.v0.y, lt.v0.z) + f3(lt.v1.x, lt.v1.y, lt.v1.z) +
+                         f3(lt.v2.x, lt.v2.y, lt.v2.z)) / 3.0f;
+            float3 toL = lp - h.position;
+            float d2 = fmaxf(dot(toL, toL), 1e-5f);
+            float dist = sqrtf(d2);
+            float3 ld = toL / dist;
+            float cosS = fmaxf(dot(n, ld), 0.0f);
+            float cosL = fmaxf(dot(f3(L.normal.x, L.normal.y, L.normal.z), -ld), 0.0f);
+            if (cosS <= 0.0f || cosL <= 0.0f) continue;
+            float3 T = f3(1.0f);
+            float3 so = h.position + n * 0.001f;
+            if (!S.volume_count) sdfCount(S.sdf_counters, kSdfShadowSceneQueries);
+            bool occluded = S.volume_count ? shadowWalk(S, mt, so, ld, dist - 0.002f, T)
+                                           : shadowLayers(S, mt, opaqueMask, so, ld, dist - 0.002f, T);
+            if (occluded) continue;
+            float3 brdf = evalBRDF(m, sp, ld);
+            float ccGloss = materialClearcoat(m) * powf(1.0f - materialClearcoatRoughness(m), 2.0f);
+            float glossW = clampf(metallic + ccGloss +
+                                      (1.0f - metallic) * powf(1.0f - roughness, 4.0f) *
+                                          clampf(m.parameters2.x, 0.0f, 1.0f),
+                                  0.0f, 1.0f);
+            float3 f0 = materialF0(m);
+            float3 diffuseOnly = (1.0f - metallic) * base * mx(f3(0.0f), f3(1.0f) - f0) * 0.31830988618f;
+            brdf = mix3(diffuseOnly, brdf, glossW);
+            float G = cosS * cosL * L.area / d2;
+            color += brdf * emission * G * T;
+        }
+        __syncthreads();
+        float3 envDiffuse = interactiveDiffuseEnv(axisEnv, n);
+        float3 refl = normalize(reflect(-view, n));
+        float3 baseRefl = interactiveSpecularEnv(S, refl, n, roughness, envDiffuse);
+        float ccRough = materialClearcoatRoughness(m);
+        float3 ccRefl = interactiveSpecularEnv(S, refl, n, ccRough, envDiffuse);
+        float nDotV = fmaxf(dot(n, view), 0.0f);
+        float3 fresnel = fresnelSchlickThinFilm(nDotV, materialF0(m), m);
+        float glossy = powf(1.0f - roughness, 4.0f);
+        float metalW = metallic * powf(1.0f - roughness, 2.0f);
+        float ccW = materialClearcoat(m) * powf(1.0f - ccRough, 3.0f);
+        float dielectricW = (1.0f - metallic) * glossy * clampf(m.parameters2.x, 0.0f, 1.0f);
+        float3 roughFresnel = mix3(fresnel, materialF0(m), smoothstepf(0.45f, 0.95f, roughness));
+        float3 ccFresnel = fresnelSchlickThinFilm(nDotV, materialClearcoatF0Color(m), m);
+        float horizon = 0.58f + 0.42f * clampf(n.y * 0.5f + 0.5f, 0.0f, 1.0f);
+        float contact = interactiveContactAO(S, mt, hit, h, m, n);
+        float diffuseStrength = 0.58f * (1.0f - metallic) * (horizon * contact);
+        float baseReflStrength = metalW * 1.05f + dielectricW * 0.32f;
+        color += base * envDiffuse * diffuseStrength;
+        color += baseRefl * roughFresnel * baseReflStrength;
+        color += ccRefl * ccFresnel * ccW * 0.42f;
+        const float3 key = normalize(f3(-0.32f, 0.78f, 0.52f));
+        color += base * (1.0f - metallic) * fmaxf(dot(n, key), 0.0f) * 0.16f * contact;
+        float subsurface = materialSubsurface(m);
+        if (subsurface > 0.0f) {
+            float wrap = powf(1.0f - nDotV, 2.0f);
+            color += clamp3(xyz(m.subsurfaceColor), f3(0.0f), f3(0.999f)) * base * envDiffuse * subsurface *
+                     (0.12f + 0.22f * wrap) * contact;
+        }
+        float transmission = materialTransmission(m);
+        if (transmission > 0.0f) {
+            float3 transmitted = sampleEnvironmentCall(S, ray.direction);
+            color = mix3(color, transmitted * materialTransmissionTint(m, 0.65f), transmission * 0.55f);
+            color += baseRefl * fresnel * transmission * 0.35f;
+        }
+        color = clamp3(color, f3(0.0f), f3(fmaxf(P.clamp, 1.0f)));
+        beauty = make_float4(color.x, color.y, color.z, P.transparent_background ? opacity : 1.0f);
+        albedo = make_float4(base.x, base.y, base.z, opacity);
+    }
+    if (!hit) return;
+    const float3 enc = ex::add(ex::mul(n, 0.5f), f3(0.5f));
+    const float mid = (float)(h.materialID + 1u), oid = (float)(h.objectID + 1u);
+    A.aov[0 * plane + pix] = make_float4(h.t, h.t, h.t, 1.0f);
+    A.aov[1 * plane + pix] = make_float4(enc.x, enc.y, enc.z, 1.0f);
+    A.aov[2 * plane + pix] = albedo;
+    A.aov[3 * plane + pix] = make_float4(mid, mid, mid, 1.0f);
+    A.aov[4 * plane + pix] = make_float4(oid, oid, oid, 1.0f);
+    float2 cur, prev;
+    if (projectToScreen(P.cam, h.position, P.width, P.height, cur) &&
+        projectToScreen(P.prev_cam, h.position, P.width, P.height, prev))
+        A.aov[5 * plane + pix] = make_float4(ex::sub(prev.x, cur.x), ex::sub(prev.y, cur.y), 0.0f, 1.0f);
+    else
+        A.aov[5 * plane + pix] = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+    storePreview(A, pix, beauty);
 }
 
 // Kahan-compensated accumulation of every path of the batch into its pixel,
@@ -1844,12 +1915,15 @@ cudaError_t launchAovPrimary(const DevScene& S, const Wave& W, int grid, cudaStr
     return cudaGetLastError();
 }
 cudaError_t launchPreview(const DevScene& S, const DevParams& P, const Accum& A, uint32_t matCount,
-                          uint32_t opaqueMask, bool interactive, int grid, cudaStream_t st) {
+                          uint32_t opaqueMask, bool interactive, cudaStream_t st) {
     const MatTable mt{0u, matCount};
+    const uint64_t warps = (uint64_t)((P.tile_w + 7u) / 8u) * ((P.tile_h + 3u) / 4u);
+    const uint32_t grid = (uint32_t)((warps * 32u + DK_PREVIEW_BLOCK - 1u) / DK_PREVIEW_BLOCK);
+    if (!grid) return cudaSuccess;
     if (interactive)
-        k_preview<true><<<grid, 128, 0, st>>>(S, P, A, mt, opaqueMask);
+        k_preview<true><<<grid, DK_PREVIEW_BLOCK, 0, st>>>(S, P, A, mt, opaqueMask);
     else
-        k_preview<false><<<grid, 128, 0, st>>>(S, P, A, mt, opaqueMask);
+        k_preview<false><<<grid, DK_PREVIEW_BLOCK, 0, st>>>(S, P, A, mt, opaqueMask);
     return cudaGetLastError();
 }
 cudaError_t launchFinalize(const Wave& W, int grid, cudaStream_t st) {
