@@ -13,6 +13,7 @@
 //               (sampleDirectLighting, :4407-4585; shadowOccluded, :4196-4274)
 //   k_finalize  Kahan-compensated accumulation + last-sample AOVs (:5520-5585)
 // Surviving paths are compacted into the next queue with warp-ballot appends.
+#include <algorithm>
 #include <cstdio>
 #include <cstdlib>
 #include <type_traits>
@@ -917,19 +918,35 @@ __device__ ShadeOut shadePath(const DevScene& S, const Wave& W, uint32_t p, uint
     return out;
 }
 
-#ifndef DK_SHADE_MIN_BLOCKS
-#define DK_SHADE_MIN_BLOCKS 4
+// Shading is bound by load latency and, at 200 to 500 KB of code, by
+// instruction fetch.  A barrier per path keeps a block's warps near each other
+// in the code, so that a fetched line serves all of them: on the large scene
+// 66.4 -> 62.4 ms a frame (1920 x 1080, 16 spp) with blocks of 128 or 256
+// threads, 63.8 with 512; without the barrier block size makes no difference.
+// The kernels with the subsurface walk keep 128 threads (the walk's lengths
+// differ), the one for volumes and the 8-wide tree no barrier either (24.4 ->
+// 25.1 ms a frame with it).
+#ifndef DK_SHADE_BLOCK
+#define DK_SHADE_BLOCK 256
 #endif
+#ifndef DK_SHADE_WARPS
+#define DK_SHADE_WARPS 16
+#endif
+template <bool kSss>
+constexpr int shadeBlock() { return kSss ? 128 : DK_SHADE_BLOCK; }
 // range 0: the whole queue; 1: the sorted queue before the subsurface bucket;
 // 2: from it on.
 template <bool kVolumes, bool kSss>
-__global__ void __launch_bounds__(128, DK_SHADE_MIN_BLOCKS) k_shade(DevScene S, Wave W, uint32_t bounce, uint32_t sel,
-                                                                  uint32_t sorted, uint32_t range) {
+__global__ void __launch_bounds__(shadeBlock<kSss>(), DK_SHADE_WARPS * 32 / shadeBlock<kSss>())
+    k_shade(DevScene S, Wave W, uint32_t bounce, uint32_t sel, uint32_t sorted, uint32_t range) {
     const uint32_t* q = sorted ? W.qsorted : W.q[sel];
     const uint32_t n = W.counts[sel];
     const uint32_t begin = range == 2u ? W.counts[7] : 0u, end = range == 1u ? W.counts[7] : n;
     if (globalId() == 0) W.counts[4] = 0u;  // extend cursor of the next bounce
-    for (uint32_t i = begin + globalId(); i < end; i += gridStride()) {
+    for (uint32_t base = begin + blockIdx.x * blockDim.x; base < end; base += gridStride()) {
+        const uint32_t i = base + threadIdx.x;
+        if (!kVolumes) __syncthreads();
+        if (i >= end) continue;
         uint32_t p = q[i];
         ShadeOut o = shadePath<kVolumes, kSss>(S, W, p, i, bounce);
         bool keep = o.survive && bounce + 1u < o.maxBounces;
@@ -1799,7 +1816,9 @@ int kernelGrid(int which, int smCount) {
     switch (which) {
         case 0: cudaOccupancyMaxActiveBlocksPerMultiprocessor(&perSM, k_generate, 256, 0); break;
         case 1: cudaOccupancyMaxActiveBlocksPerMultiprocessor(&perSM, k_extend<false>, 128, 0); break;
-        case 2: cudaOccupancyMaxActiveBlocksPerMultiprocessor(&perSM, k_shade<false, false>, 128, 0); break;
+        case 2:
+            cudaOccupancyMaxActiveBlocksPerMultiprocessor(&perSM, k_shade<false, false>, shadeBlock<false>(), 0);
+            break;
         case 3: cudaOccupancyMaxActiveBlocksPerMultiprocessor(&perSM, k_shadow_rays<false>, 128, 0); break;
         case 5: cudaOccupancyMaxActiveBlocksPerMultiprocessor(&perSM, k_extend<true>, 128, 0); break;
         case 6: cudaOccupancyMaxActiveBlocksPerMultiprocessor(&perSM, k_shadow_rays<true>, 128, 0); break;
@@ -1868,21 +1887,23 @@ cudaError_t launchShade(const DevScene& S, const Wave& W, uint32_t bounce, uint3
     }
     uint32_t sorted = (uint32_t)g_sortMaterials;
     if (sorted) {
-        k_sort_count<<<grid, 256, 0, st>>>(S, W, sel);
+        const uint32_t sortBlocks = (W.path_count + 256u * kSortItems - 1u) / (256u * kSortItems);
+        k_sort_count<<<std::min((uint32_t)grid, sortBlocks), 256, 0, st>>>(S, W, sel);
         k_sort_scan<<<1, kSortBins, 0, st>>>(W);
-        k_sort_scatter<<<(W.cap + 256u * kSortItems - 1u) / (256u * kSortItems), 256, 0, st>>>(W, sel);
+        k_sort_scatter<<<sortBlocks, 256, 0, st>>>(W, sel);
     }
+    const int sssGrid = std::max(1, grid * shadeBlock<false>() / shadeBlock<true>());
     // The general shading kernel (volume hits, random walks through
     // traceScene) also serves the 8-wide tree, keeping the layout switch out
     // of the triangle-only kernel.
     if (S.volume_count || S.wide8) {
-        k_shade<true, true><<<grid, 128, 0, st>>>(S, W, bounce, sel, sorted, 0u);
+        k_shade<true, true><<<sssGrid, shadeBlock<true>(), 0, st>>>(S, W, bounce, sel, sorted, 0u);
     } else if (sorted) {
         // materials without a subsurface weight, then those with one
-        k_shade<false, false><<<grid, 128, 0, st>>>(S, W, bounce, sel, sorted, 1u);
-        k_shade<false, true><<<grid, 128, 0, st>>>(S, W, bounce, sel, sorted, 2u);
+        k_shade<false, false><<<grid, shadeBlock<false>(), 0, st>>>(S, W, bounce, sel, sorted, 1u);
+        k_shade<false, true><<<sssGrid, shadeBlock<true>(), 0, st>>>(S, W, bounce, sel, sorted, 2u);
     } else {
-        k_shade<false, true><<<grid, 128, 0, st>>>(S, W, bounce, sel, sorted, 0u);
+        k_shade<false, true><<<sssGrid, shadeBlock<true>(), 0, st>>>(S, W, bounce, sel, sorted, 0u);
     }
     // The survivors, in path order, are the next bounce's queue.
     const uint32_t blocks = (W.path_count + kLiveBlock - 1u) / kLiveBlock;
