@@ -237,7 +237,7 @@ int kernelGrid(int which, int smCount);
 Grids kernelGrids() {
     int sm = g_prop.multiProcessorCount;
     return Grids{kernelGrid(0, sm), kernelGrid(1, sm), kernelGrid(2, sm), kernelGrid(3, sm), kernelGrid(4, sm),
-                 kernelGrid(5, sm), kernelGrid(6, sm), kernelGrid(7, sm)};
+                 kernelGrid(5, sm), kernelGrid(6, sm), kernelGrid(7, sm), kernelGrid(8, sm)};
 }
 
 bool materialBlocksShadow(const dk_material& m) {
@@ -523,6 +523,9 @@ int uploadScene(Arena& arena, const dk_scene* sc, DevScene& D, uint32_t material
 #undef TRY
     D.tri_count = sc->triangle_count;
     D.mat_count = sc->material_count;
+    D.has_subsurface = 0u;
+    for (uint32_t i = 0; i < sc->material_count; ++i)
+        if (sc->materials[i].subsurface_color.w > 0.0f) D.has_subsurface = 1u;
     D.texdesc_count = sc->texture_descriptor_count;
     D.light_count = sc->lights ? sc->light_count : 0;
     D.env_count = sc->environment_samples ? sc->environment_sample_count : 0;
@@ -638,7 +641,7 @@ int launchWave(const DevScene& S, const Wave& W, uint32_t maxBounces, bool anyDe
         MARK(1);
         DK_CUDA(launchExtend(S, W, sel, b, S.wide8 ? g.extend8 : g.extend, g.volume, q), "extend launch");
         MARK(2);
-        DK_CUDA(launchShade(S, W, b, sel, g.shade, q), "shade launch");
+        DK_CUDA(launchShade(S, W, b, sel, g.shade, g.walk, q), "shade launch");
         MARK(3);
         DK_CUDA(launchShadow(S, W, S.wide8 ? g.shadow8 : g.shadow, q), "shadow launch");
         DK_CUDA(launchResolve(W, g.final, q), "resolve launch");

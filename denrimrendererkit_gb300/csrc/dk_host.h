@@ -97,6 +97,7 @@ struct Grids {
     int gen, extend, shade, shadow, final;
     int extend8, shadow8;  // the traversal kernels over the 8-wide tree
     int volume;            // the distance-volume pass (persistent: its resident blocks)
+    int walk;              // the subsurface walk
 };
 Grids kernelGrids();
 

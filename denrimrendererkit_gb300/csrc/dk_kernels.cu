@@ -231,8 +231,9 @@ __device__ __forceinline__ float subsurfaceBoundaryPDF(float3 s, float d) {
     return fmaxf((tr.x + tr.y + tr.z) * 0.33333333333f, 1e-6f);
 }
 
-// continueSubsurfaceRandomWalk (PathTrace.metal:3525-3621).
-template <bool kVolumes>
+// continueSubsurfaceRandomWalk (PathTrace.metal:3525-3621) inside the shading
+// kernel, for scenes with volumes and the 8-wide tree; the others run
+// k_subsurface_walk before shading.
 __device__ bool continueSubsurfaceRandomWalk(const DevScene& S, const Hit& entry, const Material& m, Ray& ray,
                                              float3& tp, float& prevPdf, uint32_t& state) {
     if (materialSubsurface(m) <= 0.0f || !entry.frontFacing) return false;
@@ -245,7 +246,7 @@ __device__ bool continueSubsurfaceRandomWalk(const DevScene& S, const Hit& entry
     float anisotropy = clampf(m.subsurfaceParameters.x, -0.95f, 0.95f);
     for (uint32_t step = 0u; step < 8u; ++step) {
         sdfCount(S.sdf_counters, kSdfBounceSceneQueries);
-        HitRec r = kVolumes ? traceScene(S, medium.origin, medium.direction) : traceClosest(S, medium.origin, medium.direction);
+        HitRec r = traceScene(S, medium.origin, medium.direction);
         if (r.tri == kNoHit) return false;
         float f0 = randomFloat(state);
         float f1 = randomFloat(state);
@@ -260,7 +261,7 @@ __device__ bool continueSubsurfaceRandomWalk(const DevScene& S, const Hit& entry
             if (maxComponent(tp) <= 1e-4f) return false;
             continue;
         }
-        Hit b = kVolumes ? makeHitAny(S, medium, r) : makeHit(S, medium, r);
+        Hit b = makeHitAny(S, medium, r);
         float3 exitNormal = normalize(b.frontFacing ? b.normal : -b.normal);
         float x0 = randomFloat(state);
         float x1 = randomFloat(state);
@@ -429,7 +430,14 @@ constexpr uint32_t kNoWork = 0xffffffffu;
 #ifndef DK_STEP_BUDGET
 #define DK_STEP_BUDGET 16
 #endif
-constexpr int kStepBudget = DK_STEP_BUDGET;
+constexpr int kStepBudget = DK_STEP_BUDGET;  // the 8-wide tree's visits between refills
+// Idle lanes are refilled when fewer than this many of a warp's are running
+// (8 / 12 / 16 / 24 / 28: 58.6 / 57.7 / 57.5 / 61.1 / 63.6 ms a frame, large
+// scene at 16 spp).
+#ifndef DK_REFILL_BELOW
+#define DK_REFILL_BELOW 16
+#endif
+constexpr int kRefillBelow = DK_REFILL_BELOW;
 
 // Refills the lanes that asked for work with consecutive items of a queue of
 // length `n` through one atomic per warp; returns this lane's item or kNoWork.
@@ -491,16 +499,24 @@ __global__ void __launch_bounds__(128) k_extend(DevScene S, Wave W, uint32_t sel
             }
         }
         if (__all_sync(0xffffffffu, p == kNoWork && exhausted)) break;
-        bool done = false;
-        if (p != kNoWork) {
-            if constexpr (kWide8)
-                done = closestSteps(S, st, stack8, kStepBudget);
-            else
-                done = closestSteps(S, st, stackNode, stackT, kStepBudget);
-        }
-        if (done) {
-            W.hit[p] = make_float4(st.bestT, __uint_as_float(st.bestTri), st.bu, st.bv);
-            p = kNoWork;
+        if constexpr (kWide8) {
+            if (p != kNoWork && closestSteps(S, st, stack8, kStepBudget)) {
+                W.hit[p] = make_float4(st.bestT, __uint_as_float(st.bestTri), st.bu, st.bv);
+                p = kNoWork;
+            }
+        } else {
+            const int least = __any_sync(0xffffffffu, exhausted) ? 1 : kRefillBelow;
+            for (;;) {
+                int running;
+                const bool nodes = majorityStep(p != kNoWork, st.node, running);
+                if (running < least) break;
+                const bool leaf = (st.node & kLeafBit) != 0u;
+                if (p == kNoWork || nodes == leaf) continue;
+                if (!(leaf ? closestTriStep(S, st, stackNode, stackT) : closestNodeStep(S, st, stackNode, stackT))) {
+                    W.hit[p] = make_float4(st.bestT, __uint_as_float(st.bestTri), st.bu, st.bv);
+                    p = kNoWork;
+                }
+            }
         }
     }
 }
@@ -564,28 +580,31 @@ __global__ void __launch_bounds__(kSortBins) k_sort_scan(Wave W) {
     if (t == kSubsurfaceKey) W.counts[7] = v[t] - x;  // shading-order index of the first subsurface path
 }
 
-// Block b places queue entries [b * 2048, b * 2048 + 2048) stably: an entry's
+// Block b places its kItems x 256 queue entries stably: an entry's
 // rank among the block's entries of its key follows queue order (in-warp
 // ranks from __match_any_sync, warp offsets per key scanned in shared memory,
-// eight rounds of 256 entries in order), and one global reservation per
+// kItems rounds of 256 entries in order), and one global reservation per
 // (block, key) places the block's run.  The queue is in path order, so every
 // run of a key holds increasing path indices -- neighbouring lanes of the
 // shading kernel read neighbouring path state.
-constexpr uint32_t kSortItems = 8;
+// kItems: 8 in large waves; 2 in waves of less than kSortSmall paths, whose few
+// blocks would spend their time in the rounds.
+constexpr uint32_t kSortSmall = 1u << 22;
+template <uint32_t kItems>
 __global__ void __launch_bounds__(256) k_sort_scatter(Wave W, uint32_t sel) {
     __shared__ uint32_t cnt[kSortBins];
     __shared__ uint32_t base[kSortBins];
     __shared__ uint32_t warpCnt[8][kSortBins];
     const uint32_t* q = W.q[sel];
     const uint32_t n = W.counts[sel];
-    const uint32_t start = blockIdx.x * 256u * kSortItems;
+    const uint32_t start = blockIdx.x * 256u * kItems;
     if (start >= n) return;  // uniform over the block
     const uint32_t tid = threadIdx.x, lane = tid & 31u, warp = tid >> 5;
     const uint32_t lanesBelow = (1u << lane) - 1u;
     cnt[tid] = 0u;  // kSortBins == blockDim.x
-    uint32_t key[kSortItems], rank[kSortItems];
+    uint32_t key[kItems], rank[kItems];
 #pragma unroll
-    for (uint32_t k = 0; k < kSortItems; ++k) {
+    for (uint32_t k = 0; k < kItems; ++k) {
 #pragma unroll
         for (uint32_t w = 0; w < 8u; ++w) warpCnt[w][tid] = 0u;
         __syncthreads();
@@ -613,7 +632,7 @@ __global__ void __launch_bounds__(256) k_sort_scatter(Wave W, uint32_t sel) {
     if (cnt[tid]) base[tid] = atomicAdd(&W.bins[tid], cnt[tid]);
     __syncthreads();
 #pragma unroll
-    for (uint32_t k = 0; k < kSortItems; ++k) {
+    for (uint32_t k = 0; k < kItems; ++k) {
         uint32_t i = start + k * 256u + tid;
         if (i < n) W.qsorted[base[key[k]] + rank[k]] = q[i];
     }
@@ -702,15 +721,135 @@ __global__ void __launch_bounds__(256) k_live_scatter(Wave W, uint32_t sel) {
     }
 }
 
+// ------------------------------------------------ subsurface walk ----
+// continueSubsurfaceRandomWalk (PathTrace.metal:3525-3621) for the paths whose
+// material has a subsurface weight, ahead of the shading kernel: up to eight
+// rays inside the surface per path.  Persistent threads with per-lane refill,
+// like k_extend: a lane advances its ray a bounded number of visits, and when
+// the ray is done scatters, leaves or fetches the next path while its
+// neighbours go on.  Inside the shading kernel the same walks kept 5.8 of a
+// warp's 32 lanes busy and took 102 of the 159 ms of a 20-job serving mix whose
+// largest image has such a material; with this kernel the mix takes 67 ms.
+// The outcome goes to the path's NEE slots, which shading reads before it
+// fills them: origin and outcome, direction and RNG state, throughput and pdf.
+constexpr uint32_t kWalkNone = 0u;  // not entered: the weight's draw decided against it, or a back face
+constexpr uint32_t kWalkExit = 1u;  // left the surface: the path goes on from there
+constexpr uint32_t kWalkLost = 2u;  // absorbed, or no surface found: shading goes on with the state so far
+__global__ void __launch_bounds__(128) k_subsurface_walk(DevScene S, Wave W, uint32_t sel, uint32_t sorted) {
+    const uint32_t* q = sorted ? W.qsorted : W.q[sel];
+    const uint32_t begin = sorted ? W.counts[7] : 0u, n = W.counts[sel] - begin;
+    int stackNode[kStackSize];
+    float stackT[kStackSize];
+    ClosestState st;
+    uint32_t i = kNoWork, state = 0u, mat = 0u, step = 0u;
+    float3 tp = f3(0.0f);
+    bool exhausted = false;
+    for (;;) {
+        uint32_t idx = warpFetch(&W.counts[8], n, i == kNoWork && !exhausted, exhausted);
+        if (idx != kNoWork) {
+            const uint32_t at = begin + idx, p = q[at];
+            const float4 hr = W.hit[p];
+            const uint32_t tri = __float_as_uint(hr.y);
+            if (tri != kNoHit) {
+                const uint2 rs = W.rng[p];
+                const MatTable mt = matTable(W.jobs[rs.y >> 8]);
+                const float4 ro = W.ray_o[p], rd = W.ray_d[p];
+                const Ray ray{xyz(ro), xyz(rd)};
+                Hit h = makeHit(S, ray, HitRec{hr.x, tri, hr.z, hr.w});
+                mat = mt.base + min(h.materialID, mt.count - 1u);
+                const Material m = loadMaterial(S.mats, mat);
+                const float subsurface = materialSubsurface(m);
+                if (subsurface > 0.0f) {
+                    const uint32_t nIdx = (uint32_t)m.parameters.w, bIdx = (uint32_t)m.parameters.z;
+                    if (nIdx != 0u) h = applyNormalMap(S, h, nIdx, ray.direction);
+                    float alpha = m.baseColor.w;
+                    if (bIdx != 0u)
+                        alpha = ex::mul(alpha, sampleTexture(S, bIdx, h.uv, make_float4(1.0f, 1.0f, 1.0f, 1.0f)).w);
+                    state = rs.x;
+                    if (alpha <= 0.001f || !h.frontFacing || !(randomFloat(state) < subsurface)) {
+                        W.nee_o[at] = make_float4(0.0f, 0.0f, 0.0f, __uint_as_float(kWalkNone));
+                    } else {
+                        float e0 = randomFloat(state);
+                        float e1 = randomFloat(state);
+                        float3 entryDir = orientHemisphere(cosineHemisphere(e0, e1), -h.normal);
+                        closestInit(st, h.position + entryDir * 0.001f, entryDir);
+                        tp = xyz(W.tp[p]);
+                        step = 0u;
+                        i = at;
+                        sdfCount(S.sdf_counters, kSdfBounceSceneQueries);
+                    }
+                }
+            }
+        }
+        if (__all_sync(0xffffffffu, i == kNoWork && exhausted)) break;
+        // Advance the rays until as many lanes wait (for their event or for a new
+        // path) as run: events are long code, worth sharing.
+        bool running = i != kNoWork;
+        for (;;) {
+            int count;
+            const bool nodes = majorityStep(running, st.node, count);
+            if (__popc(__ballot_sync(0xffffffffu, !running && !(i == kNoWork && exhausted))) >= count) break;
+            const bool leaf = (st.node & kLeafBit) != 0u;
+            if (!running || nodes == leaf) continue;
+            running = leaf ? closestTriStep(S, st, stackNode, stackT) : closestNodeStep(S, st, stackNode, stackT);
+        }
+        if (i == kNoWork || running) continue;
+        uint32_t outcome = kWalkLost;
+        float3 origin = st.o, direction = st.d;
+        float pdf = 0.0f;
+        bool again = false;
+        if (st.bestTri != kNoHit) {
+            const float4* mp = reinterpret_cast<const float4*>(S.mats + mat);
+            Material m;
+            m.subsurfaceColor = __ldg(mp + 12);
+            m.subsurfaceRadius = __ldg(mp + 13);
+            m.subsurfaceParameters = __ldg(mp + 14);
+            float3 sigmaT = 1.0f / mx(xyz(m.subsurfaceRadius) * fmaxf(m.subsurfaceRadius.w, 0.0f), f3(1e-4f));
+            float f0 = randomFloat(state);
+            float f1 = randomFloat(state);
+            float freeFlight = sampleSubsurfaceFreeFlight(sigmaT, f0, f1);
+            if (freeFlight < st.bestT) {
+                float3 albedo = clamp3(xyz(m.subsurfaceColor), f3(0.0f), f3(0.999f));
+                origin += direction * freeFlight;
+                float h0 = randomFloat(state);
+                float h1 = randomFloat(state);
+                direction = sampleHenyeyGreenstein(h0, h1, direction, clampf(m.subsurfaceParameters.x, -0.95f, 0.95f));
+                float3 tr = exp3((-sigmaT) * freeFlight);
+                tp *= albedo * sigmaT * tr / subsurfaceCollisionPDF(sigmaT, freeFlight);
+                again = !(maxComponent(tp) <= 1e-4f) && ++step < 8u;
+            } else {
+                Hit b = makeHit(S, Ray{origin, direction}, HitRec{st.bestT, st.bestTri, st.bu, st.bv});
+                float3 exitNormal = normalize(b.frontFacing ? b.normal : -b.normal);
+                float x0 = randomFloat(state);
+                float x1 = randomFloat(state);
+                float bt = st.bestT;
+                direction = orientHemisphere(cosineHemisphere(x0, x1), exitNormal);
+                origin = b.position + exitNormal * 0.001f;
+                float3 tr = exp3((-sigmaT) * bt);
+                tp *= tr / subsurfaceBoundaryPDF(sigmaT, bt);
+                pdf = fmaxf(dot(exitNormal, direction), 0.0f) * 0.31830988618f;
+                outcome = kWalkExit;
+            }
+        }
+        if (again) {
+            closestInit(st, origin, direction);
+            sdfCount(S.sdf_counters, kSdfBounceSceneQueries);
+            continue;
+        }
+        W.nee_o[i] = make_float4(origin.x, origin.y, origin.z, __uint_as_float(outcome));
+        W.nee_d[i] = make_float4(direction.x, direction.y, direction.z, __uint_as_float(state));
+        W.nee_c[i] = make_float4(tp.x, tp.y, tp.z, pdf);
+        i = kNoWork;
+    }
+}
+
 struct ShadeOut { bool survive; uint32_t neeMask; uint32_t maxBounces; };
 
 // The body of the reference bounce loop (PathTrace.metal:5252-5518) for one
 // path whose closest hit is already in W.hit.
-// kSss: the subsurface random walk is compiled in (the kernel for materials
-// with a subsurface weight, and for unsorted queues); without it the walk's
-// test is false at compile time, which leaves every other material's path
-// as it was (the walk is entered only for a positive weight).
-template <bool kVolumes, bool kSss>
+// kVolumes: with the subsurface random walk; without, k_subsurface_walk has
+// left its outcome in the path's NEE slots.
+template <bool kVolumes>
 __device__ ShadeOut shadePath(const DevScene& S, const Wave& W, uint32_t p, uint32_t i, uint32_t bounce) {
     float4 ro = W.ray_o[p], rd = W.ray_d[p], tpw = W.tp[p], radw = W.rad[p], hr = W.hit[p];
     uint2 rs = W.rng[p];
@@ -772,12 +911,27 @@ __device__ ShadeOut shadePath(const DevScene& S, const Wave& W, uint32_t p, uint
         continued = true;
     } else {
         float subsurface = materialSubsurface(m);
-        if (kSss && subsurface > 0.0f && randomFloat(state) < subsurface &&
-            continueSubsurfaceRandomWalk<kVolumes>(S, h, m, ray, tp, prevPdf, state)) {
-            continued = true;
-        } else if (continueTransmissiveSurface(h, m, ray, tp, prevPdf, state)) {
-            continued = true;
+        if constexpr (kVolumes) {
+            continued = subsurface > 0.0f && randomFloat(state) < subsurface &&
+                        continueSubsurfaceRandomWalk(S, h, m, ray, tp, prevPdf, state);
+        } else if (subsurface > 0.0f) {
+            const float4 wo = W.nee_o[i];
+            const uint32_t walk = __float_as_uint(wo.w);
+            if (walk == kWalkNone) {
+                randomFloat(state);  // the draw that decided against the walk
+            } else {
+                const float4 wd = W.nee_d[i], wt = W.nee_c[i];
+                state = __float_as_uint(wd.w);
+                tp = xyz(wt);
+                if (walk == kWalkExit) {
+                    ray.origin = xyz(wo);
+                    ray.direction = xyz(wd);
+                    prevPdf = wt.w;
+                    continued = true;
+                }
+            }
         }
+        if (!continued) continued = continueTransmissiveSurface(h, m, ray, tp, prevPdf, state);
     }
     if (continued) {
         bool dead = terminatePathWithRussianRoulette(bounce, tp, state);
@@ -923,32 +1077,29 @@ __device__ ShadeOut shadePath(const DevScene& S, const Wave& W, uint32_t p, uint
 // in the code, so that a fetched line serves all of them: on the large scene
 // 66.4 -> 62.4 ms a frame (1920 x 1080, 16 spp) with blocks of 128 or 256
 // threads, 63.8 with 512; without the barrier block size makes no difference.
-// The kernels with the subsurface walk keep 128 threads (the walk's lengths
-// differ), the one for volumes and the 8-wide tree no barrier either (24.4 ->
-// 25.1 ms a frame with it).
+// The kernel for volumes and the 8-wide tree, whose paths differ more (it
+// traces rays), has 128 threads and no barrier (24.4 -> 25.1 ms a frame with
+// it).
 #ifndef DK_SHADE_BLOCK
 #define DK_SHADE_BLOCK 256
 #endif
 #ifndef DK_SHADE_WARPS
 #define DK_SHADE_WARPS 16
 #endif
-template <bool kSss>
-constexpr int shadeBlock() { return kSss ? 128 : DK_SHADE_BLOCK; }
-// range 0: the whole queue; 1: the sorted queue before the subsurface bucket;
-// 2: from it on.
-template <bool kVolumes, bool kSss>
-__global__ void __launch_bounds__(shadeBlock<kSss>(), DK_SHADE_WARPS * 32 / shadeBlock<kSss>())
-    k_shade(DevScene S, Wave W, uint32_t bounce, uint32_t sel, uint32_t sorted, uint32_t range) {
+template <bool kVolumes>
+constexpr int shadeBlock() { return kVolumes ? 128 : DK_SHADE_BLOCK; }
+template <bool kVolumes>
+__global__ void __launch_bounds__(shadeBlock<kVolumes>(), DK_SHADE_WARPS * 32 / shadeBlock<kVolumes>())
+    k_shade(DevScene S, Wave W, uint32_t bounce, uint32_t sel, uint32_t sorted) {
     const uint32_t* q = sorted ? W.qsorted : W.q[sel];
     const uint32_t n = W.counts[sel];
-    const uint32_t begin = range == 2u ? W.counts[7] : 0u, end = range == 1u ? W.counts[7] : n;
     if (globalId() == 0) W.counts[4] = 0u;  // extend cursor of the next bounce
-    for (uint32_t base = begin + blockIdx.x * blockDim.x; base < end; base += gridStride()) {
+    for (uint32_t base = blockIdx.x * blockDim.x; base < n; base += gridStride()) {
         const uint32_t i = base + threadIdx.x;
         if (!kVolumes) __syncthreads();
-        if (i >= end) continue;
+        if (i >= n) continue;
         uint32_t p = q[i];
-        ShadeOut o = shadePath<kVolumes, kSss>(S, W, p, i, bounce);
+        ShadeOut o = shadePath<kVolumes>(S, W, p, i, bounce);
         bool keep = o.survive && bounce + 1u < o.maxBounces;
         W.live[p] = keep ? 1u : 0u;  // the next queue is built from these flags in path order
         bool sh = o.neeMask != 0u;
@@ -1220,27 +1371,36 @@ __global__ void __launch_bounds__(128) k_shadow_rays(DevScene S, Wave W) {
                     S.volume_count ? nullptr : W.layer_hits + slot * kRecLayers);
         }
         if (__all_sync(0xffffffffu, e == kNoWork && exhausted)) break;
-        if (e == kNoWork) continue;
-        int r = 1;
-        if (S.node_count) {
-            if constexpr (kWide8)
-                r = anySteps(S, st, stack8, kStepBudget);
-            else
-                r = anySteps(S, st, stackNode, kStepBudget);
-        }
-        if (r == 0) continue;
-        size_t slot = (size_t)(e & 3u) * cap + (e >> 2);
-        if (r == 1 && S.volume_count) st.sawNonOpaque = true;  // distance volumes: the walk decides
-        if (r == 2) {
-            W.nee_c[slot] = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
-        } else if (st.sawNonOpaque) {
-            W.layer_count[slot] = st.recCount | (st.recOverflow ? 0x80000000u : 0u);
-            W.qr2[atomicAdd(&W.counts[6], 1u)] = e;
+        auto settle = [&](int r) {  // 1: no opaque blocker, 2: occluded
+            size_t slot = (size_t)(e & 3u) * cap + (e >> 2);
+            if (r == 1 && S.volume_count) st.sawNonOpaque = true;  // distance volumes: the walk decides
+            if (r == 2) {
+                W.nee_c[slot] = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+            } else if (st.sawNonOpaque) {
+                W.layer_count[slot] = st.recCount | (st.recOverflow ? 0x80000000u : 0u);
+                W.qr2[atomicAdd(&W.counts[6], 1u)] = e;
+            } else {
+                float4 c = W.nee_c[slot];
+                W.nee_c[slot] = make_float4(c.x / c.w, c.y / c.w, c.z / c.w, 0.0f);
+            }
+            e = kNoWork;
+        };
+        if (S.node_count == 0) {
+            if (e != kNoWork) settle(1);
+        } else if constexpr (kWide8) {
+            if (e != kNoWork)
+                if (int r = anySteps(S, st, stack8, kStepBudget)) settle(r);
         } else {
-            float4 c = W.nee_c[slot];
-            W.nee_c[slot] = make_float4(c.x / c.w, c.y / c.w, c.z / c.w, 0.0f);
+            const int least = __any_sync(0xffffffffu, exhausted) ? 1 : kRefillBelow;
+            for (;;) {
+                int running;
+                const bool nodes = majorityStep(e != kNoWork, st.node, running);
+                if (running < least) break;
+                const bool leaf = (st.node & kLeafBit) != 0u;
+                if (e == kNoWork || nodes == leaf) continue;
+                if (int r = leaf ? anyTriStep(S, st, stackNode) : anyNodeStep(S, st, stackNode)) settle(r);
+            }
         }
-        e = kNoWork;
     }
 }
 
@@ -1817,12 +1977,13 @@ int kernelGrid(int which, int smCount) {
         case 0: cudaOccupancyMaxActiveBlocksPerMultiprocessor(&perSM, k_generate, 256, 0); break;
         case 1: cudaOccupancyMaxActiveBlocksPerMultiprocessor(&perSM, k_extend<false>, 128, 0); break;
         case 2:
-            cudaOccupancyMaxActiveBlocksPerMultiprocessor(&perSM, k_shade<false, false>, shadeBlock<false>(), 0);
+            cudaOccupancyMaxActiveBlocksPerMultiprocessor(&perSM, k_shade<false>, shadeBlock<false>(), 0);
             break;
         case 3: cudaOccupancyMaxActiveBlocksPerMultiprocessor(&perSM, k_shadow_rays<false>, 128, 0); break;
         case 5: cudaOccupancyMaxActiveBlocksPerMultiprocessor(&perSM, k_extend<true>, 128, 0); break;
         case 6: cudaOccupancyMaxActiveBlocksPerMultiprocessor(&perSM, k_shadow_rays<true>, 128, 0); break;
         case 7: cudaOccupancyMaxActiveBlocksPerMultiprocessor(&perSM, k_extend_volume<false>, 128, 0); break;
+        case 8: cudaOccupancyMaxActiveBlocksPerMultiprocessor(&perSM, k_subsurface_walk, 128, 0); break;
         default: cudaOccupancyMaxActiveBlocksPerMultiprocessor(&perSM, k_finalize, 256, 0); break;
     }
     return (perSM < 1 ? 1 : perSM) * smCount;
@@ -1875,35 +2036,37 @@ uint32_t bounceLaunches(const DevScene& S) {
         g_sortMaterials = (e && e[0] == '0') ? 0 : 1;
     }
     uint32_t n = 1u + (S.volume_count ? 1u : 0u);                  // extend
-    n += 1u + (g_sortMaterials ? (S.volume_count || S.wide8 ? 3u : 4u) : 0u) + 3u;  // sort, shade, survivor queue
+    n += (g_sortMaterials ? 3u : 0u) + (S.has_subsurface && !S.volume_count && !S.wide8 ? 2u : 1u) + 3u;  // sort, (walk,) shade, survivors
     n += 1u + ((!S.all_shadow_opaque || S.volume_count) ? 1u : 0u);  // shadow
     return n + 1u;                                                   // resolve
 }
 
-cudaError_t launchShade(const DevScene& S, const Wave& W, uint32_t bounce, uint32_t sel, int grid, cudaStream_t st) {
+cudaError_t launchShade(const DevScene& S, const Wave& W, uint32_t bounce, uint32_t sel, int grid, int walkGrid,
+                        cudaStream_t st) {
     if (g_sortMaterials < 0) {
         const char* e = getenv("DK_SORT_MATERIALS");
         g_sortMaterials = (e && e[0] == '0') ? 0 : 1;
     }
     uint32_t sorted = (uint32_t)g_sortMaterials;
     if (sorted) {
-        const uint32_t sortBlocks = (W.path_count + 256u * kSortItems - 1u) / (256u * kSortItems);
+        const bool small = W.path_count < kSortSmall;
+        const uint32_t perBlock = 256u * (small ? 2u : 8u), sortBlocks = (W.path_count + perBlock - 1u) / perBlock;
         k_sort_count<<<std::min((uint32_t)grid, sortBlocks), 256, 0, st>>>(S, W, sel);
         k_sort_scan<<<1, kSortBins, 0, st>>>(W);
-        k_sort_scatter<<<sortBlocks, 256, 0, st>>>(W, sel);
+        if (small)
+            k_sort_scatter<2><<<sortBlocks, 256, 0, st>>>(W, sel);
+        else
+            k_sort_scatter<8><<<sortBlocks, 256, 0, st>>>(W, sel);
     }
-    const int sssGrid = std::max(1, grid * shadeBlock<false>() / shadeBlock<true>());
     // The general shading kernel (volume hits, random walks through
     // traceScene) also serves the 8-wide tree, keeping the layout switch out
-    // of the triangle-only kernel.
+    // of the triangle-only kernels.
     if (S.volume_count || S.wide8) {
-        k_shade<true, true><<<sssGrid, shadeBlock<true>(), 0, st>>>(S, W, bounce, sel, sorted, 0u);
-    } else if (sorted) {
-        // materials without a subsurface weight, then those with one
-        k_shade<false, false><<<grid, shadeBlock<false>(), 0, st>>>(S, W, bounce, sel, sorted, 1u);
-        k_shade<false, true><<<sssGrid, shadeBlock<true>(), 0, st>>>(S, W, bounce, sel, sorted, 2u);
+        k_shade<true><<<std::max(1, grid * shadeBlock<false>() / shadeBlock<true>()), shadeBlock<true>(), 0, st>>>(
+            S, W, bounce, sel, sorted);
     } else {
-        k_shade<false, true><<<sssGrid, shadeBlock<true>(), 0, st>>>(S, W, bounce, sel, sorted, 0u);
+        if (S.has_subsurface) k_subsurface_walk<<<walkGrid, 128, 0, st>>>(S, W, sel, sorted);
+        k_shade<false><<<grid, shadeBlock<false>(), 0, st>>>(S, W, bounce, sel, sorted);
     }
     // The survivors, in path order, are the next bounce's queue.
     const uint32_t blocks = (W.path_count + kLiveBlock - 1u) / kLiveBlock;

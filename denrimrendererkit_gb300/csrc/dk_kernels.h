@@ -42,6 +42,7 @@ struct DevScene {
     uint32_t env_guide_size;
     float env_rot_sin, env_rot_cos;  // sincosf(env_rot_y), evaluated once on the device
     uint32_t wide8;                  // traversal tree layout: 0 = 4-wide FP32, 1 = 8-wide quantised
+    uint32_t has_subsurface;         // some render's material may have a subsurface weight: the walk kernel runs
     uint32_t watertight;             // triangle test: 0 = Moller-Trumbore over edges, 1 = watertight over vertices
     // Sparse distance volumes (GPUVolumeDescriptor with metadata.w == 1).
     const dk_volume_descriptor* volumes;
@@ -153,7 +154,8 @@ int buildSahTraversal(const dk_scene* sc, const std::vector<uint32_t>& slotOfTri
 cudaError_t launchGenerate(const DevScene& S, const Wave& W, int grid, cudaStream_t st);
 cudaError_t launchExtend(const DevScene& S, const Wave& W, uint32_t sel, uint32_t bounce, int grid, int volumeGrid,
                          cudaStream_t st);
-cudaError_t launchShade(const DevScene& S, const Wave& W, uint32_t bounce, uint32_t sel, int grid, cudaStream_t st);
+cudaError_t launchShade(const DevScene& S, const Wave& W, uint32_t bounce, uint32_t sel, int grid, int walkGrid,
+                        cudaStream_t st);
 cudaError_t launchShadow(const DevScene& S, const Wave& W, int grid, cudaStream_t st);
 cudaError_t launchResolve(const Wave& W, int grid, cudaStream_t st);
 cudaError_t launchAovPrimary(const DevScene& S, const Wave& W, int grid, cudaStream_t st);

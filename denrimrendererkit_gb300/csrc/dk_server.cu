@@ -149,7 +149,8 @@ int makeSceneSlot(Server* s, const dk_scene* sc, std::unique_ptr<SceneSlot>& out
     rc = dk::uploadScene(S.arena, sc, S.scene,
                          (uint32_t)std::min<uint64_t>((uint64_t)(slots + 1) * S.matCount, 0xffffffffull));
     if (rc != DK_OK) return rc;
-    S.scene.all_shadow_opaque = 0;  // job tables may make materials cut-out or transmissive
+    S.scene.all_shadow_opaque = 0;  // job tables may make materials cut-out or transmissive,
+    S.scene.has_subsurface = 1;     // or give them a subsurface weight
     for (uint32_t k = slots; k > 0; --k) S.freeSlots.push_back(k - 1);
     rc = dk::allocWave(S.arena, S.wave, s->cfg.wave_paths, s->cfg.wave_paths, s->cfg.max_jobs_per_wave);
     if (rc != DK_OK) return rc;
