@@ -159,6 +159,12 @@ STATUS_NAMES = {
 }
 
 # Every symbol include/denrim_cuda.h declares (checked by tests/test_abi.py).
+class AdamGroup(C.Structure):
+    _fields_ = [("weights", C.c_void_p), ("grad", C.c_void_p), ("m", C.c_void_p), ("v", C.c_void_p),
+                ("wbf16", C.c_void_p), ("wflip", C.c_void_p), ("count", C.c_uint32), ("cout", C.c_uint32),
+                ("cin", C.c_uint32), ("reserved", C.c_uint32)]
+
+
 EXPORTED_SYMBOLS = (
     "dk_device_open", "dk_device_count", "dk_session_create", "dk_session_render",
     "dk_session_render_tile", "dk_session_update_camera", "dk_session_reset",
@@ -176,7 +182,7 @@ EXPORTED_SYMBOLS = (
     "dk_unet_avgpool2",
     "dk_unet_avgpool2_backward", "dk_unet_upsample2", "dk_unet_upsample2_backward", "dk_unet_copy_channels",
     "dk_unet_pack_input", "dk_unet_l1_loss", "dk_unet_unpack_output", "dk_unet_l1_loss_residual",
-    "dk_unet_unpack_output_residual", "dk_unet_adam", "dk_unet_weights_to_bf16",
+    "dk_unet_unpack_output_residual", "dk_unet_adam", "dk_unet_adam_groups", "dk_unet_weights_to_bf16",
     "dk_unet_set_conv_path", "dk_unet_error",
 )
 

@@ -1798,7 +1798,7 @@ __global__ void k_copy_channels8(const __nv_bfloat16* src, uint32_t lds, uint32_
 // depth) (1), zeros (6).
 __global__ void k_pack_input(const float4* beauty, const float4* albedo, const float4* normal, const float4* depth,
                              uint32_t imgW, uint32_t imgH, uint32_t x0, uint32_t y0, __nv_bfloat16* out, uint32_t h,
-                             uint32_t w, uint32_t batchIndex) {
+                             uint32_t w, uint32_t batchIndex, bool wide) {
     for (uint32_t i = gid(); i < h * w; i += gstride()) {
         uint32_t x = i % w, y = i / w;
         uint32_t ix = x0 + x, iy = y0 + y;
@@ -1821,9 +1821,29 @@ __global__ void k_pack_input(const float4* beauty, const float4* albedo, const f
             v[9] = dd / (1.0f + dd);
         }
         __nv_bfloat16* o = out + ((size_t)batchIndex * h * w + i) * 16u;
+        if (wide) {  // a pixel's 32 bytes as two stores (eight cost 55 us instead of 28 at 1920 x 1088)
+            st8(o, reinterpret_cast<const float(&)[8]>(v[0]));
+            st8(o + 8, reinterpret_cast<const float(&)[8]>(v[8]));
+            continue;
+        }
 #pragma unroll
         for (int k = 0; k < 16; k += 2)
             *reinterpret_cast<__nv_bfloat162*>(o + k) = __floats2bfloat162_rn(v[k], v[k + 1]);
+    }
+}
+
+// A pixel's first three channels; `wide`: as one 8-byte load (leading dimension
+// a multiple of 4, 8-byte aligned).
+__device__ __forceinline__ void ld3(const __nv_bfloat16* p, bool wide, float (&f)[3]) {
+    if (wide) {
+        const uint2 u = *reinterpret_cast<const uint2*>(p);
+        const float2 t = __bfloat1622float2(*reinterpret_cast<const __nv_bfloat162*>(&u.x));
+        f[0] = t.x;
+        f[1] = t.y;
+        f[2] = __low2float(*reinterpret_cast<const __nv_bfloat162*>(&u.y));
+    } else {
+#pragma unroll
+        for (int k = 0; k < 3; ++k) f[k] = __bfloat162float(p[k]);
     }
 }
 
@@ -1832,23 +1852,33 @@ __global__ void k_pack_input(const float4* beauty, const float4* albedo, const f
 // `base` (the network input, whose first 3 channels are log(1 + noisy)), the
 // prediction is a residual: the output is base + pred.
 __global__ void k_l1_loss(const __nv_bfloat16* pred, uint32_t ldp, const __nv_bfloat16* base, uint32_t ldb,
-                          const float4* target, uint32_t M, __nv_bfloat16* grad, uint32_t ldg, float* loss) {
+                          const float4* target, uint32_t M, __nv_bfloat16* grad, uint32_t ldg, float* loss,
+                          bool wideIn, bool wideGrad) {
     __shared__ float red[256];
     float s = 0.0f;
     const float scale = 1.0f / (3.0f * (float)M);
     for (uint32_t p = gid(); p < M; p += gstride()) {
         float4 t = target[p];
         float tl[3] = {log1pf(fmaxf(t.x, 0.0f)), log1pf(fmaxf(t.y, 0.0f)), log1pf(fmaxf(t.z, 0.0f))};
-        float g[3];
+        float g[3], yp[3], yb[3];
+        ld3(pred + (size_t)p * ldp, wideIn, yp);
+        if (base) ld3(base + (size_t)p * ldb, wideIn, yb);
 #pragma unroll
         for (int k = 0; k < 3; ++k) {
-            float y = __bfloat162float(pred[(size_t)p * ldp + k]);
-            if (base) y += __bfloat162float(base[(size_t)p * ldb + k]);
+            float y = yp[k];
+            if (base) y += yb[k];
             float d = y - tl[k];
             s += fabsf(d);
             g[k] = (d > 0.0f ? scale : (d < 0.0f ? -scale : 0.0f));
         }
         __nv_bfloat16* gp = grad + (size_t)p * ldg;
+        if (wideGrad) {  // ldg 16: the pixel's 32 bytes as two stores
+            const float lo[8] = {g[0], g[1], g[2], 0.0f, 0.0f, 0.0f, 0.0f, 0.0f};
+            const float zero[8] = {0.0f, 0.0f, 0.0f, 0.0f, 0.0f, 0.0f, 0.0f, 0.0f};
+            st8(gp, lo);
+            st8(gp + 8, zero);
+            continue;
+        }
         gp[0] = __float2bfloat16_rn(g[0]);
         gp[1] = __float2bfloat16_rn(g[1]);
         gp[2] = __float2bfloat16_rn(g[2]);
@@ -1868,18 +1898,19 @@ __global__ void k_l1_loss(const __nv_bfloat16* pred, uint32_t ldp, const __nv_bf
 // network input's log(1 + noisy) channels), summed in FP32.
 __global__ void k_unpack_output(const __nv_bfloat16* pred, uint32_t ldp, const __nv_bfloat16* base, uint32_t ldb,
                                 uint32_t h, uint32_t w, const float4* alphaSrc, uint32_t imgW, uint32_t imgH,
-                                uint32_t x0, uint32_t y0, float4* out) {
+                                uint32_t x0, uint32_t y0, float4* out, bool wideIn) {
     for (uint32_t i = gid(); i < h * w; i += gstride()) {
         uint32_t ix = x0 + i % w, iy = y0 + i / w;
         if (ix >= imgW || iy >= imgH) continue;
         size_t s = (size_t)iy * imgW + ix;
-        const __nv_bfloat16* p = pred + (size_t)i * ldp;
-        float y[3] = {__bfloat162float(p[0]), __bfloat162float(p[1]), __bfloat162float(p[2])};
+        float y[3];
+        ld3(pred + (size_t)i * ldp, wideIn, y);
         if (base) {
-            const __nv_bfloat16* b = base + (size_t)i * ldb;
-            y[0] += __bfloat162float(b[0]);
-            y[1] += __bfloat162float(b[1]);
-            y[2] += __bfloat162float(b[2]);
+            float b[3];
+            ld3(base + (size_t)i * ldb, wideIn, b);
+            y[0] += b[0];
+            y[1] += b[1];
+            y[2] += b[2];
         }
         out[s] = make_float4(fmaxf(expm1f(y[0]), 0.0f), fmaxf(expm1f(y[1]), 0.0f), fmaxf(expm1f(y[2]), 0.0f),
                              alphaSrc[s].w);
@@ -1888,16 +1919,21 @@ __global__ void k_unpack_output(const __nv_bfloat16* pred, uint32_t ldp, const _
 
 // Adam on FP32 master weights; writes the bf16 forward weights and, for 3x3
 // layers, the tap-flipped transposed copy the input gradient uses.
-__global__ void k_adam(float* wts, const float* grad, float* m, float* v, uint32_t count, float lr, float b1, float b2,
-                       float eps, float c1, float c2, __nv_bfloat16* wbf, __nv_bfloat16* wflip, uint32_t cout,
-                       uint32_t cin) {
+struct AdamRule {
+    float lr, b1, b2, eps, c1, c2;
+};
+__device__ __forceinline__ float adamStep(const AdamRule& r, float w, float g, float& m, float& v) {
+    m = r.b1 * m + (1.0f - r.b1) * g;
+    v = r.b2 * v + (1.0f - r.b2) * g * g;
+    return w - r.lr * (m / r.c1) / (sqrtf(v / r.c2) + r.eps);
+}
+__global__ void k_adam(float* wts, const float* grad, float* m, float* v, uint32_t count, AdamRule rule,
+                       __nv_bfloat16* wbf, __nv_bfloat16* wflip, uint32_t cout, uint32_t cin) {
     for (uint32_t i = gid(); i < count; i += gstride()) {
-        float g = grad[i];
-        float mi = b1 * m[i] + (1.0f - b1) * g;
-        float vi = b2 * v[i] + (1.0f - b2) * g * g;
+        float mi = m[i], vi = v[i];
+        float wv = adamStep(rule, wts[i], grad[i], mi, vi);
         m[i] = mi;
         v[i] = vi;
-        float wv = wts[i] - lr * (mi / c1) / (sqrtf(vi / c2) + eps);
         wts[i] = wv;
         if (wbf) wbf[i] = __float2bfloat16_rn(wv);
         if (wflip) {
@@ -1905,6 +1941,69 @@ __global__ void k_adam(float* wts, const float* grad, float* m, float* v, uint32
             wflip[((size_t)ci * 9u + (8u - tap)) * cout + co] = __float2bfloat16_rn(wv);
         }
     }
+}
+
+// Every tensor of an optimiser step in one launch: blocks are dealt to the
+// groups by a table in the kernel's parameters.  A block takes 1,024 elements:
+// of a 3x3 layer a 32 x 32 tile of one tap, so that the transposed copy is
+// written through shared memory in runs of output channels.  The 19 layers
+// and their biases: 148 us of kernels in 38 launches, 12 us in one.
+constexpr uint32_t kAdamGroups = 40;
+struct AdamTable {
+    dk_unet_adam_group g[kAdamGroups];
+    uint32_t first[kAdamGroups + 1];  // first block of each group
+    uint32_t groups;
+};
+__global__ void __launch_bounds__(256) k_adam_groups(const __grid_constant__ AdamTable t, AdamRule rule) {
+    __shared__ __nv_bfloat16 tile[32][36];  // [ci][co], rows of 72 bytes
+    uint32_t lo = 0, hi = t.groups - 1u;
+    while (lo < hi) {
+        const uint32_t mid = (lo + hi + 1u) >> 1;
+        if (t.first[mid] <= blockIdx.x) lo = mid;
+        else hi = mid - 1u;
+    }
+    const dk_unet_adam_group& g = t.g[lo];
+    const uint32_t b = blockIdx.x - t.first[lo];
+    __nv_bfloat16* wbf = static_cast<__nv_bfloat16*>(g.wbf16);
+    __nv_bfloat16* wflip = static_cast<__nv_bfloat16*>(g.wflip);
+    if (!wflip) {
+        for (uint32_t i = b * 1024u + threadIdx.x; i < min(g.count, b * 1024u + 1024u); i += 256u) {
+            float mi = g.m[i], vi = g.v[i];
+            const float wv = adamStep(rule, g.weights[i], g.grad[i], mi, vi);
+            g.m[i] = mi;
+            g.v[i] = vi;
+            g.weights[i] = wv;
+            if (wbf) wbf[i] = __float2bfloat16_rn(wv);
+        }
+        return;
+    }
+    const uint32_t ciTiles = (g.cin + 31u) / 32u, coTiles = (g.cout + 31u) / 32u;
+    const uint32_t tap = b / (ciTiles * coTiles), rest = b - tap * ciTiles * coTiles;
+    const uint32_t co0 = rest / ciTiles * 32u, ci0 = rest % ciTiles * 32u;
+    const uint32_t r = threadIdx.x >> 3, c4 = (threadIdx.x & 7u) * 4u;  // four input channels of an output channel
+    if (co0 + r < g.cout && ci0 + c4 < g.cin) {
+        const size_t i = ((size_t)(co0 + r) * 9u + tap) * g.cin + ci0 + c4;
+        float4 w = *reinterpret_cast<const float4*>(g.weights + i), m = *reinterpret_cast<const float4*>(g.m + i);
+        float4 v = *reinterpret_cast<const float4*>(g.v + i);
+        const float4 d = *reinterpret_cast<const float4*>(g.grad + i);
+        w.x = adamStep(rule, w.x, d.x, m.x, v.x);
+        w.y = adamStep(rule, w.y, d.y, m.y, v.y);
+        w.z = adamStep(rule, w.z, d.z, m.z, v.z);
+        w.w = adamStep(rule, w.w, d.w, m.w, v.w);
+        *reinterpret_cast<float4*>(g.weights + i) = w;
+        *reinterpret_cast<float4*>(g.m + i) = m;
+        *reinterpret_cast<float4*>(g.v + i) = v;
+        __nv_bfloat162 h[2] = {__floats2bfloat162_rn(w.x, w.y), __floats2bfloat162_rn(w.z, w.w)};
+        if (wbf) *reinterpret_cast<uint2*>(wbf + i) = *reinterpret_cast<const uint2*>(h);
+        tile[c4 + 0u][r] = __low2bfloat16(h[0]);
+        tile[c4 + 1u][r] = __high2bfloat16(h[0]);
+        tile[c4 + 2u][r] = __low2bfloat16(h[1]);
+        tile[c4 + 3u][r] = __high2bfloat16(h[1]);
+    }
+    __syncthreads();
+    if (ci0 + r < g.cin && co0 + c4 < g.cout)
+        *reinterpret_cast<uint2*>(wflip + ((size_t)(ci0 + r) * 9u + (8u - tap)) * g.cout + co0 + c4) =
+            *reinterpret_cast<const uint2*>(&tile[r][c4]);
 }
 
 __global__ void k_weights_to_bf16(const float* wts, uint32_t count, __nv_bfloat16* wbf, __nv_bfloat16* wflip,
@@ -1937,6 +2036,19 @@ inline bool vec8(std::initializer_list<uint32_t> counts, std::initializer_list<c
     for (const void* q : ptrs)
         if (reinterpret_cast<uintptr_t>(q) % 16u) return false;
     return total > 0 && total < (1ull << 31);
+}
+
+// ld3's 8-byte loads apply to every tensor given.
+inline bool wide4(std::initializer_list<uint32_t> lds, std::initializer_list<const void*> ptrs) {
+    for (uint32_t v : lds)
+        if (v % 4u) return false;
+    for (const void* q : ptrs)
+        if (reinterpret_cast<uintptr_t>(q) % 8u) return false;
+    return true;
+}
+
+inline AdamRule adamRule(float lr, float b1, float b2, float eps, uint32_t step) {
+    return AdamRule{lr, b1, b2, eps, 1.0f - powf(b1, (float)step), 1.0f - powf(b2, (float)step)};
 }
 
 // k_relu_bias8 over `pixels` pixels of `c` channels: up to six resident blocks
@@ -2504,7 +2616,7 @@ int dk_unet_pack_input(const float* beauty, const float* albedo, const float* no
     dk::k_pack_input<<<dk::gridFor((uint64_t)h * w), 256, 0, static_cast<cudaStream_t>(stream)>>>(
         reinterpret_cast<const float4*>(beauty), reinterpret_cast<const float4*>(albedo),
         reinterpret_cast<const float4*>(normal), reinterpret_cast<const float4*>(depth), imgW, imgH, x0, y0,
-        static_cast<bf16*>(out), h, w, batchIndex);
+        static_cast<bf16*>(out), h, w, batchIndex, reinterpret_cast<uintptr_t>(out) % 16u == 0u);
     DK_CUDA(cudaGetLastError(), "pack input launch");
     return DK_OK;
 }
@@ -2515,7 +2627,8 @@ int dk_unet_l1_loss(const void* pred, uint32_t ldp, const float* target, uint32_
         return dk::fail(DK_ERROR_INVALID_ARGUMENT, "dk_unet_l1_loss");
     dk::k_l1_loss<<<dk::gridFor(pixels), 256, 0, static_cast<cudaStream_t>(stream)>>>(
         static_cast<const bf16*>(pred), ldp, nullptr, 0u, reinterpret_cast<const float4*>(target), pixels,
-        static_cast<bf16*>(grad), ldg, loss);
+        static_cast<bf16*>(grad), ldg, loss,
+        dk::wide4({ldp}, {pred}), ldg == 16u && reinterpret_cast<uintptr_t>(grad) % 16u == 0u);
     DK_CUDA(cudaGetLastError(), "loss launch");
     return DK_OK;
 }
@@ -2526,7 +2639,8 @@ int dk_unet_l1_loss_residual(const void* pred, uint32_t ldp, const void* base, u
         return dk::fail(DK_ERROR_INVALID_ARGUMENT, "dk_unet_l1_loss_residual");
     dk::k_l1_loss<<<dk::gridFor(pixels), 256, 0, static_cast<cudaStream_t>(stream)>>>(
         static_cast<const bf16*>(pred), ldp, static_cast<const bf16*>(base), ldb,
-        reinterpret_cast<const float4*>(target), pixels, static_cast<bf16*>(grad), ldg, loss);
+        reinterpret_cast<const float4*>(target), pixels, static_cast<bf16*>(grad), ldg, loss,
+        dk::wide4({ldp, ldb}, {pred, base}), ldg == 16u && reinterpret_cast<uintptr_t>(grad) % 16u == 0u);
     DK_CUDA(cudaGetLastError(), "loss launch");
     return DK_OK;
 }
@@ -2536,7 +2650,7 @@ int dk_unet_unpack_output(const void* pred, uint32_t ldp, uint32_t h, uint32_t w
     if (!pred || !alphaSrc || !out) return dk::fail(DK_ERROR_INVALID_ARGUMENT, "dk_unet_unpack_output");
     dk::k_unpack_output<<<dk::gridFor((uint64_t)h * w), 256, 0, static_cast<cudaStream_t>(stream)>>>(
         static_cast<const bf16*>(pred), ldp, nullptr, 0u, h, w, reinterpret_cast<const float4*>(alphaSrc), imgW, imgH,
-        x0, y0, reinterpret_cast<float4*>(out));
+        x0, y0, reinterpret_cast<float4*>(out), dk::wide4({ldp}, {pred}));
     DK_CUDA(cudaGetLastError(), "unpack output launch");
     return DK_OK;
 }
@@ -2548,7 +2662,8 @@ int dk_unet_unpack_output_residual(const void* pred, uint32_t ldp, const void* b
         return dk::fail(DK_ERROR_INVALID_ARGUMENT, "dk_unet_unpack_output_residual");
     dk::k_unpack_output<<<dk::gridFor((uint64_t)h * w), 256, 0, static_cast<cudaStream_t>(stream)>>>(
         static_cast<const bf16*>(pred), ldp, static_cast<const bf16*>(base), ldb, h, w,
-        reinterpret_cast<const float4*>(alphaSrc), imgW, imgH, x0, y0, reinterpret_cast<float4*>(out));
+        reinterpret_cast<const float4*>(alphaSrc), imgW, imgH, x0, y0, reinterpret_cast<float4*>(out),
+        dk::wide4({ldp, ldb}, {pred, base}));
     DK_CUDA(cudaGetLastError(), "unpack output launch");
     return DK_OK;
 }
@@ -2557,12 +2672,51 @@ int dk_unet_adam(float* weights, const float* grad, float* m, float* v, uint32_t
                  float beta2, float eps, uint32_t step, void* wbf16, void* wflip, uint32_t cout, uint32_t cin,
                  void* stream) {
     if (!weights || !grad || !m || !v || step == 0) return dk::fail(DK_ERROR_INVALID_ARGUMENT, "dk_unet_adam");
-    float c1 = 1.0f - powf(beta1, (float)step), c2 = 1.0f - powf(beta2, (float)step);
     dk::k_adam<<<dk::gridFor(count), 256, 0, static_cast<cudaStream_t>(stream)>>>(
-        weights, grad, m, v, count, lr, beta1, beta2, eps, c1, c2, static_cast<bf16*>(wbf16), static_cast<bf16*>(wflip),
-        cout, cin);
+        weights, grad, m, v, count, dk::adamRule(lr, beta1, beta2, eps, step), static_cast<bf16*>(wbf16),
+        static_cast<bf16*>(wflip), cout, cin);
     DK_CUDA(cudaGetLastError(), "adam launch");
     return DK_OK;
+}
+
+int dk_unet_adam_groups(const dk_unet_adam_group* groups, uint32_t groupCount, float lr, float beta1, float beta2,
+                        float eps, uint32_t step, void* stream) {
+    if ((groupCount && !groups) || step == 0) return dk::fail(DK_ERROR_INVALID_ARGUMENT, "dk_unet_adam_groups");
+    for (uint32_t k = 0; k < groupCount; ++k)
+        if (!groups[k].weights || !groups[k].grad || !groups[k].m || !groups[k].v)
+            return dk::fail(DK_ERROR_INVALID_ARGUMENT, "dk_unet_adam_groups: null tensor");
+    const dk::AdamRule rule = dk::adamRule(lr, beta1, beta2, eps, step);
+    dk::AdamTable t;
+    t.groups = 0;
+    uint32_t blocks = 0;
+    auto flush = [&]() -> int {
+        if (t.groups == 0) return DK_OK;
+        t.first[t.groups] = blocks;
+        dk::k_adam_groups<<<blocks, 256, 0, static_cast<cudaStream_t>(stream)>>>(t, rule);
+        DK_CUDA(cudaGetLastError(), "adam launch");
+        t.groups = 0;
+        blocks = 0;
+        return DK_OK;
+    };
+    for (uint32_t k = 0; k < groupCount; ++k) {
+        const dk_unet_adam_group& g = groups[k];
+        if (g.count == 0) continue;
+        // The tiles take whole [cout][9][cin] layers in 16-byte pieces; other layouts go one tensor at a time.
+        const bool tiled = g.wflip && (uint64_t)g.cout * 9u * g.cin == g.count && g.cin % 4u == 0u && g.cout % 4u == 0u &&
+                           dk::vec8({}, {g.weights, g.grad, g.m, g.v, g.wbf16, g.wflip}, 1u);
+        if (g.wflip && !tiled) {
+            const int rc = dk_unet_adam(g.weights, g.grad, g.m, g.v, g.count, lr, beta1, beta2, eps, step, g.wbf16,
+                                        g.wflip, g.cout, g.cin, stream);
+            if (rc != DK_OK) return rc;
+            continue;
+        }
+        t.g[t.groups] = g;
+        t.first[t.groups++] = blocks;
+        blocks += tiled ? 9u * ((g.cin + 31u) / 32u) * ((g.cout + 31u) / 32u) : (g.count + 1023u) / 1024u;
+        if (t.groups == dk::kAdamGroups)
+            if (const int rc = flush()) return rc;
+    }
+    return flush();
 }
 
 int dk_unet_set_conv_path(int path) {

@@ -121,6 +121,7 @@ class UNet:
         self.step_count = 0
         self.stream = stream
         self._buffers: Dict[Tuple[int, int, int], dict] = {}
+        self._adam_tensors: List[int] = []
         self.refresh_bf16()
 
     # ----------------------------------------------------------- helpers --
@@ -333,9 +334,8 @@ class UNet:
 
     # ------------------------------------------------------------ train --
     def zero_grad(self) -> None:
-        for l in self.layers:
-            l.gw.zero_()
-            l.gb.zero_()
+        torch = _torch()
+        torch._foreach_zero_([t for l in self.layers for t in (l.gw, l.gb)])
 
     def loss(self, target, n: int, h: int, w: int) -> None:
         """L1 in log space against `target` (N*H*W RGBA32F, device); the mean
@@ -351,12 +351,18 @@ class UNet:
 
     def adam(self, lr: float = 1e-3, beta1: float = 0.9, beta2: float = 0.999, eps: float = 1e-8) -> None:
         self.step_count += 1
-        for l in self.layers:
-            self._check(self.lib.dk_unet_adam(_ptr(l.w), _ptr(l.gw), _ptr(l.mw), _ptr(l.vw), l.count, lr, beta1, beta2,
-                                              eps, self.step_count, _ptr(l.wbf), _ptr(l.wflip), l.cout, l.cin,
-                                              self._st))
-            self._check(self.lib.dk_unet_adam(_ptr(l.b), _ptr(l.gb), _ptr(l.mb), _ptr(l.vb), l.cout, lr, beta1, beta2,
-                                              eps, self.step_count, None, None, 1, 1, self._st))
+        tensors = [t.data_ptr() for l in self.layers
+                   for t in (l.w, l.gw, l.mw, l.vw, l.wbf, l.wflip, l.b, l.gb, l.mb, l.vb)]
+        if tensors != self._adam_tensors:  # the parameter table, while the tensors are where they were
+            rows = []
+            for k, l in enumerate(self.layers):
+                p = tensors[10 * k:10 * k + 10]
+                rows.append((*p[:6], l.count, l.cout, l.cin, 0))
+                rows.append((*p[6:], None, None, l.cout, 1, 1, 0))
+            self._adam_groups = (abi.AdamGroup * len(rows))(*rows)
+            self._adam_tensors = tensors
+        self._check(self.lib.dk_unet_adam_groups(self._adam_groups, len(self._adam_groups), lr, beta1, beta2, eps,
+                                                 self.step_count, self._st))
 
     # -------------------------------------------------------- inference --
     def pack(self, beauty, albedo, normal, depth, img_w: int, img_h: int, x0: int, y0: int, n: int, h: int, w: int,

@@ -122,6 +122,8 @@ def load(build_if_missing: bool = False) -> C.CDLL:
             "dk_unet_unpack_output_residual": (i32, [P, u32, P, u32, u32, u32, P, u32, u32, u32, u32, P, P]),
             "dk_unet_adam": (i32, [P, P, P, P, u32, C.c_float, C.c_float, C.c_float, C.c_float, u32, P, P, u32, u32,
                                    P]),
+            "dk_unet_adam_groups": (i32, [C.POINTER(abi.AdamGroup), u32, C.c_float, C.c_float, C.c_float, C.c_float, u32,
+                                          P]),
             "dk_unet_weights_to_bf16": (i32, [P, u32, P, P, u32, u32, P]),
             "dk_unet_set_conv_path": (i32, [i32]),
             "dk_unet_error": (i32, [C.POINTER(i32)]),

@@ -597,6 +597,19 @@ int dk_unet_unpack_output_residual(const void* pred, uint32_t ldp, const void* b
 int dk_unet_adam(float* weights, const float* grad, float* m, float* v, uint32_t count, float lr, float beta1,
                  float beta2, float eps, uint32_t step, void* wbf16, void* wflip, uint32_t cout, uint32_t cin,
                  void* stream);
+/* dk_unet_adam over several tensors in one launch.  Every group is updated as
+ * by its own dk_unet_adam call; `wbf16` and `wflip` may be null. */
+typedef struct dk_unet_adam_group {
+    float* weights;
+    const float* grad;
+    float* m;
+    float* v;
+    void* wbf16;
+    void* wflip;
+    uint32_t count, cout, cin, reserved;
+} dk_unet_adam_group;
+int dk_unet_adam_groups(const dk_unet_adam_group* groups, uint32_t group_count, float lr, float beta1, float beta2,
+                        float eps, uint32_t step, void* stream);
 int dk_unet_weights_to_bf16(const float* weights, uint32_t count, void* wbf16, void* wflip, uint32_t cout,
                             uint32_t cin, void* stream);
 /* Selects the convolution kernel (Cout <= 256 for the tcgen05 ones): 3
