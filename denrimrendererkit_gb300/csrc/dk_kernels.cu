@@ -479,6 +479,11 @@ __global__ void __launch_bounds__(128) k_extend(DevScene S, Wave W, uint32_t sel
         W.counts[7] = 0u;
         W.counts[8] = 0u;
     }
+    if (S.node_count == 0) {  // no triangles: a volume-only scene
+        for (uint32_t i = globalId(); i < n; i += gridStride())
+            W.hit[q[i]] = make_float4(INFINITY, __uint_as_float(kNoHit), 0.0f, 0.0f);
+        return;
+    }
     // The stacks stay separate objects from the scalar state, so that only
     // they live in local memory.
     int stackNode[kWide8 ? 1 : kStackSize];
@@ -493,10 +498,6 @@ __global__ void __launch_bounds__(128) k_extend(DevScene S, Wave W, uint32_t sel
             p = q[idx];
             float4 o = W.ray_o[p], d = W.ray_d[p];
             closestInit(st, xyz(o), xyz(d));
-            if (S.node_count == 0) {
-                W.hit[p] = make_float4(INFINITY, __uint_as_float(kNoHit), 0.0f, 0.0f);
-                p = kNoWork;
-            }
         }
         if (__all_sync(0xffffffffu, p == kNoWork && exhausted)) break;
         if constexpr (kWide8) {
@@ -1286,30 +1287,20 @@ __device__ bool shadowWalk(const DevScene& S, MatTable mt, float3 o, float3 d, f
 }
 
 // Distance-volume closest hit for every ray of the queue, bounded by the
-// triangle hit k_extend found (the volume half of intersectScene).
-#ifndef DK_VOLUME_MIN_BLOCKS
-#define DK_VOLUME_MIN_BLOCKS 4
-#endif
-// Scenes with one sparse volume (the common case) run it as persistent threads
-// with per-lane refill: the volume's grid constants are read once per thread,
-// each lane advances its ray `budget` grid cells at a time and takes the next
-// ray of the queue when its walk is over.  W.counts[8] is the work cursor
-// (zeroed by k_extend).  Measured on the sparse-SDF configuration: budgets of
-// 2 / 8 / 32 cells 417 / 570 / 672 Mpaths/s, 64 to 1024 cells 697-698 (a step
-// then almost always ends the walk: the per-step ballots cost more than the
-// shorter waits for a warp's longest walk save), one ray per thread over the
-// general path 493.  Scenes with several volumes, or budget 0
-// (DK_VOLUME_REFILL=0), take one ray per thread and walk the volumes in turn.
+// triangle hit k_extend found (the volume half of intersectScene): the general
+// form, one ray per thread over the scene's volumes.  With the session's
+// traversal counters (kStats) a single volume is walked by persistent threads
+// with per-lane refill, `kCountedCells` cells at a time (W.counts[8] is the
+// cursor); without them it runs k_volume_march.
+constexpr int kCountedCells = 256;
 template <bool kStats>
-__global__ void __launch_bounds__(128, DK_VOLUME_MIN_BLOCKS) k_extend_volume(DevScene S, Wave W, uint32_t sel,
-                                                                           uint32_t budget) {
+__global__ void __launch_bounds__(128, 4) k_extend_volume(DevScene S, Wave W, uint32_t sel) {
     const uint32_t* q = W.q[sel];
     const uint32_t n = W.counts[sel];
     VolumeScene V = volumeScene(S);
     DDAGrid g;
-    const bool single = budget && V.volumeCount == 1u && V.gridCount != 0u && V.gridIndexCount != 0u &&
-                        V.volumes[0].metadata.w == 1u && ddaGrid(V, 0u, g);
-    if (!single) {
+    if (!kStats || !(V.volumeCount == 1u && V.gridCount != 0u && V.gridIndexCount != 0u &&
+                     V.volumes[0].metadata.w == 1u && ddaGrid(V, 0u, g))) {
         for (uint32_t i = globalId(); i < n; i += gridStride()) {
             uint32_t p = q[i];
             float4 o = W.ray_o[p], d = W.ray_d[p];
@@ -1334,10 +1325,397 @@ __global__ void __launch_bounds__(128, DK_VOLUME_MIN_BLOCKS) k_extend_volume(Dev
             if (!ddaBegin(g, xyz(o), xyz(d), closestT, st)) p = kNoWork;  // misses the volume's bounds
         }
         if (__all_sync(0xffffffffu, p == kNoWork && exhausted)) break;
-        if (p != kNoWork && (kStats ? ddaStepsCounted(V, g, st, (int)budget, S.sdf_counters)
-                                    : ddaSteps(V, g, st, (int)budget))) {
+        if (p != kNoWork && ddaStepsCounted(V, g, st, kCountedCells, S.sdf_counters)) {
             if (st.found && st.out.t < closestT)
                 W.hit[p] = make_float4(st.out.t, __uint_as_float(kVolumeHit), __uint_as_float(st.out.brick), 0.0f);
+            p = kNoWork;
+        }
+    }
+}
+
+// The same for a scene with one sparse volume, as persistent threads with
+// per-lane refill.  A ray's walk (ddaSteps and intersectBrickT, the same
+// operations in the same order) is cut into steps of three kinds: a cell of
+// the brick grid, a distance sample with the decision that follows from it
+// (brick entry, backward search, march, bisection: all the same trilinear
+// sample at another t), and a Newton step of the cubic polish.  A warp takes
+// the kind that most of its lanes wait for, as in the triangle traversal; as
+// nested loops the lanes of a warp waited for its longest march in every
+// brick (16 of 32 busy on camera rays, 8 after the first bounce).  The sample
+// divides by the brick's extents through their reciprocals (divBy).
+// A camera ray visits 26 cells, 21 of them skipped macro cells, and takes a
+// few samples: the walk's arithmetic bounds it (issue 0.66 of the slots), so
+// it too divides through reciprocals, and the entry's constants are computed
+// once per block.  Sparse-SDF configuration, 1024 x 1024 at 16 spp, whole
+// frame: 23.3 ms as nested loops; 21.4 as steps, 19.6 with the divisions
+// through reciprocals, 18.2 with the block's constants.  Blocks per SM 5 / 6 / 7 /
+// 8: 19.2 / 18.2 / 17.7 / 17.3 ms.
+// W.counts[8] is the work cursor (zeroed by k_extend).
+#ifndef DK_VOLUME_MIN_BLOCKS
+#define DK_VOLUME_MIN_BLOCKS 8
+#endif
+constexpr int kWalkCells = 2;  // cells a lane may walk per step (1 / 2 / 4 / 16: 20.2 / 19.6 / 19.7 / 21.7 ms)
+enum MarchPhase : uint32_t { kMarchIdle, kMarchWalk, kMarchEntry, kMarchBack, kMarchStep, kMarchBisect, kMarchPolish };
+
+// a / b rounded to nearest, from y = RN(1 / b): two residual corrections of a * y, the last of
+// which rounds correctly (P. Markstein, "Computation of elementary functions on the IBM RISC
+// System/6000 processor", 1990) where no residual underflows.  b is a length of at least 1e-6 and a
+// a coordinate difference or a distance.
+__device__ __forceinline__ float divBy(float a, float b, float y) {
+    float q = ex::mul(a, y);
+    q = __fmaf_rn(__fmaf_rn(-b, q, a), y, q);
+    return __fmaf_rn(__fmaf_rn(-b, q, a), y, q);
+}
+
+// The volume's constants of a ray's entry (ddaBegin), computed once per block.
+struct MarchVolume {
+    float3 worldMin, worldMax, localMin, extent, rExtent, sampleDen, brick, rBrick;
+    float cellSize;
+};
+__device__ __forceinline__ void marchVolume(const DDAGrid& g, MarchVolume& v) {
+    const dk_volume_descriptor& vol = *g.vol;
+    v.worldMin = ld3f(vol.world_bounds_min);
+    v.worldMax = ld3f(vol.world_bounds_max);
+    v.localMin = ld3f(vol.local_bounds_min);
+    v.extent = mx(ex::sub(ld3f(vol.local_bounds_max), v.localMin), f3(1e-6f));
+    v.rExtent = rcp3(v.extent);
+    v.sampleDen = mx(ex::sub(f3((float)vol.dimensions.x, (float)vol.dimensions.y, (float)vol.dimensions.z), f3(1.0f)), f3(1.0f));
+    v.brick = mx(f3((float)g.bsz[0], (float)g.bsz[1], (float)g.bsz[2]), f3(1.0f));
+    v.rBrick = rcp3(v.brick);
+    v.cellSize = cellSizeOf(vol);
+}
+
+// One ray's constants: 1 / va of the walk (with whether divBy may use them: no
+// component so small or large that a residual could leave the normal range),
+// 1 / units per world unit, and the shortest march step.
+struct MarchRay {
+    float rva[3], rUpw, minimumStep;
+    bool byReciprocal;
+};
+
+// ddaBegin with the block's constants; a component of the local direction too
+// small for divBy's residuals takes the divisions themselves.
+__device__ __forceinline__ bool marchEnter(const DDAGrid& g, const MarchVolume& v, float3 o, float3 d, float closestT,
+                                           DDAState& s, MarchRay& r) {
+    if (!intersectAABB(o, d, v.worldMin, v.worldMax, closestT, s.tNear, s.tFar)) return false;
+    s.vr.lo = mulColumns(g.vol->world_to_local, o, 1.0f);
+    s.vr.ld = mulColumns(g.vol->world_to_local, d, 0.0f);
+    s.vr.upw = fmaxf(exLength(s.vr.ld), 1e-6f);
+    s.vr.cellSize = v.cellSize;
+    s.t = s.tNear;
+    const float3 lp = ex::sub(ex::add(s.vr.lo, ex::mul(s.vr.ld, s.t)), v.localMin);
+    const float from[3] = {lp.x, lp.y, lp.z}, dir[3] = {s.vr.ld.x, s.vr.ld.y, s.vr.ld.z};
+    const float ext[3] = {v.extent.x, v.extent.y, v.extent.z}, rExt[3] = {v.rExtent.x, v.rExtent.y, v.rExtent.z};
+    const float den[3] = {v.sampleDen.x, v.sampleDen.y, v.sampleDen.z};
+    const float bsf[3] = {v.brick.x, v.brick.y, v.brick.z}, rBsf[3] = {v.rBrick.x, v.rBrick.y, v.rBrick.z};
+    r.byReciprocal = true;
+#pragma unroll
+    for (int a = 0; a < 3; ++a) {
+        const float sp = ex::mul(divBy(from[a], ext[a], rExt[a]), den[a]);
+        s.bpa[a] = divBy(ex::add(sp, 0.5f), bsf[a], rBsf[a]);
+        const bool plain = !(dir[a] == 0.0f || fabsf(dir[a]) >= 1e-12f);
+        const float vel = ex::mul(plain ? ex::div(dir[a], ext[a]) : divBy(dir[a], ext[a], rExt[a]), den[a]);
+        s.va[a] = plain ? ex::div(vel, bsf[a]) : divBy(vel, bsf[a], rBsf[a]);
+        const float va = fabsf(s.va[a]);
+        r.rva[a] = ex::rcp(s.va[a]);
+        if (!(va == 0.0f || (va >= 1e-12f && va <= 1e12f))) r.byReciprocal = false;  // (no division by a zero component)
+        s.cell[a] = (int)clampf(floorf(s.bpa[a]), 0.0f, ex::sub((float)g.gd[a], 1.0f));
+        s.stepDir[a] = s.va[a] > 0.0f ? 1 : (s.va[a] < 0.0f ? -1 : 0);
+        const float nb = s.stepDir[a] > 0 ? ex::add((float)s.cell[a], 1.0f) : (float)s.cell[a];
+        const float x = ex::sub(nb, s.bpa[a]);
+        s.tMax[a] = s.stepDir[a] == 0
+                        ? INFINITY
+                        : ex::add(s.t, va >= 1e-12f && va <= 1e12f ? divBy(x, s.va[a], r.rva[a]) : ex::div(x, s.va[a]));
+        s.tDelta[a] = s.stepDir[a] == 0 ? INFINITY : fabsf(r.rva[a]);  // RN(1 / va)
+    }
+    s.step = 0u;
+    s.found = false;
+    s.closest = closestT;
+    r.rUpw = ex::rcp(s.vr.upw);
+    r.minimumStep = fmaxf(divBy(ex::mul(s.vr.cellSize, 0.10f), s.vr.upw, r.rUpw), 0.0005f);
+    return true;
+}
+// The distance to the plane `to` of axis `a` from `from`, in walk units.
+__device__ __forceinline__ float marchPlane(const DDAState& s, const MarchRay& r, int a, float to, float from) {
+    const float x = ex::sub(to, from);
+    return r.byReciprocal ? divBy(x, s.va[a], r.rva[a]) : ex::div(x, s.va[a]);
+}
+
+struct MarchState {
+    uint32_t phase, brick, count;
+    uint32_t dims[3], offset;               // of the brick's samples
+    float3 lo, ext, inv;                    // sample bounds: minimum, extent, 1 / extent
+    float t, lowT, lowD, highT, tFar, entryT;
+};
+
+template <class D>
+__device__ __forceinline__ float marchSample(const D& dist, const MarchState& m, float3 p) {
+    const float u[3] = {divBy(ex::sub(p.x, m.lo.x), m.ext.x, m.inv.x), divBy(ex::sub(p.y, m.lo.y), m.ext.y, m.inv.y),
+                        divBy(ex::sub(p.z, m.lo.z), m.ext.z, m.inv.z)};
+    uint32_t b[3], n[3];
+    float f[3];
+#pragma unroll
+    for (int a = 0; a < 3; ++a) {
+        const float g = ex::mul(clampf(u[a], 0.0f, 1.0f), (float)(m.dims[a] - 1u));
+        b[a] = (uint32_t)floorf(g);
+        n[a] = min(b[a] + 1u, m.dims[a] - 1u);
+        f[a] = ex::sub(g, (float)b[a]);
+    }
+    const uint32_t strideZ = m.dims[0] * m.dims[1];
+    const uint32_t y0 = b[1] * m.dims[0], y1 = n[1] * m.dims[0];
+    const uint32_t z0 = m.offset + b[2] * strideZ, z1 = m.offset + n[2] * strideZ;
+    const float c00 = exMix(dist.at(z0 + y0 + b[0]), dist.at(z0 + y0 + n[0]), f[0]);
+    const float c10 = exMix(dist.at(z0 + y1 + b[0]), dist.at(z0 + y1 + n[0]), f[0]);
+    const float c01 = exMix(dist.at(z1 + y0 + b[0]), dist.at(z1 + y0 + n[0]), f[0]);
+    const float c11 = exMix(dist.at(z1 + y1 + b[0]), dist.at(z1 + y1 + n[0]), f[0]);
+    return exMix(exMix(c00, c10, f[1]), exMix(c01, c11, f[1]), f[2]);
+}
+
+// The walk leaves its cell: false when the ray is finished.
+__device__ __forceinline__ bool marchNextCell(DDAState& s) {
+    const float nextT = fminf(s.tMax[0], fminf(s.tMax[1], s.tMax[2]));
+    if (s.found && s.closest <= ex::add(nextT, 0.0005f)) return false;
+    if (nextT > s.tFar || nextT >= s.closest) return false;
+    if (s.tMax[0] <= s.tMax[1] && s.tMax[0] <= s.tMax[2]) {
+        s.cell[0] += s.stepDir[0];
+        s.t = s.tMax[0];
+        s.tMax[0] = ex::add(s.tMax[0], s.tDelta[0]);
+    } else if (s.tMax[1] <= s.tMax[2]) {
+        s.cell[1] += s.stepDir[1];
+        s.t = s.tMax[1];
+        s.tMax[1] = ex::add(s.tMax[1], s.tDelta[1]);
+    } else {
+        s.cell[2] += s.stepDir[2];
+        s.t = s.tMax[2];
+        s.tMax[2] = ex::add(s.tMax[2], s.tDelta[2]);
+    }
+    ++s.step;
+    return true;
+}
+
+// One cell of the walk: the lane stays in kMarchWalk, enters a brick
+// (kMarchEntry) or is finished (kMarchIdle).
+__device__ __forceinline__ void marchWalk(const VolumeScene& V, const DDAGrid& g, const uint32_t* macroShift,
+                                          DDAState& s, const MarchRay& ray, MarchState& m) {
+    m.phase = kMarchIdle;
+    if (!(s.step < g.maxSteps && s.t <= s.tFar && s.t < s.closest)) return;
+    if (s.cell[0] < 0 || s.cell[1] < 0 || s.cell[2] < 0 || s.cell[0] >= (int)g.gd[0] || s.cell[1] >= (int)g.gd[1] ||
+        s.cell[2] >= (int)g.gd[2])
+        return;
+    if (g.hasMacro) {
+        uint32_t mc[3];
+#pragma unroll
+        for (int a = 0; a < 3; ++a) {
+            const uint32_t c = (uint32_t)s.cell[a];
+            mc[a] = min(macroShift[a] < 32u ? c >> macroShift[a] : c / g.msz[a], g.md[a] - 1u);
+        }
+        const uint64_t macroSlot = (uint64_t)g.macroOffset + mc[0] + mc[1] * g.md[0] + mc[2] * g.md[0] * g.md[1];
+        if (macroSlot < V.gridIndexCount && __ldg(V.gridIndices + macroSlot) == 0u) {
+            const float dt = ex::sub(s.t, s.tNear);
+            float mt[3];
+#pragma unroll
+            for (int a = 0; a < 3; ++a) {
+                const float cb = ex::add(s.bpa[a], ex::mul(s.va[a], dt));
+                const float mb = s.stepDir[a] > 0 ? (float)min((mc[a] + 1u) * g.msz[a], g.gd[a]) : (float)(mc[a] * g.msz[a]);
+                mt[a] = s.stepDir[a] == 0 ? INFINITY : ex::add(s.t, marchPlane(s, ray, a, mb, cb));
+            }
+            const float macroNextT = fminf(mt[0], fminf(mt[1], mt[2]));
+            if (macroNextT > ex::add(s.t, 1e-6f)) {
+                if (macroNextT > s.tFar || macroNextT >= s.closest) return;
+                s.t = ex::add(macroNextT, 1e-5f);
+                const float dt2 = ex::sub(s.t, s.tNear);
+#pragma unroll
+                for (int a = 0; a < 3; ++a) {
+                    const float c2 = ex::add(s.bpa[a], ex::mul(s.va[a], dt2));
+                    s.cell[a] = (int)clampf(floorf(c2), 0.0f, ex::sub((float)g.gd[a], 1.0f));
+                    const float nb = s.stepDir[a] > 0 ? ex::add((float)s.cell[a], 1.0f) : (float)s.cell[a];
+                    s.tMax[a] = s.stepDir[a] == 0 ? INFINITY : ex::add(s.t, marchPlane(s, ray, a, nb, c2));
+                }
+                ++s.step;
+                m.phase = kMarchWalk;
+                return;
+            }
+        }
+    }
+    const uint64_t slot = (uint64_t)g.gridOffset + (uint32_t)s.cell[0] + (uint32_t)s.cell[1] * g.gd[0] +
+                          (uint32_t)s.cell[2] * g.gd[0] * g.gd[1];
+    if (slot < V.gridIndexCount) {
+        const uint32_t bi = __ldg(V.gridIndices + slot);
+        if (bi != 0xffffffffu && bi < V.brickCount) {
+            const dk_volume_brick_descriptor& brick = V.bricks[bi];
+            float tNear, tFar;
+            if (intersectAABB(s.vr.lo, s.vr.ld, ld3f(brick.local_bounds_min), ld3f(brick.local_bounds_max), s.closest,
+                              tNear, tFar)) {
+                const BrickCtx c = makeBrickCtx(brick, V.sampleCount);
+                if (c.valid && !(__ldg(&brick.sample_bounds_min.w) > 0.0f || __ldg(&brick.sample_bounds_max.w) < 0.0f)) {
+                    m.brick = bi;
+#pragma unroll
+                    for (int a = 0; a < 3; ++a) m.dims[a] = c.dims[a];
+                    m.offset = c.sampleOffset;
+                    m.lo = c.sampleMin;
+                    m.ext = c.sampleExtent;
+                    m.inv = rcp3(c.sampleExtent);
+                    m.tFar = tFar;
+                    m.t = m.entryT = tNear;
+                    m.phase = kMarchEntry;
+                    return;
+                }
+            }
+        }
+    }
+    if (marchNextCell(s)) m.phase = kMarchWalk;
+}
+
+// The march from the brick's entry (or the point the backward search found):
+// kMarchStep at its first t, or the brick is left without a hit.
+__device__ __forceinline__ bool marchBegin(MarchState& m, float closest, float upw, float rUpw, float minimumStep) {
+    m.t = fmaxf(m.entryT, ex::add(m.lowT, fmaxf(ex::mul(divBy(fabsf(m.lowD), upw, rUpw), 0.9f), minimumStep)));
+    m.count = 0u;
+    m.phase = kMarchStep;
+    return m.t <= m.tFar && m.t < closest;
+}
+
+template <class D>
+__global__ void __launch_bounds__(128, DK_VOLUME_MIN_BLOCKS) k_volume_march(DevScene S, Wave W, uint32_t sel, D dist) {
+    const uint32_t* q = W.q[sel];
+    const uint32_t n = W.counts[sel];
+    const VolumeScene V = volumeScene(S);
+    DDAGrid g;
+    if (V.gridCount == 0u || V.gridIndexCount == 0u || V.volumes[0].metadata.w != 1u || !ddaGrid(V, 0u, g)) return;
+    __shared__ MarchVolume vol;
+    if (threadIdx.x == 0) marchVolume(g, vol);
+    __syncthreads();
+    uint32_t macroShift[3];  // of the macro size where it is a power of two, else 32
+#pragma unroll
+    for (int a = 0; a < 3; ++a) macroShift[a] = (g.msz[a] & (g.msz[a] - 1u)) ? 32u : 31u - __clz(g.msz[a]);
+    DDAState s;
+    MarchState m;
+    MarchRay ray = {};
+    m.phase = kMarchIdle;
+    uint32_t p = kNoWork;
+    bool exhausted = false;
+    for (;;) {
+        uint32_t idx = warpFetch(&W.counts[8], n, p == kNoWork && !exhausted, exhausted);
+        if (idx != kNoWork) {
+            p = q[idx];
+            float4 o = W.ray_o[p], d = W.ray_d[p];
+            if (marchEnter(g, vol, xyz(o), xyz(d), W.hit[p].x, s, ray))
+                m.phase = kMarchWalk;
+            else
+                p = kNoWork;  // misses the volume's bounds
+        }
+        if (__all_sync(0xffffffffu, p == kNoWork && exhausted)) break;
+        const int least = __any_sync(0xffffffffu, exhausted) ? 1 : kRefillBelow;
+        for (;;) {
+            const unsigned walkers = __ballot_sync(0xffffffffu, m.phase == kMarchWalk);
+            const unsigned samplers = __ballot_sync(0xffffffffu, m.phase >= kMarchEntry && m.phase <= kMarchBisect);
+            const unsigned polishers = __ballot_sync(0xffffffffu, m.phase == kMarchPolish);
+            const int nw = __popc(walkers), ns = __popc(samplers), np = __popc(polishers);
+            if (nw + ns + np < least) break;
+            if (np > max(nw, ns)) {
+                if (m.phase != kMarchPolish) continue;
+                // Two Newton steps on the cubic interpolant: lowT, highT the bracket, t the refined distance.
+                BrickCtx c;
+#pragma unroll
+                for (int a = 0; a < 3; ++a) c.dims[a] = m.dims[a];
+                c.sampleOffset = m.offset;
+                c.strideY = m.dims[0];
+                c.strideZ = m.dims[0] * m.dims[1];
+                c.sampleMin = m.lo;
+                c.sampleExtent = m.ext;
+                c.valid = true;
+                const DistGrad pg = brickDistGradCubic(dist, c, ex::add(s.vr.lo, ex::mul(s.vr.ld, m.t)));
+                const float slope = ex::dot(pg.gradient, s.vr.ld);
+                bool more = isfinite(pg.distance) && !(fabsf(slope) <= 1e-6f);
+                if (more) {
+                    const float projected = ex::sub(m.t, ex::div(pg.distance, slope));
+                    more = !(projected <= m.lowT || projected >= m.highT);
+                    if (more) m.t = projected;
+                }
+                if (more && ++m.count < 2u) continue;
+            } else if (ns >= nw) {
+                if (m.phase < kMarchEntry || m.phase > kMarchBisect) continue;
+                const float dd = marchSample(dist, m, ex::add(s.vr.lo, ex::mul(s.vr.ld, m.t)));
+                const bool finite = isfinite(dd);
+                bool miss = false;
+                if (m.phase == kMarchBisect) {
+                    if ((m.lowD > 0.0f && dd > 0.0f) || (m.lowD < 0.0f && dd < 0.0f)) {
+                        m.lowT = m.t;
+                        m.lowD = dd;
+                    } else {
+                        m.highT = m.t;
+                    }
+                    m.t = ex::mul(0.5f, ex::add(m.lowT, m.highT));
+                    if (++m.count < 8u) continue;
+                    if (s.vr.cellSize <= 0.03f) {
+                        m.phase = kMarchPolish;
+                        m.count = 0u;
+                        continue;
+                    }
+                } else {
+                    if (m.phase == kMarchStep) {
+                        if (!finite) {
+                            miss = true;
+                        } else if ((m.lowD > 0.0f && dd <= 0.0f) || (m.lowD < 0.0f && dd >= 0.0f)) {
+                            m.highT = m.t;
+                            m.t = ex::mul(0.5f, ex::add(m.lowT, m.highT));
+                            m.count = 0u;
+                            m.phase = kMarchBisect;
+                            continue;
+                        } else {
+                            m.lowT = m.t;
+                            m.lowD = dd;
+                            m.t = ex::add(m.t, fmaxf(ex::mul(divBy(fabsf(dd), s.vr.upw, ray.rUpw), 0.8f), ray.minimumStep));
+                            miss = !(++m.count < 192u && m.t <= m.tFar && m.t < s.closest);
+                        }
+                    } else if (m.phase == kMarchEntry) {
+                        m.lowT = m.t;
+                        m.lowD = dd;
+                        if (!finite) {
+                            miss = true;
+                        } else if (dd <= 0.0f) {
+                            m.phase = kMarchBack;
+                            m.count = 0u;
+                        } else {
+                            miss = !marchBegin(m, s.closest, s.vr.upw, ray.rUpw, ray.minimumStep);
+                        }
+                    } else {  // kMarchBack
+                        if (finite && dd > 0.0f) {
+                            m.lowT = m.t;
+                            m.lowD = dd;
+                        }
+                        if (!finite || dd > 0.0f || m.t <= 0.0005f || ++m.count == 12u)
+                            miss = !marchBegin(m, s.closest, s.vr.upw, ray.rUpw, ray.minimumStep);
+                    }
+                    if (!miss) {
+                        if (m.phase == kMarchBack)
+                            m.t = fmaxf(ex::sub(m.t, fmaxf(ex::mul(ex::div(s.vr.cellSize, s.vr.upw), 0.5f), ray.minimumStep)),
+                                        0.0005f);
+                        continue;
+                    }
+                }
+                if (miss) {  // the brick is left without a hit
+                    m.phase = marchNextCell(s) ? kMarchWalk : kMarchIdle;
+                    if (m.phase == kMarchWalk) continue;
+                }
+            } else {
+                if (m.phase != kMarchWalk) continue;
+#pragma unroll 1
+                for (int k = 0; k < kWalkCells && m.phase == kMarchWalk; ++k) marchWalk(V, g, macroShift, s, ray, m);
+                if (m.phase != kMarchIdle) continue;
+            }
+            // Here: a hit at m.t (phase bisect or polish), or the ray is finished (idle).
+            if (m.phase != kMarchIdle) {
+                if (m.t < s.closest) {
+                    s.closest = m.t;
+                    s.out.t = m.t;
+                    s.out.brick = m.brick;
+                    s.found = true;
+                }
+                m.phase = marchNextCell(s) ? kMarchWalk : kMarchIdle;
+                if (m.phase == kMarchWalk) continue;
+            }
+            if (s.found) W.hit[p] = make_float4(s.out.t, __uint_as_float(kVolumeHit), __uint_as_float(s.out.brick), 0.0f);
             p = kNoWork;
         }
     }
@@ -1982,7 +2360,7 @@ int kernelGrid(int which, int smCount) {
         case 3: cudaOccupancyMaxActiveBlocksPerMultiprocessor(&perSM, k_shadow_rays<false>, 128, 0); break;
         case 5: cudaOccupancyMaxActiveBlocksPerMultiprocessor(&perSM, k_extend<true>, 128, 0); break;
         case 6: cudaOccupancyMaxActiveBlocksPerMultiprocessor(&perSM, k_shadow_rays<true>, 128, 0); break;
-        case 7: cudaOccupancyMaxActiveBlocksPerMultiprocessor(&perSM, k_extend_volume<false>, 128, 0); break;
+        case 7: cudaOccupancyMaxActiveBlocksPerMultiprocessor(&perSM, k_volume_march<DistF16>, 128, 0); break;
         case 8: cudaOccupancyMaxActiveBlocksPerMultiprocessor(&perSM, k_subsurface_walk, 128, 0); break;
         default: cudaOccupancyMaxActiveBlocksPerMultiprocessor(&perSM, k_finalize, 256, 0); break;
     }
@@ -2000,16 +2378,16 @@ cudaError_t launchExtend(const DevScene& S, const Wave& W, uint32_t sel, uint32_
     else
         k_extend<false><<<grid, 128, 0, st>>>(S, W, sel, bounce);
     if (S.volume_count) {
-        // grid cells per refill step (DK_VOLUME_BUDGET, default 256); DK_VOLUME_REFILL=0: one ray per thread
-        const char* refill = getenv("DK_VOLUME_REFILL");
-        const char* env = getenv("DK_VOLUME_BUDGET");
-        uint32_t budget = env ? (uint32_t)strtoul(env, nullptr, 10) : 256u;
-        budget = budget < 1u ? 1u : (budget > 1024u ? 1024u : budget);
-        if (refill && refill[0] == '0') budget = 0u;
-        if (S.sdf_counters)  // the counting instantiation only when the session collects them
-            k_extend_volume<true><<<volumeGrid, 128, 0, st>>>(S, W, sel, budget);
-        else
-            k_extend_volume<false><<<volumeGrid, 128, 0, st>>>(S, W, sel, budget);
+        if (S.volume_count > 1u || S.sdf_counters) {
+            if (S.sdf_counters)  // the counting instantiation only when the session collects them
+                k_extend_volume<true><<<volumeGrid, 128, 0, st>>>(S, W, sel);
+            else
+                k_extend_volume<false><<<volumeGrid, 128, 0, st>>>(S, W, sel);
+        } else if (S.brick_dist16) {
+            k_volume_march<<<volumeGrid, 128, 0, st>>>(S, W, sel, DistF16{S.brick_dist16});
+        } else {
+            k_volume_march<<<volumeGrid, 128, 0, st>>>(S, W, sel, DistF32{S.brick_dist});
+        }
     }
     return cudaGetLastError();
 }
