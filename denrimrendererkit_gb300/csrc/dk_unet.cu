@@ -12,6 +12,7 @@
 //             tap-flipped, transposed weights;
 //   wgrad     dW[co][tap][ci] += sum_p dOut[p][co] in[p + tap][ci]
 //             M = taps x Cin, N = Cout, K = pixels, split over CTAs.
+#include <atomic>
 #include <cstdint>
 #include <cstdlib>
 #include <initializer_list>
@@ -232,6 +233,16 @@ __device__ __forceinline__ void mmaF16(uint32_t d, uint32_t aLo, uint32_t bLo, u
         "r"(aLo), "r"(bLo), "r"(hi), "r"(idesc), "r"(acc));
 }
 
+// tcgen05.mma with the operands' own high descriptor words, skipped when `on` is 0.
+__device__ __forceinline__ void mmaF16If(uint32_t on, uint32_t d, uint32_t aLo, uint32_t aHi, uint32_t bLo, uint32_t bHi,
+                                         uint32_t idesc, uint32_t acc) {
+    asm volatile(
+        "{\n.reg .pred p, q;\n.reg .b64 da, db;\nsetp.ne.b32 p, %6, 0;\nsetp.ne.b32 q, %7, 0;\n"
+        "mov.b64 da, {%1, %2};\nmov.b64 db, {%3, %4};\n"
+        "@q tcgen05.mma.cta_group::1.kind::f16 [%0], da, db, %5, p;\n}\n" ::"r"(d),
+        "r"(aLo), "r"(aHi), "r"(bLo), "r"(bHi), "r"(idesc), "r"(acc), "r"(on));
+}
+
 __device__ __forceinline__ bool mbarTryWait(uint32_t bar, uint32_t parity) {
     uint32_t done;
     asm volatile(
@@ -248,6 +259,21 @@ __device__ __forceinline__ bool mbarWait(uint32_t bar, uint32_t parity) {
         if (mbarTryWait(bar, parity)) return true;
         if (clock64() - start > 4000000000ll) return false;  // about 2 s
     }
+}
+
+// The MMA role is run by its whole warp with values the compiler can keep in
+// uniform registers (warp index and tensor-memory address broadcast by a
+// shuffle, loop counters, ring positions), and one elected lane issues.  Issued
+// from a divergent single thread, every tcgen05.mma moved its descriptors and
+// addresses from vector to uniform registers first: about 96 cycles each,
+// whatever N (a 128 x 64 x 16 MMA runs in 32 to 48).
+__device__ __forceinline__ bool electOne() {
+    uint32_t p;
+    asm volatile("{\n.reg .pred p;\nelect.sync _|p, 0xffffffff;\nselp.u32 %0, 1, 0, p;\n}\n" : "=r"(p));
+    return p != 0u;
+}
+__device__ __forceinline__ bool mbarWaitWarp(uint32_t bar, uint32_t parity) {
+    return __all_sync(0xffffffffu, mbarWait(bar, parity));
 }
 
 // A slot of an n-slot ring and the parity of its current use, advanced one
@@ -605,20 +631,11 @@ __device__ __forceinline__ void epilogueRow(uint32_t src, uint32_t c0, uint32_t 
     __syncwarp();
 }
 
-// The K steps of one row-tap stage: for dx = 0, 1, 2 the A operand is the
-// stage's input row from pixel dx on (128 bytes further per pixel) and the B
-// operand the weights of tap (dy, dx); straight-line code (see the halo
-// kernel on branches between MMAs).
-template <uint32_t kSteps>
-__device__ __forceinline__ void rowTapMmas(uint32_t d, uint32_t aLo, uint32_t bLo, uint32_t bTapU, uint32_t hi,
-                                           uint32_t idesc, uint32_t acc) {
-#pragma unroll
-    for (uint32_t dx = 0; dx < 3u; ++dx)
-#pragma unroll
-        for (uint32_t ks = 0; ks < kSteps; ++ks)
-            mmaF16(d, aLo + dx * 8u + 2u * ks, bLo + dx * bTapU + 2u * ks, hi, idesc, (dx | ks) ? 1u : acc);
-}
-
+// A row-tap stage's K steps: for dx = 0, 1, 2 the A operand is the stage's
+// input row from pixel dx on (128 bytes further per pixel) and the B operand
+// the weights of tap (dy, dx); steps past a partial last chunk are predicated
+// off.
+//
 // kRowTap (images at least 128 pixels wide): an output tile is 128 pixels of
 // one row and a pipeline stage is (dy, 64-channel chunk): one box of the input
 // row y + dy - 1, 130 pixels wide, and the weights of the three taps (dy, 0..2),
@@ -641,7 +658,7 @@ __global__ void __launch_bounds__(320, 1)
     uint32_t* tslot = reinterpret_cast<uint32_t*>(bars + 2 * kTmaStagesMax + 8);
     const uint32_t nbuf = accBuffers(a.cols), bufShift = nbuf == 4u ? 2u : 1u;
     int* abortFlag = reinterpret_cast<int*>(tslot + 1);
-    const uint32_t tid = threadIdx.x, warp = tid >> 5, lane = tid & 31u;
+    const uint32_t tid = threadIdx.x, lane = tid & 31u, warp = __shfl_sync(0xffffffffu, tid >> 5, 0);
 
     if (warp == 1) {
         asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;\n" ::"r"(smemAddr(tslot)),
@@ -666,7 +683,7 @@ __global__ void __launch_bounds__(320, 1)
     asm volatile("tcgen05.fence::after_thread_sync;\n" ::: "memory");
     pdlRelease();
     pdlWait();
-    const uint32_t taddr = *tslot;
+    const uint32_t taddr = __shfl_sync(0xffffffffu, *tslot, 0);
     const uint32_t txBytes = (kRowTap ? kHaloPix * 128u : aBytes) + bBytes;
     volatile int* abortV = abortFlag;
 
@@ -724,57 +741,49 @@ __global__ void __launch_bounds__(320, 1)
             if (!ok) *abortV = 1;
         }
     } else if (warp == 1) {
-        if (lane == 0) {
-            const uint32_t idesc = (1u << 4) | (1u << 7) | (1u << 10) | ((N >> 3) << 17) | ((128u >> 4) << 24);
-            const uint32_t hi = descHi(), aLo0 = descLo(smemAddr(sA)), bLo0 = descLo(smemAddr(sB));
-            const uint32_t lastSteps = (a.cin - (a.chunks - 1u) * 64u + 15u) / 16u;
-            RingPos pos{0u, 0u};
-            uint32_t t = 0;
-            for (uint32_t tile = blockIdx.x; tile < a.numTiles && !*abortV; tile += gridDim.x, ++t) {
-                uint32_t b = t & (nbuf - 1u), v = t >> bufShift;
-                if (v > 0 && !mbarWait(accEmptyBar + 8u * b, (v - 1u) & 1u)) {
-                    *abortV = 1;
-                    break;
-                }
-                asm volatile("tcgen05.fence::after_thread_sync;\n" ::: "memory");
-                const uint32_t dAddr = taddr + b * a.cols;
-                bool ok = true;
-                uint32_t acc = 0u;
-                for (uint32_t it = 0; ok && it < (kRowTap ? 3u : 9u); ++it) {
-                    for (uint32_t c = 0; c < a.chunks; ++c, pos.advance(S)) {
-                        if (!mbarWait(fullBar + 8u * pos.slot, pos.phase)) {
-                            ok = false;
-                            break;
-                        }
-                        asm volatile("tcgen05.fence::after_thread_sync;\n" ::: "memory");
-                        // K steps of 16 channels in this (tap, chunk): 4, fewer in a partial last chunk
-                        const uint32_t steps = c + 1u < a.chunks ? 4u : lastSteps;
-                        const uint32_t aLo = aLo0 + pos.slot * (aBytes >> 4), bLo = bLo0 + pos.slot * (bBytes >> 4);
-                        if (kRowTap) {
-                            const uint32_t bTapU = (N * 128u) >> 4;
-                            if (steps == 4u) rowTapMmas<4>(dAddr, aLo, bLo, bTapU, hi, idesc, acc);
-                            else if (steps == 3u) rowTapMmas<3>(dAddr, aLo, bLo, bTapU, hi, idesc, acc);
-                            else if (steps == 2u) rowTapMmas<2>(dAddr, aLo, bLo, bTapU, hi, idesc, acc);
-                            else rowTapMmas<1>(dAddr, aLo, bLo, bTapU, hi, idesc, acc);
-                            acc = 1u;
-                            umaCommit(emptyBar + 8u * pos.slot);
-                            continue;
-                        }
-                        mmaF16(dAddr, aLo, bLo, hi, idesc, acc);
-                        acc = 1u;
-                        if (steps > 1u) mmaF16(dAddr, aLo + 2u, bLo + 2u, hi, idesc, 1u);
-                        if (steps > 2u) mmaF16(dAddr, aLo + 4u, bLo + 4u, hi, idesc, 1u);
-                        if (steps > 3u) mmaF16(dAddr, aLo + 6u, bLo + 6u, hi, idesc, 1u);
+        const uint32_t idesc = (1u << 4) | (1u << 7) | (1u << 10) | ((N >> 3) << 17) | ((128u >> 4) << 24);
+        const uint32_t hi = descHi(), aLo0 = descLo(smemAddr(sA)), bLo0 = descLo(smemAddr(sB));
+        const uint32_t lastSteps = (a.cin - (a.chunks - 1u) * 64u + 15u) / 16u;
+        RingPos pos{0u, 0u};
+        uint32_t t = 0;
+        bool ok = true;
+        for (uint32_t tile = blockIdx.x; ok && tile < a.numTiles; tile += gridDim.x, ++t) {
+            const uint32_t b = t & (nbuf - 1u), v = t >> bufShift;
+            if (v > 0 && !mbarWaitWarp(accEmptyBar + 8u * b, (v - 1u) & 1u)) {
+                ok = false;
+                break;
+            }
+            asm volatile("tcgen05.fence::after_thread_sync;\n" ::: "memory");
+            const uint32_t dAddr = taddr + b * a.cols;
+            uint32_t acc = 0u;
+            for (uint32_t it = 0; ok && it < (kRowTap ? 3u : 9u); ++it) {
+                for (uint32_t c = 0; c < a.chunks; ++c, pos.advance(S)) {
+                    if (!mbarWaitWarp(fullBar + 8u * pos.slot, pos.phase)) {
+                        ok = false;
+                        break;
+                    }
+                    asm volatile("tcgen05.fence::after_thread_sync;\n" ::: "memory");
+                    // K steps of 16 channels in this (tap, chunk): 4, fewer in a partial last chunk
+                    const uint32_t steps = c + 1u < a.chunks ? 4u : lastSteps;
+                    const uint32_t aLo = aLo0 + pos.slot * (aBytes >> 4), bLo = bLo0 + pos.slot * (bBytes >> 4);
+                    if (electOne()) {
+                        const uint32_t bTapU = (N * 128u) >> 4;
+#pragma unroll
+                        for (uint32_t dx = 0; dx < (kRowTap ? 3u : 1u); ++dx)
+#pragma unroll
+                            for (uint32_t ks = 0; ks < 4u; ++ks)
+                                mmaF16If(ks < steps, dAddr, aLo + dx * 8u + 2u * ks, hi, bLo + dx * bTapU + 2u * ks, hi,
+                                         idesc, (dx | ks) ? 1u : acc);
                         umaCommit(emptyBar + 8u * pos.slot);  // the stage is free once these MMAs are done
                     }
+                    __syncwarp();
+                    acc = 1u;
                 }
-                if (!ok) {
-                    *abortV = 1;
-                    break;
-                }
-                umaCommit(accFullBar + 8u * b);  // the accumulator is complete
             }
+            if (ok && electOne()) umaCommit(accFullBar + 8u * b);  // the accumulator is complete
+            __syncwarp();
         }
+        if (!ok && lane == 0) *abortV = 1;
     } else {
         // Epilogue warps 2..9: TMEM lane quarter warp % 4, channel half (warp - 2) / 4.
         const uint32_t q = warp & 3u, half = (warp - 2u) >> 2;
@@ -808,6 +817,253 @@ __global__ void __launch_bounds__(320, 1)
 size_t tmaSmemBytes(uint32_t cout, bool staged, uint32_t stages, bool rowTap) {
     const size_t stage = rowTap ? kHaloSlotBytes + 3u * cout * 128u : 128u * 128u + cout * 128u;
     return (size_t)stages * stage + 1024u + kTmaBarBytes + (staged ? kEpiWarps * epiWarpBytes(cout) : 0u);
+}
+
+// ------------------------------------- tcgen05 + TMA, 2-D halo tiles ----
+// The convolution for the layers the halo-row kernel does not take (narrow
+// images, or weights beyond one CTA's shared memory).  The per-tap kernel above
+// re-reads every input pixel for each tap (9 x 16 KB a tile and chunk) and
+// every tile re-reads the weights, and waits on L2 for both.  Here an output
+// tile is 8 x 16 pixels and its input, 10 x 18 pixels per 64-channel chunk, is
+// loaded once and stays for all nine taps: an MMA's A operand is sixteen groups
+// of eight pixels, one image row apart (stride byte offset = the halo's row),
+// starting at the tap's pixel.  With kT = 2 two tiles side by side share the
+// halo and every weight box.  The weights stream through a ring in stages of
+// three (tap, chunk) boxes, one run of straight-line MMAs each (stages of one
+// box left the tensor core idle for 230 cycles a box: the 160-to-64-channel
+// layer at 960 x 544 takes 118 us with three, 146 with one, and 135 with three
+// waited for but released one by one); K steps past a partial last chunk are
+// predicated off.  Few tiles split the output
+// channels over CTAs.  Warps: 0 weights, 1 MMA, 2-9 epilogue, 10 input.
+// The K order of an output is the replaced kernel's: (dy, chunk, dx) for images
+// at least 128 pixels wide, (tap, chunk) for narrower ones.
+constexpr uint32_t kTileW = 8u, kTileH = 16u;
+constexpr uint32_t kTileChunksMax = 8u;
+constexpr uint32_t kTilePairs = 3u;  // (tap, chunk) boxes of a weight stage
+constexpr uint32_t kTileWStagesMax = 8u;
+constexpr uint32_t kTileBars = 2u * kTileWStagesMax + 8u;
+constexpr uint32_t kTileBarBytes = 8u * kTileBars + 9u * kTileChunksMax * 4u + 32u;
+template <uint32_t kT>
+__host__ __device__ constexpr uint32_t tilePitch() { return kT * kTileW + 2u; }  // halo pixels per row
+template <uint32_t kT>
+__host__ __device__ constexpr uint32_t tileChunkBytes() {
+    return (tilePitch<kT>() * (kTileH + 2u) * 128u + 1023u) & ~1023u;
+}
+
+constexpr uint32_t kTileWStagesMin = 2u;
+struct TileConvArgs {
+    const float* bias;
+    __nv_bfloat16* out;
+    uint32_t n, h, w, ldo, coOff;
+    uint32_t tilesX, tilesY, items;  // groups of kT tiles; work items (image x tiles x channel blocks)
+    uint32_t chunks, lastSteps, pairs, rowOrder;
+    uint32_t nB, nSplit, cols;       // output channels per CTA, blocks of them, accumulator columns
+    uint32_t aSlots, wStages;
+    int act, accumulate, staged;
+};
+
+template <uint32_t kT>
+__global__ void __launch_bounds__(352, 1)
+    k_conv3x3_tile(const __grid_constant__ CUtensorMap mapIn, const __grid_constant__ CUtensorMap mapW,
+                   TileConvArgs a) {
+    constexpr uint32_t kPitch = tilePitch<kT>(), kChunk = tileChunkBytes<kT>();
+    extern __shared__ unsigned char dsm[];
+    const uint32_t raw = smemAddr(dsm);
+    unsigned char* sm = dsm + (((raw + 1023u) & ~1023u) - raw);
+    const uint32_t aBytes = a.chunks * kChunk, wBox = a.nB * 128u, wBytes = kTilePairs * wBox;
+    unsigned char* sW = sm + a.aSlots * aBytes;
+    unsigned char* sEpi = sW + a.wStages * wBytes;
+    uint64_t* bars = reinterpret_cast<uint64_t*>(sEpi + (a.staged ? kEpiWarps * epiWarpBytes(a.nB) : 0u));
+    const uint32_t wFull = smemAddr(bars), wEmpty = wFull + 8u * kTileWStagesMax, aFull = wEmpty + 8u * kTileWStagesMax;
+    const uint32_t aEmpty = aFull + 16u, accFull = aEmpty + 16u, accEmpty = accFull + 16u;
+    uint32_t* table = reinterpret_cast<uint32_t*>(bars + kTileBars);  // per (tap, chunk): A offset | steps << 16 | tap << 20 | chunk << 24
+    uint32_t* tslot = table + 9u * kTileChunksMax;
+    int* abortFlag = reinterpret_cast<int*>(tslot + 1);
+    const uint32_t tid = threadIdx.x, lane = tid & 31u, warp = __shfl_sync(0xffffffffu, tid >> 5, 0);
+    const uint32_t tmemCols = 2u * kT * a.cols <= 64u ? 64u : 2u * kT * a.cols <= 128u ? 128u
+                              : 2u * kT * a.cols <= 256u ? 256u : 512u;
+
+    if (warp == 1) {
+        asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;\n" ::"r"(smemAddr(tslot)),
+                     "r"(tmemCols));
+        asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;\n" ::);
+    }
+    if (tid == 0) {
+        for (uint32_t s = 0; s < a.wStages; ++s) {
+            mbarInit(wFull + 8u * s, 1);
+            mbarInit(wEmpty + 8u * s, 1);
+        }
+        for (uint32_t b = 0; b < 2u; ++b) {
+            mbarInit(aFull + 8u * b, 1);
+            mbarInit(aEmpty + 8u * b, 1);
+            mbarInit(accFull + 8u * b, 1);
+            mbarInit(accEmpty + 8u * b, kT * (epiSplit(a.nB) ? 256u : 128u));
+        }
+        *abortFlag = 0;
+        asm volatile("fence.mbarrier_init.release.cluster;\n" ::: "memory");
+        asm volatile("prefetch.tensormap [%0];\n" ::"l"(&mapIn) : "memory");
+        asm volatile("prefetch.tensormap [%0];\n" ::"l"(&mapW) : "memory");
+    }
+    if (tid < a.pairs) {
+        uint32_t tap, c;
+        if (a.rowOrder) {  // (dy, chunk, dx)
+            const uint32_t dy = tid / (3u * a.chunks), rest = tid - dy * 3u * a.chunks;
+            c = rest / 3u;
+            tap = 3u * dy + rest - 3u * c;
+        } else {  // (tap, chunk)
+            tap = tid / a.chunks;
+            c = tid - tap * a.chunks;
+        }
+        const uint32_t off = c * (kChunk >> 4) + ((tap / 3u) * kPitch + tap % 3u) * 8u;
+        table[tid] = off | ((c + 1u < a.chunks ? 4u : a.lastSteps) << 16) | (tap << 20) | (c << 24);
+    }
+    __syncthreads();
+    asm volatile("tcgen05.fence::after_thread_sync;\n" ::: "memory");
+    pdlRelease();
+    pdlWait();
+    const uint32_t taddr = __shfl_sync(0xffffffffu, *tslot, 0);
+    volatile int* abortV = abortFlag;
+    const uint32_t stages = a.pairs / kTilePairs;  // weight stages of a work item
+
+    if (warp == 0) {
+        if (lane == 0) {  // weights
+            uint32_t g = 0;
+            RingPos pos{0u, 0u};
+            bool ok = true;
+            for (uint32_t item = blockIdx.x; ok && item < a.items && !*abortV; item += gridDim.x) {
+                const int co0 = (int)((item % a.nSplit) * a.nB);
+                for (uint32_t s = 0; s < stages; ++s, ++g, pos.advance(a.wStages)) {
+                    if (g >= a.wStages && !mbarWait(wEmpty + 8u * pos.slot, pos.phase ^ 1u)) {
+                        ok = false;
+                        break;
+                    }
+                    const uint32_t full = wFull + 8u * pos.slot;
+                    mbarExpectTx(full, wBytes);
+#pragma unroll
+                    for (uint32_t j = 0; j < kTilePairs; ++j) {
+                        const uint32_t e = table[s * kTilePairs + j];
+                        tmaLoad3(smemAddr(sW + pos.slot * wBytes + j * wBox), &mapW, (int)((e >> 24) * 64u),
+                                 (int)((e >> 20) & 15u), co0, full);
+                    }
+                }
+            }
+            if (!ok) *abortV = 1;
+        }
+    } else if (warp == 10) {
+        if (lane == 0) {  // input halos
+            RingPos pos{0u, 0u};
+            uint32_t g = 0;
+            for (uint32_t item = blockIdx.x; item < a.items && !*abortV; item += gridDim.x, ++g, pos.advance(a.aSlots)) {
+                if (g >= a.aSlots && !mbarWait(aEmpty + 8u * pos.slot, pos.phase ^ 1u)) {
+                    *abortV = 1;
+                    break;
+                }
+                const uint32_t tile = item / a.nSplit, tx = tile % a.tilesX, rest = tile / a.tilesX;
+                const uint32_t ty = rest % a.tilesY, img = rest / a.tilesY;
+                const uint32_t full = aFull + 8u * pos.slot;
+                mbarExpectTx(full, a.chunks * kPitch * (kTileH + 2u) * 128u);
+                for (uint32_t c = 0; c < a.chunks; ++c)
+                    tmaLoad4(smemAddr(sm + pos.slot * aBytes + c * kChunk), &mapIn, (int)(c * 64u),
+                             (int)(tx * kT * kTileW) - 1, (int)(ty * kTileH) - 1, (int)img, full);
+            }
+        }
+    } else if (warp == 1) {
+        // MMAs
+        const uint32_t idesc = (1u << 4) | (1u << 7) | (1u << 10) | ((a.nB >> 3) << 17) | ((128u >> 4) << 24);
+        const uint32_t bHi = descHi(), aHi = (bHi & ~0x3FFFu) | (kPitch * 8u);  // stride: a halo row, in 16 bytes
+        const uint32_t aLo0 = descLo(smemAddr(sm)), bLo0 = descLo(smemAddr(sW));
+        RingPos ap{0u, 0u}, wp{0u, 0u};
+        uint32_t t = 0;
+        bool ok = true;
+        for (uint32_t item = blockIdx.x; ok && item < a.items; item += gridDim.x, ++t, ap.advance(a.aSlots)) {
+            const uint32_t b = t & 1u, v = t >> 1;
+            if ((v > 0 && !mbarWaitWarp(accEmpty + 8u * b, (v - 1u) & 1u)) ||
+                !mbarWaitWarp(aFull + 8u * ap.slot, ap.phase)) {
+                ok = false;
+                break;
+            }
+            const uint32_t dAddr = taddr + b * kT * a.cols, aBase = aLo0 + ap.slot * (aBytes >> 4);
+            uint32_t dy = 0u, dx = 0u, c = 0u, acc = 0u;  // the next (tap, chunk) pair
+            for (uint32_t s = 0; s < stages; ++s, wp.advance(a.wStages)) {
+                uint32_t aLo[kTilePairs], steps[kTilePairs];
+#pragma unroll
+                for (uint32_t j = 0; j < kTilePairs; ++j) {
+                    aLo[j] = aBase + c * (kChunk >> 4) + (dy * kPitch + dx) * 8u;
+                    steps[j] = c + 1u < a.chunks ? 4u : a.lastSteps;
+                    if (a.rowOrder) {
+                        if (++dx == 3u) {
+                            dx = 0u;
+                            if (++c == a.chunks) {
+                                c = 0u;
+                                ++dy;
+                            }
+                        }
+                    } else if (++c == a.chunks) {
+                        c = 0u;
+                        if (++dx == 3u) {
+                            dx = 0u;
+                            ++dy;
+                        }
+                    }
+                }
+                if (!mbarWaitWarp(wFull + 8u * wp.slot, wp.phase)) {
+                    ok = false;
+                    break;
+                }
+                asm volatile("tcgen05.fence::after_thread_sync;\n" ::: "memory");
+                const uint32_t bBase = bLo0 + wp.slot * (wBytes >> 4);
+                if (electOne()) {
+#pragma unroll
+                    for (uint32_t j = 0; j < kTilePairs; ++j)
+#pragma unroll
+                        for (uint32_t ks = 0; ks < 4u; ++ks)
+#pragma unroll
+                            for (uint32_t q = 0; q < kT; ++q)
+                                mmaF16If(ks < steps[j], dAddr + q * a.cols, aLo[j] + q * (kTileW * 8u) + 2u * ks, aHi,
+                                         bBase + j * (wBox >> 4) + 2u * ks, bHi, idesc, (j | ks) ? 1u : acc);
+                    umaCommit(wEmpty + 8u * wp.slot);
+                }
+                __syncwarp();
+                acc = 1u;
+            }
+            if (ok && electOne()) {
+                umaCommit(aEmpty + 8u * ap.slot);
+                umaCommit(accFull + 8u * b);
+            }
+            __syncwarp();
+        }
+        if (!ok && lane == 0) *abortV = 1;
+    } else {
+        // Epilogue warps 2..9: TMEM lane quarter warp % 4 (four rows of eight pixels), channel half (warp - 2) / 4.
+        const uint32_t q = warp & 3u, half = (warp - 2u) >> 2, N = a.nB;
+        const uint32_t cw = epiCols(N), c0 = half * cw, c1 = epiSplit(N) ? c0 + cw : (half ? 0u : N);
+        unsigned char* stage = a.staged ? sEpi + (warp - 2u) * epiWarpBytes(N) : nullptr;
+        uint32_t t = 0;
+        for (uint32_t item = blockIdx.x; c1 > c0 && item < a.items; item += gridDim.x, ++t) {
+            const uint32_t b = t & 1u, v = t >> 1;
+            if (!mbarWait(accFull + 8u * b, v & 1u)) {
+                *abortV = 1;
+                break;
+            }
+            asm volatile("tcgen05.fence::after_thread_sync;\n" ::: "memory");
+            const uint32_t tile = item / a.nSplit, co0 = (item - tile * a.nSplit) * N;
+            const uint32_t tx = tile % a.tilesX, rest = tile / a.tilesX, ty = rest % a.tilesY, img = rest / a.tilesY;
+            const uint32_t py = ty * kTileH + q * 4u + (lane >> 3);
+#pragma unroll
+            for (uint32_t j = 0; j < kT; ++j) {
+                const uint32_t px = (tx * kT + j) * kTileW + (lane & 7u);
+                const bool valid = px < a.w && py < a.h;
+                __nv_bfloat16* orow =
+                    valid ? a.out + ((size_t)(img * a.h + py) * a.w + px) * a.ldo + a.coOff + co0 : nullptr;
+                epilogueRow(taddr + ((q * 32u) << 16) + (b * kT + j) * a.cols, c0, c1, a.bias ? a.bias + co0 : nullptr,
+                            a.act, a.accumulate, orow, stage, accEmpty + 8u * b);
+            }
+        }
+    }
+    __syncthreads();
+    if (*abortV && tid == 0) atomicExch(&g_unetError, 5);
+    asm volatile("tcgen05.fence::after_thread_sync;\n" ::: "memory");
+    if (warp == 1) asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;\n" ::"r"(taddr), "r"(tmemCols));
 }
 
 // -------------------------------------- tcgen05 + TMA, halo-row ring ----
@@ -995,8 +1251,8 @@ __device__ __forceinline__ uint32_t rangeBegin(const HaloConvArgs& a, uint32_t c
 // kC: 64-channel chunks of the input (Cin / 64 rounded up), kLast: K steps of
 // 16 channels in the last chunk.  Both are compile-time so that each output
 // row's MMAs are straight-line code: a branch between two tcgen05.mma costs
-// the issuing thread a few hundred cycles (measured), about the time of a
-// 128 x 32 x 16 MMA twenty times over.
+// the issuing warp a few hundred cycles (measured), about the time of a
+// 128 x 32 x 16 MMA (40 cycles) ten times over.
 template <bool kStack, uint32_t kC, uint32_t kLast>
 __global__ void __launch_bounds__(320, 1)
     k_conv3x3_halo(const __grid_constant__ CUtensorMap mapIn, const __grid_constant__ CUtensorMap mapW,
@@ -1022,7 +1278,7 @@ __global__ void __launch_bounds__(320, 1)
     const uint32_t bufShift = kStack ? a.logSlots : (nbuf == 4u ? 2u : 1u);
     const uint32_t tmemCols = kStack ? 512u : nbuf * a.cols;
     int* abortFlag = reinterpret_cast<int*>(tslot + 1);
-    const uint32_t tid = threadIdx.x, warp = tid >> 5, lane = tid & 31u;
+    const uint32_t tid = threadIdx.x, lane = tid & 31u, warp = __shfl_sync(0xffffffffu, tid >> 5, 0);
 
     if (warp == 1) {
         asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;\n" ::"r"(smemAddr(tslot)),
@@ -1048,7 +1304,7 @@ __global__ void __launch_bounds__(320, 1)
     asm volatile("tcgen05.fence::after_thread_sync;\n" ::: "memory");
     pdlRelease();
     pdlWait();
-    const uint32_t taddr = *tslot;
+    const uint32_t taddr = __shfl_sync(0xffffffffu, *tslot, 0);
     volatile int* abortV = abortFlag;
 
     if (warp == 0) {
@@ -1090,133 +1346,136 @@ __global__ void __launch_bounds__(320, 1)
             }
         }
     } else if (warp == 1 && kStack) {
-        if (lane == 0) {
-            // Per halo row k of a segment of `rows` output rows: the row's
-            // contributions to output rows k - 2, k - 1, k (taps dy = 2, 1, 0).
-            // Between the segment's edges, and when the three rows' slots are
-            // adjacent, that is one MMA per (dx, chunk, K step) with N = 3 Cout
-            // into the three slots; otherwise one MMA with N = Cout per valid
-            // row.  Slots start zeroed (the epilogue clears a slot when it has
-            // read it), so every MMA accumulates.
-            const uint32_t idesc1 = (1u << 4) | (1u << 7) | (1u << 10) | ((N >> 3) << 17) | ((128u >> 4) << 24);
-            const uint32_t idesc3 = (1u << 4) | (1u << 7) | (1u << 10) | (((3u * N) >> 3) << 17) | ((128u >> 4) << 24);
-            const uint32_t hi = descHi(), aLo0 = descLo(smemAddr(sRing)), bLo0 = descLo(smemAddr(sW));
-            const uint32_t tileU = (3u * wBoxBytes) >> 4, dyU = wBoxBytes >> 4;  // in 16-byte units
-            const uint32_t Q = nbuf;
-            // One halo row's stacked MMAs (N = 3 Cout) into the slots from `d` on.
-            auto stackedRow = [&](uint32_t aRow, uint32_t d) {
+        // Per halo row k of a segment of `rows` output rows: the row's
+        // contributions to output rows k - 2, k - 1, k (taps dy = 2, 1, 0).
+        // Between the segment's edges, and when the three rows' slots are
+        // adjacent, that is one MMA per (dx, chunk, K step) with N = 3 Cout
+        // into the three slots; otherwise one MMA with N = Cout per valid
+        // row.  Slots start zeroed (the epilogue clears a slot when it has
+        // read it), so every MMA accumulates.
+        const uint32_t idesc1 = (1u << 4) | (1u << 7) | (1u << 10) | ((N >> 3) << 17) | ((128u >> 4) << 24);
+        const uint32_t idesc3 = (1u << 4) | (1u << 7) | (1u << 10) | (((3u * N) >> 3) << 17) | ((128u >> 4) << 24);
+        const uint32_t hi = descHi(), aLo0 = descLo(smemAddr(sRing)), bLo0 = descLo(smemAddr(sW));
+        const uint32_t tileU = (3u * wBoxBytes) >> 4, dyU = wBoxBytes >> 4;  // in 16-byte units
+        const uint32_t Q = nbuf;
+        // One halo row's stacked MMAs (N = 3 Cout) into the slots from `d` on.
+        auto stackedRow = [&](uint32_t aRow, uint32_t d) {
 #pragma unroll
-                for (uint32_t dx = 0; dx < 3u; ++dx)
+            for (uint32_t dx = 0; dx < 3u; ++dx)
 #pragma unroll
-                    for (uint32_t c = 0; c < kC; ++c)
+                for (uint32_t c = 0; c < kC; ++c)
 #pragma unroll
-                        for (uint32_t ks = 0; ks < (c + 1u < kC ? 4u : kLast); ++ks)
-                            mmaF16(d, aRow + dx * 8u + c * (kHaloSlotBytes >> 4) + 2u * ks,  // pixel dx: 128 B on
-                                   bLo0 + (dx * kC + c) * tileU + 2u * ks, hi, idesc3, 1u);
-            };
-            bool ok = mbarWait(wBar, 0u);
-            uint32_t t0 = 0;      // output rows of the earlier segments
-            RingPos hp{0u, 0u};   // the current halo row's ring slot
-            uint32_t cur = rangeBegin(a, blockIdx.x);
-            const uint32_t end = rangeBegin(a, blockIdx.x + 1u);
-            RowSegment sg;
-            while (ok && !*abortV && nextSegment(a, cur, end, sg)) {
-                const uint32_t rows = sg.y1 - sg.y0;
-                for (uint32_t k = 0; k < rows + 2u;) {
-                    // Two interior halo rows at once when both stack into adjacent
-                    // slots: their waits first, then both rows' MMAs and commits as
-                    // one straight-line run (one branch per two rows).
-                    if (k >= 2u && k + 1u < rows && ((t0 + k - 2u) & (Q - 1u)) + 3u < Q) {
-                        RingPos hp1 = hp;
-                        hp1.advance(R);
-                        const uint32_t t = t0 + k, sLo = (t0 + k - 2u) & (Q - 1u);
-                        if (!mbarWait(accEmptyBar + 8u * (t & (Q - 1u)), (t >> bufShift) & 1u) ||
-                            !mbarWait(accEmptyBar + 8u * ((t + 1u) & (Q - 1u)), ((t + 1u) >> bufShift) & 1u) ||
-                            !mbarWait(fullBar + 8u * hp.slot, hp.phase) || !mbarWait(fullBar + 8u * hp1.slot, hp1.phase)) {
-                            ok = false;
-                            break;
-                        }
-                        asm volatile("tcgen05.fence::after_thread_sync;\n" ::: "memory");
+                    for (uint32_t ks = 0; ks < (c + 1u < kC ? 4u : kLast); ++ks)
+                        mmaF16(d, aRow + dx * 8u + c * (kHaloSlotBytes >> 4) + 2u * ks,  // pixel dx: 128 B on
+                               bLo0 + (dx * kC + c) * tileU + 2u * ks, hi, idesc3, 1u);
+        };
+        bool ok = mbarWaitWarp(wBar, 0u);
+        uint32_t t0 = 0;      // output rows of the earlier segments
+        RingPos hp{0u, 0u};   // the current halo row's ring slot
+        uint32_t cur = rangeBegin(a, blockIdx.x);
+        const uint32_t end = rangeBegin(a, blockIdx.x + 1u);
+        RowSegment sg;
+        while (ok && !__any_sync(0xffffffffu, *abortV) && nextSegment(a, cur, end, sg)) {
+            const uint32_t rows = sg.y1 - sg.y0;
+            for (uint32_t k = 0; k < rows + 2u;) {
+                // Two interior halo rows at once when both stack into adjacent
+                // slots: their waits first, then both rows' MMAs and commits as
+                // one straight-line run (one branch per two rows).
+                if (k >= 2u && k + 1u < rows && ((t0 + k - 2u) & (Q - 1u)) + 3u < Q) {
+                    RingPos hp1 = hp;
+                    hp1.advance(R);
+                    const uint32_t t = t0 + k, sLo = (t0 + k - 2u) & (Q - 1u);
+                    if (!mbarWaitWarp(accEmptyBar + 8u * (t & (Q - 1u)), (t >> bufShift) & 1u) ||
+                        !mbarWaitWarp(accEmptyBar + 8u * ((t + 1u) & (Q - 1u)), ((t + 1u) >> bufShift) & 1u) ||
+                        !mbarWaitWarp(fullBar + 8u * hp.slot, hp.phase) || !mbarWaitWarp(fullBar + 8u * hp1.slot, hp1.phase)) {
+                        ok = false;
+                        break;
+                    }
+                    asm volatile("tcgen05.fence::after_thread_sync;\n" ::: "memory");
+                    if (electOne()) {
                         stackedRow(aLo0 + hp.slot * (slotBytes >> 4), taddr + sLo * N);
                         umaCommit(emptyBar + 8u * hp.slot);
                         umaCommit(accFullBar + 8u * sLo);
                         stackedRow(aLo0 + hp1.slot * (slotBytes >> 4), taddr + (sLo + 1u) * N);
                         umaCommit(emptyBar + 8u * hp1.slot);
                         umaCommit(accFullBar + 8u * (sLo + 1u));
-                        k += 2u;
-                        hp = hp1;
-                        hp.advance(R);
-                        continue;
                     }
-                    if (k < rows) {  // output row k enters: its slot must have been read and cleared
-                        const uint32_t t = t0 + k;
-                        if (!mbarWait(accEmptyBar + 8u * (t & (Q - 1u)), (t >> bufShift) & 1u)) ok = false;
+                    __syncwarp();
+                    k += 2u;
+                    hp = hp1;
+                    hp.advance(R);
+                    continue;
+                }
+                if (k < rows) {  // output row k enters: its slot must have been read and cleared
+                    const uint32_t t = t0 + k;
+                    if (!mbarWaitWarp(accEmptyBar + 8u * (t & (Q - 1u)), (t >> bufShift) & 1u)) ok = false;
+                }
+                if (ok && !mbarWaitWarp(fullBar + 8u * hp.slot, hp.phase)) ok = false;
+                if (!ok) break;
+                asm volatile("tcgen05.fence::after_thread_sync;\n" ::: "memory");
+                const uint32_t aRow = aLo0 + hp.slot * (slotBytes >> 4);
+                const uint32_t jLo = k >= 2u ? k - 2u : 0u, jHi = min(k, rows - 1u);
+                const uint32_t sLo = (t0 + jLo) & (Q - 1u);
+                const bool stacked = k >= 2u && k < rows && sLo + 2u < Q;
+                if (electOne()) {
+                    if (stacked) stackedRow(aRow, taddr + sLo * N);
+                    for (uint32_t j = jLo; !stacked && j <= jHi; ++j) {
+                        const uint32_t dy = k - j;
+                        const uint32_t d = taddr + ((t0 + j) & (Q - 1u)) * N;
+#pragma unroll
+                        for (uint32_t dx = 0; dx < 3u; ++dx)
+#pragma unroll
+                            for (uint32_t c = 0; c < kC; ++c)
+#pragma unroll
+                                for (uint32_t ks = 0; ks < (c + 1u < kC ? 4u : kLast); ++ks)
+                                    mmaF16(d, aRow + dx * 8u + c * (kHaloSlotBytes >> 4) + 2u * ks,
+                                           bLo0 + (dx * kC + c) * tileU + (2u - dy) * dyU + 2u * ks, hi, idesc1,
+                                           1u);
                     }
-                    if (ok && !mbarWait(fullBar + 8u * hp.slot, hp.phase)) ok = false;
-                    if (!ok) break;
-                    asm volatile("tcgen05.fence::after_thread_sync;\n" ::: "memory");
-                    const uint32_t aRow = aLo0 + hp.slot * (slotBytes >> 4);
-                    const uint32_t jLo = k >= 2u ? k - 2u : 0u, jHi = min(k, rows - 1u);
-                    const uint32_t sLo = (t0 + jLo) & (Q - 1u);
-                    const bool stacked = k >= 2u && k < rows && sLo + 2u < Q;
-                    if (stacked) {
-                        stackedRow(aRow, taddr + sLo * N);
-                    } else {
-                        for (uint32_t j = jLo; j <= jHi; ++j) {
-                            const uint32_t dy = k - j;
-                            const uint32_t d = taddr + ((t0 + j) & (Q - 1u)) * N;
-#pragma unroll
-                            for (uint32_t dx = 0; dx < 3u; ++dx)
-#pragma unroll
-                                for (uint32_t c = 0; c < kC; ++c)
-#pragma unroll
-                                    for (uint32_t ks = 0; ks < (c + 1u < kC ? 4u : kLast); ++ks)
-                                        mmaF16(d, aRow + dx * 8u + c * (kHaloSlotBytes >> 4) + 2u * ks,
-                                               bLo0 + (dx * kC + c) * tileU + (2u - dy) * dyU + 2u * ks, hi, idesc1,
-                                               1u);
-                        }
-                    }
+                }
+                if (electOne()) {
                     umaCommit(emptyBar + 8u * hp.slot);  // halo row k has no reader left
                     if (k >= 2u) umaCommit(accFullBar + 8u * ((t0 + k - 2u) & (Q - 1u)));  // row k - 2 is complete
-                    ++k;
-                    hp.advance(R);
                 }
-                t0 += rows;
+                __syncwarp();
+                ++k;
+                hp.advance(R);
             }
-            if (!ok) *abortV = 1;
+            t0 += rows;
         }
+        if (!ok) *abortV = 1;
     } else if (warp == 1) {
-        if (lane == 0) {
-            const uint32_t idesc = (1u << 4) | (1u << 7) | (1u << 10) | ((N >> 3) << 17) | ((128u >> 4) << 24);
-            const uint32_t hi = descHi(), aLo0 = descLo(smemAddr(sRing)), bLo0 = descLo(smemAddr(sW));
-            bool ok = mbarWait(wBar, 0u);
-            uint32_t t = 0;
-            RingPos top{0u, 0u};  // the item's first halo row
-            uint32_t cur = rangeBegin(a, blockIdx.x);
-            const uint32_t end = rangeBegin(a, blockIdx.x + 1u);
-            RowSegment sg;
-            while (ok && !*abortV && nextSegment(a, cur, end, sg)) {
-                const uint32_t rows = sg.y1 - sg.y0;
-                // halo rows w0, w1, w2 feed the current output row
-                RingPos w0 = top, w1 = top, w2;
-                w1.advance(R);
-                w2 = w1;
-                w2.advance(R);
-                if (!mbarWait(fullBar + 8u * w0.slot, w0.phase) || !mbarWait(fullBar + 8u * w1.slot, w1.phase))
-                    ok = false;
-                for (uint32_t k = 0; ok && k < rows; ++k, ++t) {
-                    if (!mbarWait(fullBar + 8u * w2.slot, w2.phase)) ok = false;
-                    const uint32_t b = t & (nbuf - 1u), v = t >> bufShift;
-                    if (ok && v > 0 && !mbarWait(accEmptyBar + 8u * b, (v - 1u) & 1u)) ok = false;
-                    if (!ok) break;
-                    asm volatile("tcgen05.fence::after_thread_sync;\n" ::: "memory");
-                    const uint32_t dAddr = taddr + b * a.cols;
-                    // A run that starts inside the 1024-byte swizzle pattern (pixel dx)
-                    // takes the plain descriptor: the tensor core applies the 128-byte
-                    // swizzle to absolute shared-memory address bits, as the copy engine
-                    // wrote it (measured: a base offset of (start >> 7) & 7 gives wrong sums).
-                    const uint32_t rowLo[3] = {aLo0 + w0.slot * (slotBytes >> 4), aLo0 + w1.slot * (slotBytes >> 4),
-                                               aLo0 + w2.slot * (slotBytes >> 4)};
+        const uint32_t idesc = (1u << 4) | (1u << 7) | (1u << 10) | ((N >> 3) << 17) | ((128u >> 4) << 24);
+        const uint32_t hi = descHi(), aLo0 = descLo(smemAddr(sRing)), bLo0 = descLo(smemAddr(sW));
+        bool ok = mbarWaitWarp(wBar, 0u);
+        uint32_t t = 0;
+        RingPos top{0u, 0u};  // the item's first halo row
+        uint32_t cur = rangeBegin(a, blockIdx.x);
+        const uint32_t end = rangeBegin(a, blockIdx.x + 1u);
+        RowSegment sg;
+        while (ok && !__any_sync(0xffffffffu, *abortV) && nextSegment(a, cur, end, sg)) {
+            const uint32_t rows = sg.y1 - sg.y0;
+            // halo rows w0, w1, w2 feed the current output row
+            RingPos w0 = top, w1 = top, w2;
+            w1.advance(R);
+            w2 = w1;
+            w2.advance(R);
+            if (!mbarWaitWarp(fullBar + 8u * w0.slot, w0.phase) || !mbarWaitWarp(fullBar + 8u * w1.slot, w1.phase))
+                ok = false;
+            for (uint32_t k = 0; ok && k < rows; ++k, ++t) {
+                if (!mbarWaitWarp(fullBar + 8u * w2.slot, w2.phase)) ok = false;
+                const uint32_t b = t & (nbuf - 1u), v = t >> bufShift;
+                if (ok && v > 0 && !mbarWaitWarp(accEmptyBar + 8u * b, (v - 1u) & 1u)) ok = false;
+                if (!ok) break;
+                asm volatile("tcgen05.fence::after_thread_sync;\n" ::: "memory");
+                const uint32_t dAddr = taddr + b * a.cols;
+                // A run that starts inside the 1024-byte swizzle pattern (pixel dx)
+                // takes the plain descriptor: the tensor core applies the 128-byte
+                // swizzle to absolute shared-memory address bits, as the copy engine
+                // wrote it (measured: a base offset of (start >> 7) & 7 gives wrong sums).
+                const uint32_t rowLo[3] = {aLo0 + w0.slot * (slotBytes >> 4), aLo0 + w1.slot * (slotBytes >> 4),
+                                           aLo0 + w2.slot * (slotBytes >> 4)};
+                if (electOne()) {
 #pragma unroll
                     for (uint32_t tap = 0; tap < 9u; ++tap) {
                         const uint32_t dy = tap / 3u, dx = tap - dy * 3u;
@@ -1231,17 +1490,21 @@ __global__ void __launch_bounds__(320, 1)
                     }
                     umaCommit(accFullBar + 8u * b);          // output row complete
                     umaCommit(emptyBar + 8u * w0.slot);      // its top halo row has no reader left
-                    w0 = w1;
-                    w1 = w2;
-                    w2.advance(R);
                 }
-                if (!ok) break;
+                __syncwarp();
+                w0 = w1;
+                w1 = w2;
+                w2.advance(R);
+            }
+            if (!ok) break;
+            if (electOne()) {
                 umaCommit(emptyBar + 8u * w0.slot);  // the item's last two halo rows
                 umaCommit(emptyBar + 8u * w1.slot);
-                top = w2;
             }
-            if (!ok) *abortV = 1;
+            __syncwarp();
+            top = w2;
         }
+        if (!ok) *abortV = 1;
     } else {
         // Epilogue warps 2..9: TMEM lane quarter warp % 4 (one output pixel per
         // thread); set (warp - 2) / 4.  Stacked: set s takes every channel of
@@ -1374,7 +1637,7 @@ __global__ void __launch_bounds__(128, 1)
     extern __shared__ unsigned char dsm[];
     const uint32_t raw = smemAddr(dsm);
     unsigned char* sm = dsm + (((raw + 1023u) & ~1023u) - raw);
-    const uint32_t tid = threadIdx.x, warp = tid >> 5, lane = tid & 31u;
+    const uint32_t tid = threadIdx.x, lane = tid & 31u, warp = __shfl_sync(0xffffffffu, tid >> 5, 0);
     const uint32_t coBlock = blockIdx.y / a.ciGroups, chunk0 = (blockIdx.y - coBlock * a.ciGroups) * a.cpc;
     const uint32_t co0 = coBlock * a.coB, nc = min(a.cpc, a.chunks - chunk0);
     const uint32_t stageBytes = a.cpc * kWgInSlot + a.coChunks * kWgOutSlot;
@@ -1402,7 +1665,7 @@ __global__ void __launch_bounds__(128, 1)
     }
     __syncthreads();
     asm volatile("tcgen05.fence::after_thread_sync;\n" ::: "memory");
-    const uint32_t taddr = *tslot;
+    const uint32_t taddr = __shfl_sync(0xffffffffu, *tslot, 0);
     volatile int* abortV = abortFlag;
 
     if (tid == 0) {  // TMA producer
@@ -1424,7 +1687,7 @@ __global__ void __launch_bounds__(128, 1)
                 tmaLoad4(base + a.cpc * kWgInSlot + j * kWgOutSlot, &mapOut, (int)(co0 + j * 32u), x0, y0, (int)img,
                          full);
         }
-    } else if (tid == 32) {  // MMA issuer
+    } else if (warp == 1) {  // MMAs
         // kind::f16: D f32, A and B bf16, both MN-major, N = coB, M = 128.
         const uint32_t idesc = (1u << 4) | (1u << 7) | (1u << 10) | (1u << 15) | (1u << 16) | ((a.coB >> 3) << 17) |
                                ((128u >> 4) << 24);
@@ -1435,7 +1698,7 @@ __global__ void __launch_bounds__(128, 1)
         uint32_t acc = 0u;
         bool ok = true;
         for (uint32_t tile = blockIdx.x; tile < a.numTiles; tile += gridDim.x, pos.advance(a.stages)) {
-            if (*abortV || !mbarWait(fullBar + 8u * pos.slot, pos.phase)) {
+            if (!mbarWaitWarp(fullBar + 8u * pos.slot, pos.phase)) {
                 ok = false;
                 break;
             }
@@ -1445,18 +1708,23 @@ __global__ void __launch_bounds__(128, 1)
             for (uint32_t c = 0; c < nc; ++c) {
                 const uint32_t aLo = (((base + c * kWgInSlot) & 0x3FFFFu) >> 4) | aLbo;
                 const uint32_t d = taddr + 3u * c * a.coB;
+                if (electOne()) {
 #pragma unroll
-                for (uint32_t r = 0; r < kWgTile; ++r)
+                    for (uint32_t r = 0; r < kWgTile; ++r)
 #pragma unroll
-                    for (uint32_t dy = 0; dy < 3u; ++dy)
-                        mmaF16(d + dy * a.coB, aLo + (r + dy) * (kWgHalo * 64u / 16u), bLo + r * (kWgTile * 64u / 16u),
-                               hi, idesc, r ? 1u : acc);
+                        for (uint32_t dy = 0; dy < 3u; ++dy)
+                            mmaF16(d + dy * a.coB, aLo + (r + dy) * (kWgHalo * 64u / 16u),
+                                   bLo + r * (kWgTile * 64u / 16u), hi, idesc, r ? 1u : acc);
+                }
+                __syncwarp();
             }
             acc = 1u;
-            umaCommit(emptyBar + 8u * pos.slot);
+            if (electOne()) umaCommit(emptyBar + 8u * pos.slot);
+            __syncwarp();
         }
-        if (ok) umaCommit(doneBar);
-        else *abortV = 1;
+        if (!ok) *abortV = 1;
+        else if (electOne()) umaCommit(doneBar);
+        __syncwarp();
     }
     __syncwarp();
     // Lanes of warp q hold rows 32 q..: horizontal tap q, input channel = lane.
@@ -2260,6 +2528,92 @@ int launchConvHalo(const ConvArgs& c, cudaStream_t st, __nv_bfloat16* pool = nul
     return DK_OK;
 }
 
+// The 2-D halo-tile kernel's launch, or kHaloUnfit (nothing launched).
+int launchConvTile(const ConvArgs& c, cudaStream_t st) {
+    const uint32_t chunks = (c.cin + 63u) / 64u;
+    if (chunks > kTileChunksMax) return kHaloUnfit;
+    const uint32_t sms = (uint32_t)deviceProp().multiProcessorCount;
+    const size_t optin = (size_t)deviceProp().sharedMemPerBlockOptin;
+    const uint64_t tiles = (uint64_t)c.n * ((c.w_ + kTileW - 1u) / kTileW) * ((c.h + kTileH - 1u) / kTileH);
+    if (tiles >= (1ull << 27)) return kHaloUnfit;
+    TileConvArgs a;
+    auto bytes = [&](uint32_t kT, uint32_t nB, uint32_t aSlots, uint32_t wStages, bool staged) {
+        return (size_t)aSlots * chunks * (kT == 2u ? tileChunkBytes<2>() : tileChunkBytes<1>()) +
+               (size_t)wStages * kTilePairs * nB * 128u + (staged ? kEpiWarps * epiWarpBytes(nB) : 0u) + 1024u +
+               kTileBarBytes;
+    };
+    // Output channels per CTA: the most blocks of at least 32 that still find an SM each where the
+    // tiles are few, and more where a block does not fit.
+    a.nSplit = 1u;
+    for (uint32_t k = 2u; k <= c.cout / 32u; ++k)
+        if (c.cout % (16u * k) == 0u && tiles * k <= sms) a.nSplit = k;
+    while (bytes(1u, c.cout / a.nSplit, 1u, kTileWStagesMin, false) > optin && a.nSplit < c.cout / 16u)
+        do ++a.nSplit;
+        while (c.cout % (16u * a.nSplit));
+    a.nB = c.cout / a.nSplit;
+    if (bytes(1u, a.nB, 1u, kTileWStagesMin, false) > optin) return kHaloUnfit;
+    a.cols = (a.nB + 31u) / 32u * 32u;
+    const bool wantStaged = stagedStores(c);
+    // Two tiles per item where there are enough of them and they fit with their epilogue's staging.
+    const bool pair = tiles * a.nSplit >= 2ull * sms && 4u * a.cols <= 512u &&
+                      bytes(2u, a.nB, 1u, kTileWStagesMin, wantStaged) <= optin;
+    // Wide images in single tiles read more weights than the row-tap kernel's rows: 96 to 128 channels at
+    // 240 x 136 15.5 against 12.1 us, 224 to 96 at 480 x 272 63 against 52.
+    if (!pair && c.w_ >= 128u) return kHaloUnfit;
+    const uint32_t kT = pair ? 2u : 1u;
+    const bool staged = wantStaged && bytes(kT, a.nB, 1u, kTileWStagesMin, true) <= optin;
+    a.aSlots = bytes(kT, a.nB, 2u, kTileWStagesMin, staged) <= optin ? 2u : 1u;
+    a.wStages = kTileWStagesMin;
+    while (a.wStages < kTileWStagesMax && bytes(kT, a.nB, a.aSlots, a.wStages + 1u, staged) <= optin) ++a.wStages;
+    const size_t smem = bytes(kT, a.nB, a.aSlots, a.wStages, staged);
+    a.bias = c.bias;
+    a.out = c.out;
+    a.n = c.n;
+    a.h = c.h;
+    a.w = c.w_;
+    a.ldo = c.ldo;
+    a.coOff = c.coOff;
+    a.tilesX = (c.w_ + kT * kTileW - 1u) / (kT * kTileW);
+    a.tilesY = (c.h + kTileH - 1u) / kTileH;
+    a.items = c.n * a.tilesX * a.tilesY * a.nSplit;
+    a.chunks = chunks;
+    a.lastSteps = (c.cin - (chunks - 1u) * 64u + 15u) / 16u;
+    a.pairs = 9u * chunks;
+    a.rowOrder = c.w_ >= 128u && tmaSmemBytes(c.cout, false, 2u, true) <= optin ? 1u : 0u;  // launchConvTma's choice
+    a.act = c.act;
+    a.accumulate = c.accumulate;
+    a.staged = staged ? 1 : 0;
+    EncodeTiledFn enc = encodeTiled();
+    if (!enc) return fail(DK_ERROR_COMMAND_FAILED, "cuTensorMapEncodeTiled is not available");
+    alignas(64) CUtensorMap mapIn, mapW;
+    cuuint32_t unit[4] = {1u, 1u, 1u, 1u};
+    cuuint64_t dimIn[4] = {c.cin, c.w_, c.h, c.n};
+    cuuint64_t strideIn[3] = {(cuuint64_t)c.ldi * 2u, (cuuint64_t)c.w_ * c.ldi * 2u, (cuuint64_t)c.h * c.w_ * c.ldi * 2u};
+    cuuint32_t boxIn[4] = {64u, kT * kTileW + 2u, kTileH + 2u, 1u};
+    CUresult r = enc(&mapIn, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 4, const_cast<__nv_bfloat16*>(c.in), dimIn, strideIn,
+                     boxIn, unit, CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_128B,
+                     CU_TENSOR_MAP_L2_PROMOTION_L2_256B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
+    if (r != CUDA_SUCCESS) return fail(DK_ERROR_INVALID_ARGUMENT, "activation tensor map rejected");
+    cuuint64_t dimW[3] = {c.cin, 9u, c.cout};
+    cuuint64_t strideW[2] = {(cuuint64_t)c.cin * 2u, (cuuint64_t)9u * c.cin * 2u};
+    cuuint32_t boxW[3] = {64u, 1u, a.nB};
+    r = enc(&mapW, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 3, const_cast<__nv_bfloat16*>(c.w), dimW, strideW, boxW, unit,
+            CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_256B,
+            CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
+    if (r != CUDA_SUCCESS) return fail(DK_ERROR_INVALID_ARGUMENT, "weight tensor map rejected");
+    static std::atomic<bool> configured[2];  // one size for every call: threads may set it twice
+    if (!configured[pair].load()) {
+        DK_CUDA(cudaFuncSetAttribute(pair ? k_conv3x3_tile<2> : k_conv3x3_tile<1>,
+                                     cudaFuncAttributeMaxDynamicSharedMemorySize, (int)optin),
+                "conv3x3 (tiles) shared memory");
+        configured[pair].store(true);
+    }
+    const dim3 grid(std::min(sms, a.items));
+    DK_CUDA(launchPdl(pair ? k_conv3x3_tile<2> : k_conv3x3_tile<1>, grid, dim3(352), smem, st, mapIn, mapW, a),
+            "conv3x3 (tiles) launch");
+    return DK_OK;
+}
+
 // rowTap: the row-tap mode (images at least 128 pixels wide); else one stage
 // per (tap, chunk) over 2-D tiles.
 int launchConvTma(const ConvArgs& c, cudaStream_t st, bool rowTap) {
@@ -2382,11 +2736,12 @@ int launchWgrad(const __nv_bfloat16* in, uint32_t ldi, const __nv_bfloat16* dout
     if (encode(&mapOut, dout, ldd, cout, kWgTile) != CUDA_SUCCESS)
         return fail(DK_ERROR_INVALID_ARGUMENT, "gradient tensor map rejected");
     const size_t smem = a.stages * stageBytes(a.cpc) + 1024u + kWgBarBytes;
-    static size_t configured = 0;
-    if (smem > configured) {
-        DK_CUDA(cudaFuncSetAttribute(k_conv3x3_wgrad, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem),
+    static std::atomic<bool> configured;  // one size for every call: threads may set it twice
+    if (!configured.load()) {
+        DK_CUDA(cudaFuncSetAttribute(k_conv3x3_wgrad, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                     (int)deviceProp().sharedMemPerBlockOptin),
                 "conv3x3 wgrad shared memory");
-        configured = smem;
+        configured.store(true);
     }
     const uint32_t gx = std::min(a.numTiles, std::max(1u, sms / groups));
     k_conv3x3_wgrad<<<dim3(gx, groups), 128, smem, st>>>(mapIn, mapOut, a);
@@ -2417,6 +2772,7 @@ int dk_unet_conv3x3(const void* in, uint32_t n, uint32_t h, uint32_t w, uint32_t
     cudaStream_t st = static_cast<cudaStream_t>(stream);
     if (dk::g_convPath == 3 && cout <= 256u) {
         int rc = dk::launchConvHalo(a, st);
+        if (rc == dk::kHaloUnfit) rc = dk::launchConvTile(a, st);
         if (rc != dk::kHaloUnfit) return rc;
     }
     if (dk::g_convPath >= 2 && cout <= 256u) {
