@@ -579,7 +579,7 @@ int allocWave(Arena& arena, Wave& W, uint64_t capPaths, uint32_t pixelCap, uint3
     TRY(arena.alloc(&W.scan, (cap + kLiveBlock - 1) / kLiveBlock + 1, "survivor block offsets"));
     TRY(arena.alloc(&W.qsorted, cap, "material-ordered queue"));
     TRY(arena.alloc(&W.keys, cap, "material keys"));
-    TRY(arena.alloc(&W.bins, kSortBins + 1, "material bins"));
+    TRY(arena.alloc(&W.bins, 2 * kSortBins, "material bins"));
     DevJob* jobs = nullptr;
     TRY(arena.alloc(&jobs, std::max(jobCap, 1u), "job table"));
     W.jobs = jobs;

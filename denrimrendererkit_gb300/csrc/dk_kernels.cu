@@ -465,7 +465,7 @@ __global__ void __launch_bounds__(128) k_extend(DevScene S, Wave W, uint32_t sel
     const uint32_t* q = W.q[sel];
     const uint32_t n = W.counts[sel];
     if (blockIdx.x == 0)
-        for (uint32_t b = threadIdx.x; b <= kSortBins; b += blockDim.x) W.bins[b] = 0u;
+        for (uint32_t b = threadIdx.x; b < 2u * kSortBins; b += blockDim.x) W.bins[b] = 0u;
     if (globalId() == 0) {
         // one scene query per active path and bounce (PathTrace.metal:5252-5256)
         if (S.sdf_counters && n)
@@ -548,6 +548,30 @@ __device__ __forceinline__ uint32_t shadeKey(const DevScene& S, const Wave& W, u
     return 1u + min(id, kSortBins - 3u);
 }
 
+// Exclusive scan of one value per thread over a block of 256, and the sum.
+__device__ __forceinline__ uint32_t blockExclusiveScan256(uint32_t v, uint32_t& total) {
+    __shared__ uint32_t warpSums[8];
+    const uint32_t lane = threadIdx.x & 31u, warp = threadIdx.x >> 5;
+    uint32_t x = v;
+#pragma unroll
+    for (uint32_t o = 1; o < 32u; o <<= 1) {
+        const uint32_t y = __shfl_up_sync(0xffffffffu, x, o);
+        if (lane >= o) x += y;
+    }
+    if (lane == 31u) warpSums[warp] = x;
+    __syncthreads();
+    uint32_t before = 0u;
+    total = 0u;
+#pragma unroll
+    for (uint32_t w = 0; w < 8u; ++w) {
+        const uint32_t c = warpSums[w];
+        if (w < warp) before += c;
+        total += c;
+    }
+    __syncthreads();
+    return before + x - v;
+}
+
 __global__ void __launch_bounds__(256) k_sort_count(DevScene S, Wave W, uint32_t sel) {
     __shared__ uint32_t hist[kSortBins];
     for (uint32_t b = threadIdx.x; b < kSortBins; b += blockDim.x) hist[b] = 0u;
@@ -564,30 +588,15 @@ __global__ void __launch_bounds__(256) k_sort_count(DevScene S, Wave W, uint32_t
         if (hist[b]) atomicAdd(&W.bins[b], hist[b]);
 }
 
-// Exclusive scan of the histogram into bucket cursors (one block of kSortBins threads).
-__global__ void __launch_bounds__(kSortBins) k_sort_scan(Wave W) {
-    __shared__ uint32_t v[kSortBins];
-    uint32_t t = threadIdx.x;
-    uint32_t x = W.bins[t];
-    v[t] = x;
-    __syncthreads();
-    for (uint32_t o = 1; o < kSortBins; o <<= 1) {
-        uint32_t y = t >= o ? v[t - o] : 0u;
-        __syncthreads();
-        v[t] += y;
-        __syncthreads();
-    }
-    W.bins[t] = v[t] - x;
-    if (t == kSubsurfaceKey) W.counts[7] = v[t] - x;  // shading-order index of the first subsurface path
-}
-
 // Block b places its kItems x 256 queue entries stably: an entry's
 // rank among the block's entries of its key follows queue order (in-warp
 // ranks from __match_any_sync, warp offsets per key scanned in shared memory,
 // kItems rounds of 256 entries in order), and one global reservation per
 // (block, key) places the block's run.  The queue is in path order, so every
 // run of a key holds increasing path indices -- neighbouring lanes of the
-// shading kernel read neighbouring path state.
+// shading kernel read neighbouring path state.  Every block scans the histogram
+// itself: 256 counts cost less than a launch of one block that leaves the other
+// SMs idle.
 // kItems: 8 in large waves; 2 in waves of less than kSortSmall paths, whose few
 // blocks would spend their time in the rounds.
 constexpr uint32_t kSortSmall = 1u << 22;
@@ -603,6 +612,9 @@ __global__ void __launch_bounds__(256) k_sort_scatter(Wave W, uint32_t sel) {
     const uint32_t tid = threadIdx.x, lane = tid & 31u, warp = tid >> 5;
     const uint32_t lanesBelow = (1u << lane) - 1u;
     cnt[tid] = 0u;  // kSortBins == blockDim.x
+    uint32_t entries;
+    const uint32_t first = blockExclusiveScan256(W.bins[tid], entries);  // of key `tid` in shading order
+    if (blockIdx.x == 0u && tid == kSubsurfaceKey) W.counts[7] = first;
     uint32_t key[kItems], rank[kItems];
 #pragma unroll
     for (uint32_t k = 0; k < kItems; ++k) {
@@ -630,7 +642,7 @@ __global__ void __launch_bounds__(256) k_sort_scatter(Wave W, uint32_t sel) {
         rank[k] = valid ? warpCnt[warp][key[k]] + inWarp : 0u;
         __syncthreads();
     }
-    if (cnt[tid]) base[tid] = atomicAdd(&W.bins[tid], cnt[tid]);
+    if (cnt[tid]) base[tid] = first + atomicAdd(&W.bins[kSortBins + tid], cnt[tid]);
     __syncthreads();
 #pragma unroll
     for (uint32_t k = 0; k < kItems; ++k) {
@@ -641,10 +653,11 @@ __global__ void __launch_bounds__(256) k_sort_scatter(Wave W, uint32_t sel) {
 
 // ------------------------------------------ survivors in path order ----
 // Shading writes a flag per path; the next bounce's queue is the flagged
-// paths in increasing path order: a count per block of kLiveBlock paths, one
-// block's scan of the counts, and a scatter of each block's paths at its
-// offset.  Path order keeps the extension stage's and (through the stable
-// material sort) the shading stage's path-state accesses coalesced.
+// paths in increasing path order: a count per block of kLiveBlock paths, and a
+// scatter of each block's paths after those of the blocks before it, whose
+// counts (a few thousand at most) every block adds up itself.  Path order keeps
+// the extension stage's and (through the stable material sort) the shading
+// stage's path-state accesses coalesced.
 __device__ __forceinline__ uint32_t liveCount16(const Wave& W, uint32_t first, uint32_t n, uint32_t& bits) {
     bits = 0u;
     if (first + 16u <= n) {
@@ -660,29 +673,6 @@ __device__ __forceinline__ uint32_t liveCount16(const Wave& W, uint32_t first, u
     return __popc(bits);
 }
 
-__device__ __forceinline__ uint32_t blockExclusiveScan256(uint32_t v, uint32_t& total) {
-    __shared__ uint32_t warpSums[8];
-    const uint32_t lane = threadIdx.x & 31u, warp = threadIdx.x >> 5;
-    uint32_t x = v;
-#pragma unroll
-    for (uint32_t o = 1; o < 32u; o <<= 1) {
-        const uint32_t y = __shfl_up_sync(0xffffffffu, x, o);
-        if (lane >= o) x += y;
-    }
-    if (lane == 31u) warpSums[warp] = x;
-    __syncthreads();
-    uint32_t before = 0u;
-    total = 0u;
-#pragma unroll
-    for (uint32_t w = 0; w < 8u; ++w) {
-        const uint32_t c = warpSums[w];
-        if (w < warp) before += c;
-        total += c;
-    }
-    __syncthreads();
-    return before + x - v;
-}
-
 __global__ void __launch_bounds__(256) k_live_count(Wave W) {
     const uint32_t n = W.path_count;
     const uint32_t first = blockIdx.x * kLiveBlock + threadIdx.x * 16u;
@@ -692,28 +682,16 @@ __global__ void __launch_bounds__(256) k_live_count(Wave W) {
     if (threadIdx.x == 0) W.scan[blockIdx.x] = total;
 }
 
-// Exclusive scan of the block counts (one block); the total is the next queue's length.
-__global__ void __launch_bounds__(256) k_live_scan(Wave W, uint32_t sel, uint32_t blocks) {
-    const uint32_t per = (blocks + 255u) / 256u;
-    const uint32_t b0 = threadIdx.x * per;
-    uint32_t sum = 0u;
-    for (uint32_t b = b0; b < b0 + per && b < blocks; ++b) sum += W.scan[b];
-    uint32_t total;
-    uint32_t run = blockExclusiveScan256(sum, total);
-    for (uint32_t b = b0; b < b0 + per && b < blocks; ++b) {
-        const uint32_t c = W.scan[b];
-        W.scan[b] = run;
-        run += c;
-    }
-    if (threadIdx.x == 0) W.counts[sel ^ 1u] = total;
-}
-
 __global__ void __launch_bounds__(256) k_live_scatter(Wave W, uint32_t sel) {
     const uint32_t n = W.path_count;
     const uint32_t first = blockIdx.x * kLiveBlock + threadIdx.x * 16u;
     uint32_t bits = 0u, total;
     const uint32_t c = first < n ? liveCount16(W, first, n, bits) : 0u;
-    uint32_t slot = W.scan[blockIdx.x] + blockExclusiveScan256(c, total);
+    uint32_t sum = 0u, before;
+    for (uint32_t b = threadIdx.x; b < blockIdx.x; b += 256u) sum += W.scan[b];
+    blockExclusiveScan256(sum, before);
+    uint32_t slot = before + blockExclusiveScan256(c, total);
+    if (blockIdx.x == gridDim.x - 1u && threadIdx.x == 0u) W.counts[sel ^ 1u] = before + total;  // the next queue's length
     uint32_t* qNext = W.q[sel ^ 1u];
     while (bits) {
         const uint32_t j = __ffs(bits) - 1u;
@@ -2414,7 +2392,7 @@ uint32_t bounceLaunches(const DevScene& S) {
         g_sortMaterials = (e && e[0] == '0') ? 0 : 1;
     }
     uint32_t n = 1u + (S.volume_count ? 1u : 0u);                  // extend
-    n += (g_sortMaterials ? 3u : 0u) + (S.has_subsurface && !S.volume_count && !S.wide8 ? 2u : 1u) + 3u;  // sort, (walk,) shade, survivors
+    n += (g_sortMaterials ? 2u : 0u) + (S.has_subsurface && !S.volume_count && !S.wide8 ? 2u : 1u) + 2u;  // sort, (walk,) shade, survivors
     n += 1u + ((!S.all_shadow_opaque || S.volume_count) ? 1u : 0u);  // shadow
     return n + 1u;                                                   // resolve
 }
@@ -2430,7 +2408,6 @@ cudaError_t launchShade(const DevScene& S, const Wave& W, uint32_t bounce, uint3
         const bool small = W.path_count < kSortSmall;
         const uint32_t perBlock = 256u * (small ? 2u : 8u), sortBlocks = (W.path_count + perBlock - 1u) / perBlock;
         k_sort_count<<<std::min((uint32_t)grid, sortBlocks), 256, 0, st>>>(S, W, sel);
-        k_sort_scan<<<1, kSortBins, 0, st>>>(W);
         if (small)
             k_sort_scatter<2><<<sortBlocks, 256, 0, st>>>(W, sel);
         else
@@ -2450,10 +2427,7 @@ cudaError_t launchShade(const DevScene& S, const Wave& W, uint32_t bounce, uint3
     const uint32_t blocks = (W.path_count + kLiveBlock - 1u) / kLiveBlock;
     if (blocks) {
         k_live_count<<<blocks, 256, 0, st>>>(W);
-        k_live_scan<<<1, 256, 0, st>>>(W, sel, blocks);
         k_live_scatter<<<blocks, 256, 0, st>>>(W, sel);
-    } else {
-        k_live_scan<<<1, 256, 0, st>>>(W, sel, 0u);
     }
     return cudaGetLastError();
 }

@@ -128,10 +128,10 @@ struct Wave {
     uint2* layer_hits;      // kRecLayers per shadow-ray slot: (t bits, triangle slot) of crossed non-opaque triangles
     uint32_t* layer_count;  // per shadow-ray slot: recorded layers, bit 31 = more than kRecLayers
     uint8_t* live;     // per path: 1 when it goes on to the next bounce (written by shading)
-    uint32_t* scan;    // per block of kLiveBlock paths: live count, then its queue offset
+    uint32_t* scan;    // per block of kLiveBlock paths: live count
     uint32_t* qsorted; // the active queue reordered by material (the shading order)
     uint32_t* keys;    // material key of each active-queue entry
-    uint32_t* bins;    // kSortBins + 1 counters: key histogram, then bucket cursors
+    uint32_t* bins;    // 2 x kSortBins: the keys' histogram, entries placed per key
     const DevJob* jobs;
     uint32_t cap;
     uint32_t aov_stride;
