@@ -1329,9 +1329,7 @@ __global__ void __launch_bounds__(128, 4) k_extend_volume(DevScene S, Wave W, ui
 // through reciprocals, 18.2 with the block's constants.  Blocks per SM 5 / 6 / 7 /
 // 8: 19.2 / 18.2 / 17.7 / 17.3 ms.
 // W.counts[8] is the work cursor (zeroed by k_extend).
-#ifndef DK_VOLUME_MIN_BLOCKS
-#define DK_VOLUME_MIN_BLOCKS 8
-#endif
+constexpr int kVolumeMinBlocks = 8;
 constexpr int kWalkCells = 2;  // cells a lane may walk per step (1 / 2 / 4 / 16: 20.2 / 19.6 / 19.7 / 21.7 ms)
 enum MarchPhase : uint32_t { kMarchIdle, kMarchWalk, kMarchEntry, kMarchBack, kMarchStep, kMarchBisect, kMarchPolish };
 
@@ -1554,7 +1552,7 @@ __device__ __forceinline__ bool marchBegin(MarchState& m, float closest, float u
 }
 
 template <class D>
-__global__ void __launch_bounds__(128, DK_VOLUME_MIN_BLOCKS) k_volume_march(DevScene S, Wave W, uint32_t sel, D dist) {
+__global__ void __launch_bounds__(128, kVolumeMinBlocks) k_volume_march(DevScene S, Wave W, uint32_t sel, D dist) {
     const uint32_t* q = W.q[sel];
     const uint32_t n = W.counts[sel];
     const VolumeScene V = volumeScene(S);

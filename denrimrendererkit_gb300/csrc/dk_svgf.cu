@@ -212,11 +212,9 @@ __device__ __forceinline__ float lg2(float x) {
     asm("lg2.approx.ftz.f32 %0, %1;" : "=f"(r) : "f"(x));
     return r;
 }
-#ifndef DK_SVGF_ROWS
-#define DK_SVGF_ROWS 2  // 1 / 2 / 3 / 4: 524 / 454 / 473 / 552 us a frame
-#endif
+constexpr int kAtrousRows = 2;  // 1 / 2 / 3 / 4: 524 / 454 / 473 / 552 us a frame
 template <int R>
-constexpr int atrousRows() { return R <= 2 ? DK_SVGF_ROWS : 1; }
+constexpr int atrousRows() { return R <= 2 ? kAtrousRows : 1; }
 
 // A pixel of the pass: its depth + normal, luminance, luminance scale (log2
 // units) and sums.
