@@ -548,7 +548,7 @@ def sdf_measure(args, flush, steps=3, warmup=2):
         peak, kind = measured_peaks()
         ext_ms = out["fp16"]["extend_ms"]
         achieved = vol_bytes / (ext_ms * 1e-3) / 1e9
-        roof = {"kernel": "k_extend_volume (volume pass of the extend stage)", "bound": "hbm", "achieved": achieved,
+        roof = {"kernel": "k_volume_march (volume pass of the extend stage)", "bound": "hbm", "achieved": achieved,
                 "peak": peak, "unit": "GB/s", "frac": achieved / peak,
                 "peak_source": f"{kind} (MEASURED_PEAKS.json hbm_gbs)" if kind == "measured" else "fallback 6.8 TB/s",
                 "algorithmic_bytes_per_frame": vol_bytes,
@@ -558,8 +558,8 @@ def sdf_measure(args, flush, steps=3, warmup=2):
                 "units": "16 B per brick sample read, 4 B per grid or macro cell, 128 B per brick descriptor "
                          "(the reference's layouts), counted by the oracle on every 16th pixel in x and y, scaled",
                 "note": "a lower bound of the memory side only: the 92 MB of FP16 samples stay in L2 and the pass "
-                        "is bound by instruction issue and dependent-load latency (ncu, small case: 0.49 TB/s "
-                        "of L2, 41 % issue-active at bounce 0; profiles/k_extend_volume_sdf_spheres.md)"}
+                        "is bound by instruction issue and dependent-load latency (ncu, small case: 1.1 TB/s "
+                        "of L2, 55 % issue-active at bounce 0; profiles/k_volume_march_sdf_spheres.md)"}
     return {"workload": "sdf-spheres 768^3, 8^3 bricks (26.8 K kept, 3 %), 1024x1024 x 16 spp, 8 bounces",
             "value": out["fp16"]["mpaths_s"], "unit": METRIC, "fp16": out["fp16"], "fp32": out["fp32"],
             "fp16_vs_fp32": out["fp16_vs_fp32"], "roofline": roof,
@@ -761,7 +761,7 @@ def unet_inference_measure(reps=10):
     best = out["path3"]
     return {"workload": "5-level U-Net 32-64-96-128-160, one 1920x1088 image, forward", "ms": best["ms"],
             "gflop": flops / 1e9,
-            "roofline": {"kernel": "k_conv3x3_halo (stacked taps) / k_conv3x3_tma (row-tap) / avgpool / upsample "
+            "roofline": {"kernel": "k_conv3x3_halo (stacked taps) / k_conv3x3_tile / k_conv3x3_tma (row-tap) / avgpool / upsample "
                                    "(whole forward pass)", "bound": "tensor",
                          "achieved": best["tflops"], "peak": peak, "unit": "TFLOP/s", "frac": best["tflops"] / peak,
                          "peak_source": f"{kind} (MEASURED_PEAKS.json bf16_tflops)"},
@@ -1054,8 +1054,9 @@ def svgf_timing(width=1920, height=1080, frames=10):
     e1.record()
     torch.cuda.synchronize()
     s.close()
-    return {"ms_per_frame_1080p": e0.elapsed_time(e1) / frames, "launches_per_frame": 9,
-            "note": "pack, temporal, variance, 5 a-trous passes, output copy; synthetic planes, history full"}
+    return {"ms_per_frame_1080p": e0.elapsed_time(e1) / frames, "launches_per_frame": 7,
+            "note": "temporal (with the pack), variance, 5 a-trous passes (the last with the output copy); synthetic "
+                    "planes, history full"}
 
 
 def serve_batches_with_denoising(net, wl, build, plain_spp, batch=8, batches=10):
