@@ -2547,9 +2547,11 @@ int launchConvTile(const ConvArgs& c, cudaStream_t st) {
     a.nSplit = 1u;
     for (uint32_t k = 2u; k <= c.cout / 32u; ++k)
         if (c.cout % (16u * k) == 0u && tiles * k <= sms) a.nSplit = k;
-    while (bytes(1u, c.cout / a.nSplit, 1u, kTileWStagesMin, false) > optin && a.nSplit < c.cout / 16u)
+    while ((c.cout > 256u * a.nSplit || bytes(1u, c.cout / a.nSplit, 1u, kTileWStagesMin, false) > optin) &&
+           a.nSplit < c.cout / 16u)
         do ++a.nSplit;
         while (c.cout % (16u * a.nSplit));
+    if (tiles * a.nSplit >= (1ull << 31)) return kHaloUnfit;
     a.nB = c.cout / a.nSplit;
     if (bytes(1u, a.nB, 1u, kTileWStagesMin, false) > optin) return kHaloUnfit;
     a.cols = (a.nB + 31u) / 32u * 32u;
@@ -2557,9 +2559,9 @@ int launchConvTile(const ConvArgs& c, cudaStream_t st) {
     // Two tiles per item where there are enough of them and they fit with their epilogue's staging.
     const bool pair = tiles * a.nSplit >= 2ull * sms && 4u * a.cols <= 512u &&
                       bytes(2u, a.nB, 1u, kTileWStagesMin, wantStaged) <= optin;
-    // Wide images in single tiles read more weights than the row-tap kernel's rows: 96 to 128 channels at
+    // Wide images in single tiles (up to 256 output channels: the row-tap kernel takes no more) read more weights than the row-tap kernel's rows: 96 to 128 channels at
     // 240 x 136 15.5 against 12.1 us, 224 to 96 at 480 x 272 63 against 52.
-    if (!pair && c.w_ >= 128u) return kHaloUnfit;
+    if (!pair && c.w_ >= 128u && c.cout <= 256u) return kHaloUnfit;
     const uint32_t kT = pair ? 2u : 1u;
     const bool staged = wantStaged && bytes(kT, a.nB, 1u, kTileWStagesMin, true) <= optin;
     a.aSlots = bytes(kT, a.nB, 2u, kTileWStagesMin, staged) <= optin ? 2u : 1u;
@@ -2775,7 +2777,9 @@ int dk_unet_conv3x3(const void* in, uint32_t n, uint32_t h, uint32_t w, uint32_t
     dk::ConvArgs a{static_cast<const bf16*>(in), static_cast<const bf16*>(weight), bias, static_cast<bf16*>(out),
                    n, h, w, cin, ldi, cout, ldo, coOff, (uint32_t)M, act, accumulate};
     cudaStream_t st = static_cast<cudaStream_t>(stream);
-    if (dk::g_convPath == 3 && cout <= 256u) {
+    // More than 256 output channels (one accumulator) go in tiles too, split over CTAs: 128 to 288 channels
+    // on 16 images of 32 x 32 take 21 us, with the mma.sync kernel below 98; 16 to 272 at 480 x 272 83 and 192.
+    if (dk::g_convPath == 3) {
         int rc = dk::launchConvHalo(a, st);
         if (rc == dk::kHaloUnfit) rc = dk::launchConvTile(a, st);
         if (rc != dk::kHaloUnfit) return rc;

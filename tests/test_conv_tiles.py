@@ -55,3 +55,27 @@ def test_tiles_match(lib, n, h, w, cin, cout, pad, accumulate):
     got = outs[0][..., pad:].double()
     # one bf16 rounding of the result (2^-9) over the FP32 sum
     assert float((got - want).norm() / want.norm().clamp(min=1e-30)) <= 2.0 ** -8
+
+
+@pytest.mark.parametrize("n,h,w,cin,cout,accumulate", [
+    (1, 1, 1, 16, 272, 0), (2, 17, 9, 128, 288, 1), (16, 32, 32, 128, 288, 0), (1, 20, 150, 48, 320, 0),
+    (3, 16, 8, 512, 512, 0), (1, 5, 30, 528, 272, 0)])
+def test_more_output_channels_than_one_accumulator(lib, n, h, w, cin, cout, accumulate):
+    g = torch.Generator().manual_seed(cin + cout + w)
+    x = torch.randn(n, h, w, cin, generator=g).to(torch.bfloat16).cuda()
+    weight = (torch.randn(cout, 9, cin, generator=g) / (3 * cin ** 0.5)).to(torch.bfloat16).cuda()
+    bias = torch.randn(cout, generator=g).cuda()
+    prior = torch.randn(n, h, w, cout, generator=g).to(torch.bfloat16).cuda()
+    p = torch.nn.functional.pad(x.double(), (0, 0, 1, 1, 1, 1))
+    want = bias.double() + sum(p[:, dy:dy + h, dx:dx + w] @ weight[:, 3 * dy + dx].double().T
+                               for dy in range(3) for dx in range(3))
+    want = want + prior.double() if accumulate else want.clamp(min=0.0)
+    for path in (3, 0):
+        library.check(lib.dk_unet_set_conv_path(path))
+        out = prior.clone()
+        library.check(lib.dk_unet_conv3x3(x.data_ptr(), n, h, w, cin, cin, weight.data_ptr(), bias.data_ptr(), cout,
+                                          out.data_ptr(), cout, 0, 1 - accumulate, accumulate, None))
+        torch.cuda.synchronize()
+        # one bf16 rounding of the result (2^-9) over the FP32 sum
+        assert float((out.double() - want).norm() / want.norm()) <= 2.0 ** -8
+    library.check(lib.dk_unet_set_conv_path(3))
