@@ -851,6 +851,10 @@ __host__ __device__ constexpr uint32_t tileChunkBytes() {
 }
 
 constexpr uint32_t kTileWStagesMin = 2u;
+// The epilogue's staging: of four warps where the output channels are not split between two.
+__host__ __device__ constexpr uint32_t tileStageBytes(uint32_t nB) {
+    return (epiSplit(nB) ? kEpiWarps : kEpiWarps / 2u) * epiWarpBytes(nB);
+}
 struct TileConvArgs {
     const float* bias;
     __nv_bfloat16* out;
@@ -873,7 +877,7 @@ __global__ void __launch_bounds__(352, 1)
     const uint32_t aBytes = a.chunks * kChunk, wBox = a.nB * 128u, wBytes = kTilePairs * wBox;
     unsigned char* sW = sm + a.aSlots * aBytes;
     unsigned char* sEpi = sW + a.wStages * wBytes;
-    uint64_t* bars = reinterpret_cast<uint64_t*>(sEpi + (a.staged ? kEpiWarps * epiWarpBytes(a.nB) : 0u));
+    uint64_t* bars = reinterpret_cast<uint64_t*>(sEpi + (a.staged ? tileStageBytes(a.nB) : 0u));
     const uint32_t wFull = smemAddr(bars), wEmpty = wFull + 8u * kTileWStagesMax, aFull = wEmpty + 8u * kTileWStagesMax;
     const uint32_t aEmpty = aFull + 16u, accFull = aEmpty + 16u, accEmpty = accFull + 16u;
     uint32_t* table = reinterpret_cast<uint32_t*>(bars + kTileBars);  // per (tap, chunk): A offset | steps << 16 | tap << 20 | chunk << 24
@@ -2539,29 +2543,51 @@ int launchConvTile(const ConvArgs& c, cudaStream_t st) {
     TileConvArgs a;
     auto bytes = [&](uint32_t kT, uint32_t nB, uint32_t aSlots, uint32_t wStages, bool staged) {
         return (size_t)aSlots * chunks * (kT == 2u ? tileChunkBytes<2>() : tileChunkBytes<1>()) +
-               (size_t)wStages * kTilePairs * nB * 128u + (staged ? kEpiWarps * epiWarpBytes(nB) : 0u) + 1024u +
+               (size_t)wStages * kTilePairs * nB * 128u + (staged ? tileStageBytes(nB) : 0u) + 1024u +
                kTileBarBytes;
     };
-    // Output channels per CTA: the most blocks of at least 32 that still find an SM each where the
-    // tiles are few, and more where a block does not fit.
-    a.nSplit = 1u;
-    for (uint32_t k = 2u; k <= c.cout / 32u; ++k)
-        if (c.cout % (16u * k) == 0u && tiles * k <= sms) a.nSplit = k;
-    while ((c.cout > 256u * a.nSplit || bytes(1u, c.cout / a.nSplit, 1u, kTileWStagesMin, false) > optin) &&
-           a.nSplit < c.cout / 16u)
-        do ++a.nSplit;
-        while (c.cout % (16u * a.nSplit));
-    if (tiles * a.nSplit >= (1ull << 31)) return kHaloUnfit;
-    a.nB = c.cout / a.nSplit;
-    if (bytes(1u, a.nB, 1u, kTileWStagesMin, false) > optin) return kHaloUnfit;
-    a.cols = (a.nB + 31u) / 32u * 32u;
     const bool wantStaged = stagedStores(c);
-    // Two tiles per item where there are enough of them and they fit with their epilogue's staging.
-    const bool pair = tiles * a.nSplit >= 2ull * sms && 4u * a.cols <= 512u &&
-                      bytes(2u, a.nB, 1u, kTileWStagesMin, wantStaged) <= optin;
-    // Wide images in single tiles (up to 256 output channels: the row-tap kernel takes no more) read more weights than the row-tap kernel's rows: 96 to 128 channels at
-    // 240 x 136 15.5 against 12.1 us, 224 to 96 at 480 x 272 63 against 52.
-    if (!pair && c.w_ >= 128u && c.cout <= 256u) return kHaloUnfit;
+    // Two tiles per item, which halves the weights read, where there are enough of them and they fit with
+    // their epilogue's staging; on narrow images with the fewest blocks of at least 64 output channels that
+    // fit.  (Smaller blocks, or splitting where that leaves each SM an item or two, are slower: 240 to 96
+    // channels on two images of 35 x 232 21 us, whole single tiles 11; wide images 141 us against the
+    // row-tap kernel's 86, 192 to 128 on 13 of 225 x 82.)
+    bool pair = false;
+    const uint32_t most = c.w_ < 128u && tiles >= 2ull * sms ? std::max(1u, c.cout / 64u) : 1u;
+    for (a.nSplit = 0u; !pair && a.nSplit < most;) {
+        ++a.nSplit;
+        a.nB = c.cout / a.nSplit;
+        pair = c.cout % (16u * a.nSplit) == 0u && a.nB <= 128u && tiles >= 2ull * sms &&
+               bytes(2u, a.nB, 1u, kTileWStagesMin, wantStaged) <= optin;
+    }
+    if (!pair) {
+        // Wide images in single tiles (up to 256 output channels: the row-tap kernel takes no more) read
+        // more weights than the row-tap kernel's rows: 96 to 128 channels at 240 x 136 15.5 against 12.1 us,
+        // 224 to 96 at 480 x 272 63 against 52.
+        if (c.w_ >= 128u && c.cout <= 256u) return kHaloUnfit;
+        // Output channels per CTA: the most blocks of at least 32 that still find an SM each where the
+        // tiles are few, and more where a block does not fit -- with its epilogue's staging while it keeps
+        // 64 channels: 96 to 224 channels on 16 images of 64 x 64 took 60 us with lane-by-lane stores, 30 staged.
+        a.nSplit = 1u;
+        for (uint32_t k = 2u; k <= c.cout / 32u; ++k)
+            if (c.cout % (16u * k) == 0u && tiles * k <= sms) a.nSplit = k;
+        auto fits = [&](uint32_t k, bool staged) {
+            return c.cout % (16u * k) == 0u && c.cout <= 256u * k &&
+                   bytes(1u, c.cout / k, 1u, kTileWStagesMin, staged) <= optin;
+        };
+        uint32_t k = a.nSplit;
+        while (!fits(k, wantStaged) && c.cout >= 64u * (k + 1u)) ++k;
+        if (fits(k, wantStaged)) a.nSplit = k;
+        while (!fits(a.nSplit, false) && a.nSplit < c.cout / 16u) ++a.nSplit;
+        a.nB = c.cout / a.nSplit;
+        if (bytes(1u, a.nB, 1u, kTileWStagesMin, false) > optin) return kHaloUnfit;
+        // Many small blocks (channel counts with few divisors): 16 to 272 channels at 480 x 272 take 124 us
+        // in single tiles, 83 in pairs.
+        pair = a.nB < 64u && tiles * a.nSplit >= 2ull * sms &&
+               bytes(2u, a.nB, 1u, kTileWStagesMin, wantStaged) <= optin;
+    }
+    if (tiles * a.nSplit >= (1ull << 31)) return kHaloUnfit;
+    a.cols = (a.nB + 31u) / 32u * 32u;
     const uint32_t kT = pair ? 2u : 1u;
     const bool staged = wantStaged && bytes(kT, a.nB, 1u, kTileWStagesMin, true) <= optin;
     a.aSlots = bytes(kT, a.nB, 2u, kTileWStagesMin, staged) <= optin ? 2u : 1u;
@@ -2778,7 +2804,7 @@ int dk_unet_conv3x3(const void* in, uint32_t n, uint32_t h, uint32_t w, uint32_t
                    n, h, w, cin, ldi, cout, ldo, coOff, (uint32_t)M, act, accumulate};
     cudaStream_t st = static_cast<cudaStream_t>(stream);
     // More than 256 output channels (one accumulator) go in tiles too, split over CTAs: 128 to 288 channels
-    // on 16 images of 32 x 32 take 21 us, with the mma.sync kernel below 98; 16 to 272 at 480 x 272 83 and 192.
+    // on 16 images of 32 x 32 take 13 us, with the mma.sync kernel below 98; 16 to 272 at 480 x 272 82 and 192.
     if (dk::g_convPath == 3) {
         int rc = dk::launchConvHalo(a, st);
         if (rc == dk::kHaloUnfit) rc = dk::launchConvTile(a, st);

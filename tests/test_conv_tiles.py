@@ -26,7 +26,8 @@ def lib(dk_lib):
 @pytest.mark.parametrize("n,h,w,cin,cout,pad,accumulate", [
     (1, 1, 1, 16, 16, 0, 0), (1, 16, 8, 64, 96, 0, 0), (2, 17, 9, 96, 96, 8, 0), (1, 15, 7, 48, 80, 0, 1),
     (3, 16, 16, 160, 160, 0, 0), (16, 64, 64, 96, 96, 0, 0), (3, 32, 32, 288, 128, 0, 0), (2, 33, 100, 224, 176, 2, 0),
-    (1, 24, 60, 256, 256, 0, 0), (4, 40, 64, 512, 32, 0, 1), (1, 34, 140, 160, 64, 0, 0), (1, 20, 300, 112, 128, 24, 0)])
+    (1, 24, 60, 256, 256, 0, 0), (4, 40, 64, 512, 32, 0, 1), (1, 34, 140, 160, 64, 0, 0), (1, 20, 300, 112, 128, 24, 0),
+    (16, 64, 64, 96, 224, 0, 0), (16, 64, 64, 96, 224, 0, 1), (8, 63, 61, 64, 192, 8, 0)])
 def test_tiles_match(lib, n, h, w, cin, cout, pad, accumulate):
     g = torch.Generator().manual_seed(cin + cout + w)
     x = torch.randn(n, h, w, cin + pad, generator=g).to(torch.bfloat16).cuda()
