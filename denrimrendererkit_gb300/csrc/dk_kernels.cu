@@ -1343,6 +1343,13 @@ __device__ __forceinline__ float divBy(float a, float b, float y) {
     return __fmaf_rn(__fmaf_rn(-b, q, a), y, q);
 }
 
+// The same for a stored distance, which may be as large as FP32 goes: a quotient beyond its range leaves
+// divBy's corrections without a number, and takes the division.
+__device__ __forceinline__ float divDistance(float a, float b, float y) {
+    const float q = divBy(a, b, y);
+    return isfinite(q) ? q : ex::div(a, b);
+}
+
 // The volume's constants of a ray's entry (ddaBegin), computed once per block.
 struct MarchVolume {
     float3 worldMin, worldMax, localMin, extent, rExtent, sampleDen, brick, rBrick;
@@ -1545,7 +1552,7 @@ __device__ __forceinline__ void marchWalk(const VolumeScene& V, const DDAGrid& g
 // The march from the brick's entry (or the point the backward search found):
 // kMarchStep at its first t, or the brick is left without a hit.
 __device__ __forceinline__ bool marchBegin(MarchState& m, float closest, float upw, float rUpw, float minimumStep) {
-    m.t = fmaxf(m.entryT, ex::add(m.lowT, fmaxf(ex::mul(divBy(fabsf(m.lowD), upw, rUpw), 0.9f), minimumStep)));
+    m.t = fmaxf(m.entryT, ex::add(m.lowT, fmaxf(ex::mul(divDistance(fabsf(m.lowD), upw, rUpw), 0.9f), minimumStep)));
     m.count = 0u;
     m.phase = kMarchStep;
     return m.t <= m.tFar && m.t < closest;
@@ -1641,7 +1648,8 @@ __global__ void __launch_bounds__(128, kVolumeMinBlocks) k_volume_march(DevScene
                         } else {
                             m.lowT = m.t;
                             m.lowD = dd;
-                            m.t = ex::add(m.t, fmaxf(ex::mul(divBy(fabsf(dd), s.vr.upw, ray.rUpw), 0.8f), ray.minimumStep));
+                            m.t = ex::add(m.t,
+                                          fmaxf(ex::mul(divDistance(fabsf(dd), s.vr.upw, ray.rUpw), 0.8f), ray.minimumStep));
                             miss = !(++m.count < 192u && m.t <= m.tFar && m.t < s.closest);
                         }
                     } else if (m.phase == kMarchEntry) {
