@@ -269,7 +269,8 @@ __global__ void __launch_bounds__(256) k_svgf_atrous(const float4* __restrict__ 
     constexpr float kLog2e = 1.4426950408889634f;
     constexpr int kRows = atrousRows<R>();
     const int W = (int)p.width, H = (int)p.height, step = p.step;
-    const int x = blockIdx.x * 32 + (threadIdx.x & 31), row = blockIdx.y * 8 + (threadIdx.x >> 5);
+    const int x = blockIdx.x * 32 + (threadIdx.x & 31);
+    const int row = (blockIdx.z * gridDim.y + blockIdx.y) * 8 + (threadIdx.x >> 5);
     const int y0 = (row / step) * step * kRows + row % step;  // uniform over the warp
     if (x >= W || y0 >= H) return;
     const float gpre = 1.0f / (2.0f * p.prefilterSigma * p.prefilterSigma);
@@ -431,7 +432,9 @@ int dk_svgf_denoise(dk_svgf* svgf, const float* beauty, const float* depth, cons
         p.writeHistory = it == 0;
         const int per = r <= 2 ? dk::atrousRows<2>() : dk::atrousRows<4>();
         const uint64_t rows = ((uint64_t)H + p.step * per - 1) / (p.step * per) * p.step;
-        pass[r - 1]<<<dim3((W + 31) / 32, (uint32_t)((rows + 7) / 8)), 256, 0, st>>>(
+        // A grid's y extent ends at 65,535: eight rows a block reach half as far as the other passes' sixteen.
+        const uint32_t blocks = (uint32_t)((rows + 7) / 8), layers = (blocks + 65534u) / 65535u;
+        pass[r - 1]<<<dim3((W + 31) / 32, (blocks + layers - 1u) / layers, layers), 256, 0, st>>>(
             s->work[src], s->var[src], s->dn[c], s->work[1 - src], s->var[1 - src], s->color[c], f4(beauty),
             it == iterations - 1 ? reinterpret_cast<float4*>(out) : nullptr, p);
         src = 1 - src;
