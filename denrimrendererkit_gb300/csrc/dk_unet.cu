@@ -55,6 +55,12 @@ __device__ __forceinline__ void ldmatrixX4(uint32_t& r0, uint32_t& r1, uint32_t&
                  : "r"(smemAddr(p)));
 }
 
+__device__ __forceinline__ void ldmatrixX4T(uint32_t& r0, uint32_t& r1, uint32_t& r2, uint32_t& r3, const void* p) {
+    asm volatile("ldmatrix.sync.aligned.m8n8.x4.trans.shared.b16 {%0, %1, %2, %3}, [%4];\n"
+                 : "=r"(r0), "=r"(r1), "=r"(r2), "=r"(r3)
+                 : "r"(smemAddr(p)));
+}
+
 // D = A (16x16 bf16, row) * B (16x8 bf16, col) + D (fp32).
 __device__ __forceinline__ void mmaBf16(float* d, const uint32_t* a, uint32_t b0, uint32_t b1) {
     asm volatile(
@@ -1765,6 +1771,125 @@ __global__ void __launch_bounds__(128, 1)
     if (warp == 0) asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;\n" ::"r"(taddr), "r"(a.cols));
 }
 
+// The same sums on mma.sync for small problems: blocks of 64 x 64 channels of
+// one tap over a run of pixels, operands by cp.async (zero fill for the padding)
+// through an XOR swizzle that keeps the transposing ldmatrix conflict-free.  It
+// has no set-up and packs the pixels of any image densely: 128 to 128 channels
+// at 32 x 32 take 8.6 us against 18.7 in the kernel above, on 1,531 images of
+// one pixel 8.5 against 64 (launchWgrad chooses).
+struct WgradMmaArgs {
+    const __nv_bfloat16* in;    // [M][ldi], channels [0, cin)
+    const __nv_bfloat16* dout;  // [M][ldd], channels [0, cout)
+    float* dw;                  // [cout][9][cin], accumulated
+    uint32_t n, h, w_, cin, ldi, cout, ldd, M;
+    uint32_t chunk;             // pixels per block (multiple of 32)
+};
+
+constexpr int kWB = 64;  // co and ci per block
+
+// Byte offset of 16-byte chunk `seg` (0..7) of row `r` in a 128-byte-row tile.
+__device__ __forceinline__ uint32_t swz128(uint32_t r, uint32_t seg) { return r * 128u + ((seg ^ (r & 7u)) << 4); }
+
+__global__ void __launch_bounds__(128) k_conv3x3_wgrad_mma(WgradMmaArgs a) {
+    __shared__ __align__(128) unsigned char sA[2][32 * 128];  // [pixel][64 co]
+    __shared__ __align__(128) unsigned char sB[2][32 * 128];  // [pixel][64 ci]
+    const uint32_t tid = threadIdx.x, lane = tid & 31u, warp = tid >> 5;
+    const uint32_t tap = blockIdx.z;
+    const uint32_t ciTiles = (a.cin + kWB - 1) / kWB;
+    const uint32_t co0 = (blockIdx.y / ciTiles) * kWB, ci0 = (blockIdx.y % ciTiles) * kWB;
+    const uint32_t p0 = blockIdx.x * a.chunk, p1 = min(p0 + a.chunk, a.M);
+    const int dy = (int)(tap / 3u) - 1, dx = (int)(tap % 3u) - 1;
+    const uint32_t HW = a.h * a.w_;
+    const uint32_t wm = warp >> 1, wn = warp & 1u;  // 2 x 2 warps of 32 co x 32 ci
+
+    auto loadStage = [&](uint32_t pb, int stage) {
+        // 32 pixels x 8 chunks for each operand: 2 + 2 chunks per thread.
+#pragma unroll
+        for (uint32_t k = 0; k < 2; ++k) {
+            uint32_t i = tid + k * 128u, row = i >> 3, seg = i & 7u;
+            uint32_t p = pb + row;
+            bool pv = p < p1;
+            bool v = pv && co0 + seg * 8u < a.cout;
+            const __nv_bfloat16* src = a.dout + (size_t)p * a.ldd + co0 + seg * 8u;
+            cpAsync16(&sA[stage][swz128(row, seg)], v ? src : a.dout, v ? 16u : 0u);
+            bool vb = false;
+            const __nv_bfloat16* bsrc = a.in;
+            if (pv && ci0 + seg * 8u < a.cin) {
+                uint32_t img = p / HW, rem = p - img * HW;
+                int yy = (int)(rem / a.w_) + dy, xx = (int)(rem % a.w_) + dx;
+                if (yy >= 0 && yy < (int)a.h && xx >= 0 && xx < (int)a.w_) {
+                    vb = true;
+                    bsrc = a.in + ((size_t)(img * a.h + (uint32_t)yy) * a.w_ + (uint32_t)xx) * a.ldi + ci0 + seg * 8u;
+                }
+            }
+            cpAsync16(&sB[stage][swz128(row, seg)], bsrc, vb ? 16u : 0u);
+        }
+    };
+
+    float acc[2][4][4];
+#pragma unroll
+    for (int i = 0; i < 2; ++i)
+#pragma unroll
+        for (int j = 0; j < 4; ++j)
+#pragma unroll
+            for (int k = 0; k < 4; ++k) acc[i][j][k] = 0.0f;
+
+    const uint32_t steps = (p1 > p0) ? (p1 - p0 + 31u) / 32u : 0u;
+    if (steps > 0) loadStage(p0, 0);
+    cpAsyncCommit();
+    for (uint32_t s = 0; s < steps; ++s) {
+        if (s + 1 < steps) loadStage(p0 + (s + 1) * 32u, (int)((s + 1) & 1u));
+        cpAsyncCommit();
+        cpAsyncWait<1>();
+        __syncthreads();
+        const int st = (int)(s & 1u);
+#pragma unroll
+        for (uint32_t kk = 0; kk < 2; ++kk) {  // 16 pixels each
+            uint32_t af[2][4];
+#pragma unroll
+            for (uint32_t mt = 0; mt < 2; ++mt) {
+                // A (co x p) from sA[p][co] through transposed 8x8 loads:
+                // matrices (co 0-7, p 0-7), (co 8-15, p 0-7), (co 0-7, p 8-15), (co 8-15, p 8-15).
+                uint32_t id = lane >> 3;
+                uint32_t prow = kk * 16u + ((id >> 1) << 3) + (lane & 7u);
+                uint32_t seg = (wm * 32u + mt * 16u) / 8u + (id & 1u);
+                ldmatrixX4T(af[mt][0], af[mt][1], af[mt][2], af[mt][3], &sA[st][swz128(prow, seg)]);
+            }
+#pragma unroll
+            for (uint32_t np = 0; np < 2; ++np) {
+                // B (p x ci): matrices (p 0-7, ci 0-7), (p 8-15, ci 0-7), (p 0-7, ci 8-15), (p 8-15, ci 8-15).
+                uint32_t id = lane >> 3;
+                uint32_t prow = kk * 16u + ((id & 1u) << 3) + (lane & 7u);
+                uint32_t seg = (wn * 32u + np * 16u) / 8u + (id >> 1);
+                uint32_t b0, b1, b2, b3;
+                ldmatrixX4T(b0, b1, b2, b3, &sB[st][swz128(prow, seg)]);
+#pragma unroll
+                for (uint32_t mt = 0; mt < 2; ++mt) {
+                    mmaBf16(acc[mt][2 * np], af[mt], b0, b1);
+                    mmaBf16(acc[mt][2 * np + 1], af[mt], b2, b3);
+                }
+            }
+        }
+        __syncthreads();
+    }
+    cpAsyncWait<0>();
+#pragma unroll
+    for (uint32_t mt = 0; mt < 2; ++mt)
+#pragma unroll
+        for (uint32_t half = 0; half < 2; ++half) {
+            uint32_t co = co0 + wm * 32u + mt * 16u + (lane >> 2) + half * 8u;
+            if (co >= a.cout) continue;
+#pragma unroll
+            for (uint32_t nt = 0; nt < 4; ++nt) {
+                uint32_t ci = ci0 + wn * 32u + nt * 8u + (lane & 3u) * 2u;
+                if (ci >= a.cin) continue;
+                float* dst = a.dw + ((size_t)co * 9u + tap) * a.cin + ci;
+                atomicAdd(dst, acc[mt][nt][half * 2 + 0]);
+                atomicAdd(dst + 1, acc[mt][nt][half * 2 + 1]);
+            }
+        }
+}
+
 // ------------------------------------------------------- elementwise ----
 __device__ __forceinline__ uint32_t gid() { return blockIdx.x * blockDim.x + threadIdx.x; }
 __device__ __forceinline__ uint32_t gstride() { return gridDim.x * blockDim.x; }
@@ -2717,6 +2842,25 @@ int launchConvTma(const ConvArgs& c, cudaStream_t st, bool rowTap) {
     return DK_OK;
 }
 
+// Pixels per block of the mma.sync kernel: blocks for the GPU several times over, 256 pixels at least.
+uint32_t wgradMmaChunk(uint64_t M, uint32_t cin, uint32_t cout) {
+    const uint32_t tiles = ((cout + 63u) / 64u) * ((cin + 63u) / 64u);
+    const uint64_t target = (uint64_t)deviceProp().multiProcessorCount * 8u;
+    const uint64_t perTile = (target + 9u * tiles - 1u) / (9u * tiles);
+    const uint64_t chunk = ((M + perTile - 1u) / perTile + 31u) / 32u * 32u;
+    return (uint32_t)std::max<uint64_t>(chunk, 256u);
+}
+
+int launchWgradMma(const __nv_bfloat16* in, uint32_t ldi, const __nv_bfloat16* dout, uint32_t ldd, uint32_t n,
+                   uint32_t h, uint32_t w, uint32_t cin, uint32_t cout, float* dw, cudaStream_t st) {
+    const uint64_t M = (uint64_t)n * h * w;
+    const uint32_t chunk = wgradMmaChunk(M, cin, cout), tiles = ((cout + 63u) / 64u) * ((cin + 63u) / 64u);
+    const WgradMmaArgs a{in, dout, dw, n, h, w, cin, ldi, cout, ldd, (uint32_t)M, chunk};
+    k_conv3x3_wgrad_mma<<<dim3((uint32_t)((M + chunk - 1u) / chunk), tiles, 9), 128, 0, st>>>(a);
+    DK_CUDA(cudaGetLastError(), "conv3x3 wgrad launch");
+    return DK_OK;
+}
+
 // The weight gradient's launch: input blocks per CTA from the accumulator
 // columns (3 x coB per block of 32 channels) and two pipeline stages of shared
 // memory, fewer where the pixel tiles alone would leave SMs idle, two at most.
@@ -2727,8 +2871,6 @@ int launchConvTma(const ConvArgs& c, cudaStream_t st, bool rowTap) {
 // less of a training step's 2.3 ms and differed by up to 3e-5.
 int launchWgrad(const __nv_bfloat16* in, uint32_t ldi, const __nv_bfloat16* dout, uint32_t ldd, uint32_t n, uint32_t h,
                 uint32_t w, uint32_t cin, uint32_t cout, float* dw, cudaStream_t st) {
-    EncodeTiledFn enc = encodeTiled();
-    if (!enc) return fail(DK_ERROR_COMMAND_FAILED, "cuTensorMapEncodeTiled is not available");
     if (deviceProp().multiProcessorCount == 0) ensureDevice();
     const uint32_t sms = (uint32_t)deviceProp().multiProcessorCount;
     const size_t budget = (size_t)deviceProp().sharedMemPerBlockOptin - 1024u - kWgBarBytes;
@@ -2750,6 +2892,20 @@ int launchWgrad(const __nv_bfloat16* in, uint32_t ldi, const __nv_bfloat16* dout
     a.ciGroups = (a.chunks + a.cpc - 1u) / a.cpc;
     a.cpc = (a.chunks + a.ciGroups - 1u) / a.ciGroups;
     const uint32_t groups = coBlocks * a.ciGroups;
+    const uint32_t gx = std::min(a.numTiles, std::max(1u, sms / groups));
+    // Both kernels' times in us, fitted to 260 shapes from 1 x 1 pixel to 16 x 256^2 on 16 to 512 channels (root
+    // mean square errors 7 and 6 %): this one's read-out of 9 x 32 x coB sums a block and its tiles, whatever
+    // part of a tile the image fills, against the other's pixels.  The choice costs 8 % or more on two of
+    // them (19 and 13 %); 128 to 160 channels at 16 x 16 22.8 -> 8.5 us, 80 to 144 on 2 of 20 x 25 24.9 -> 10.4.
+    const uint64_t M = (uint64_t)n * h * w;
+    const float tilesPerCta = (float)((a.numTiles + gx - 1u) / gx), rounds = (float)((gx * (uint64_t)groups + sms - 1u) / sms);
+    const float here = 5.5f + rounds * (0.1f * (float)(a.cpc * a.coB) +
+                                        tilesPerCta * (0.2f + (float)a.cpc * (0.8f + 0.0062f * (float)a.coB)));
+    const float mma = 4.2f + 0.013f * (float)std::min<uint64_t>(M, 256u) +
+                      4.0e-4f * (float)M * (float)(((cin + 63u) / 64u) * ((cout + 63u) / 64u));
+    if (mma < here) return launchWgradMma(in, ldi, dout, ldd, n, h, w, cin, cout, dw, st);
+    EncodeTiledFn enc = encodeTiled();
+    if (!enc) return fail(DK_ERROR_COMMAND_FAILED, "cuTensorMapEncodeTiled is not available");
     a.stages = 2u;
     while (a.stages < kWgStagesMax && (a.stages + 1u) * stageBytes(a.cpc) <= budget) ++a.stages;
     a.cols = 32u;
@@ -2776,7 +2932,6 @@ int launchWgrad(const __nv_bfloat16* in, uint32_t ldi, const __nv_bfloat16* dout
                 "conv3x3 wgrad shared memory");
         configured.store(true);
     }
-    const uint32_t gx = std::min(a.numTiles, std::max(1u, sms / groups));
     k_conv3x3_wgrad<<<dim3(gx, groups), 128, smem, st>>>(mapIn, mapOut, a);
     DK_CUDA(cudaGetLastError(), "conv3x3 wgrad launch");
     return DK_OK;
@@ -2849,6 +3004,8 @@ int dk_unet_conv3x3_wgrad(const void* in, uint32_t ldi, const void* dout, uint32
     if (!in || !dout || !dweight) return dk::fail(DK_ERROR_INVALID_ARGUMENT, "dk_unet_conv3x3_wgrad: null argument");
     if (!dk::aligned16(cin) || !dk::aligned16(cout) || ldi < cin || ldd < cout || ldi % 8u || ldd % 8u)
         return dk::fail(DK_ERROR_INVALID_ARGUMENT, "dk_unet_conv3x3_wgrad: channel counts must be multiples of 16");
+    if (reinterpret_cast<uintptr_t>(in) % 16u || reinterpret_cast<uintptr_t>(dout) % 16u)
+        return dk::fail(DK_ERROR_INVALID_ARGUMENT, "dk_unet_conv3x3_wgrad: tensors must be 16-byte aligned");
     uint64_t M = (uint64_t)n * h * w;
     if (M == 0) return DK_OK;
     if (M >= (1ull << 31)) return dk::fail(DK_ERROR_INVALID_ARGUMENT, "dk_unet_conv3x3_wgrad: tensor too large");

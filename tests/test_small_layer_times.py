@@ -1,0 +1,45 @@
+"""The convolution calls on layers of a few pixels: the kernel that large
+layers want has set-up of its own, which a small one must not pay."""
+import pytest
+
+torch = pytest.importorskip("torch")
+
+from denrimrendererkit_gb300 import DenrimRenderer, library
+
+pytestmark = pytest.mark.gpu
+
+
+@pytest.fixture(scope="module")
+def lib(dk_lib):
+    DenrimRenderer(0)
+    return library.load()
+
+
+def microseconds(call):
+    """Of one call among others on the device (median of 15 runs of ten)."""
+    begin, end = torch.cuda.Event(enable_timing=True), torch.cuda.Event(enable_timing=True)
+    times = []
+    for _ in range(15):
+        torch.cuda._sleep(400_000)  # the launches queue up behind it
+        begin.record()
+        for _ in range(10):
+            call()
+        end.record()
+        torch.cuda.synchronize()
+        times.append(begin.elapsed_time(end) * 100.0)
+    return sorted(times)[7]
+
+
+def weight_gradient(lib, n, h, w, cin, cout):
+    x = torch.randn(n, h, w, cin, device="cuda").to(torch.bfloat16)
+    dy = torch.randn(n, h, w, cout, device="cuda").to(torch.bfloat16)
+    gw = torch.zeros(cout, 9, cin, device="cuda")
+    return lambda: library.check(lib.dk_unet_conv3x3_wgrad(x.data_ptr(), cin, dy.data_ptr(), cout, n, h, w, cin, cout,
+                                                           gw.data_ptr(), None))
+
+
+@pytest.mark.parametrize("small,large", [((1, 8, 8, 128, 128), (16, 64, 64, 128, 128)),
+                                         ((1, 4, 4, 160, 160), (16, 64, 64, 160, 160))])
+def test_small_weight_gradient(lib, small, large):
+    # a 1,024th and a 4,096th of the work; set-up and read-out alone took 0.7 of the large one's time
+    assert microseconds(weight_gradient(lib, *small)) <= 0.4 * microseconds(weight_gradient(lib, *large))
