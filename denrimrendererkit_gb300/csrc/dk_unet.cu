@@ -1631,6 +1631,7 @@ struct WgradArgs {
     uint32_t chunks, cpc, ciGroups;  // 32-channel input blocks: in all, per CTA; groups of them
     uint32_t coB, coChunks;          // output channels per CTA and their 32-channel blocks
     uint32_t stages, cols;
+    uint32_t n, w, h, sets;          // accumulator sets, which take a CTA's tiles in turn
 };
 constexpr uint32_t kWgTile = 16u;                                   // tile edge in pixels
 constexpr uint32_t kWgHalo = kWgTile + 2u;
@@ -1640,6 +1641,51 @@ constexpr uint32_t kWgOutSlot = kWgTile * kWgTile * 64u;
 constexpr uint32_t kWgStagesMax = 4u;
 constexpr uint32_t kWgBarBytes = 128u;
 constexpr uint32_t kWgCoMax = 160u;
+constexpr uint32_t kWgRunMax = 64u;  // tiles of one sum
+
+// Image and first pixel of a tile.  The order goes by kind -- whole tiles, then those cut by the right edge, by the
+// lower edge, by both -- so that the tiles of a CTA, gridDim.x apart, hold the same share of every kind: in row
+// order two CTAs' sums may hold the whole tiles and the slivers of an image 17 pixels wide.
+__device__ __forceinline__ void wgradTile(const WgradArgs& a, uint32_t tile, uint32_t& img, int& x0, int& y0) {
+    const uint32_t fx = a.w / kWgTile, fy = a.h / kWgTile;
+    uint32_t nx = fx, ny = fy, bx = 0u, by = 0u;
+    if (tile >= a.n * fx * fy) {
+        tile -= a.n * fx * fy;
+        const uint32_t right = a.tilesX > fx ? a.n * fy : 0u, lower = a.tilesY > fy ? a.n * fx : 0u;
+        nx = 1u;
+        bx = fx;
+        if (tile >= right) {
+            tile -= right;
+            nx = fx;
+            bx = 0u;
+            ny = 1u;
+            by = fy;
+            if (tile >= lower) {
+                tile -= lower;
+                nx = 1u;
+                bx = fx;
+            }
+        }
+    }
+    const uint32_t tx = tile % nx, rest = tile / nx, ty = rest % ny;
+    img = rest / ny;
+    x0 = (int)((bx + tx) * kWgTile);
+    y0 = (int)((by + ty) * kWgTile);
+}
+
+// Sixteen accumulator columns of a warp's lanes.
+__device__ __forceinline__ void wgradLoad(uint32_t taddr, float (&f)[16]) {
+    uint32_t r[16];
+    asm volatile(
+        "tcgen05.ld.sync.aligned.32x32b.x16.b32 {%0, %1, %2, %3, %4, %5, %6, %7, %8, %9, %10, %11, "
+        "%12, %13, %14, %15}, [%16];\n"
+        : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]), "=r"(r[4]), "=r"(r[5]), "=r"(r[6]), "=r"(r[7]), "=r"(r[8]),
+          "=r"(r[9]), "=r"(r[10]), "=r"(r[11]), "=r"(r[12]), "=r"(r[13]), "=r"(r[14]), "=r"(r[15])
+        : "r"(taddr));
+    asm volatile("tcgen05.wait::ld.sync.aligned;\n" ::: "memory");
+#pragma unroll
+    for (int k = 0; k < 16; ++k) f[k] = __uint_as_float(r[k]);
+}
 
 __global__ void __launch_bounds__(128, 1)
     k_conv3x3_wgrad(const __grid_constant__ CUtensorMap mapIn, const __grid_constant__ CUtensorMap mapOut,
@@ -1687,8 +1733,9 @@ __global__ void __launch_bounds__(128, 1)
                 *abortV = 1;
                 break;
             }
-            const uint32_t tx = tile % a.tilesX, rest = tile / a.tilesX, ty = rest % a.tilesY, img = rest / a.tilesY;
-            const int x0 = (int)(tx * kWgTile), y0 = (int)(ty * kWgTile);
+            uint32_t img;
+            int x0, y0;
+            wgradTile(a, tile, img, x0, y0);
             const uint32_t full = fullBar + 8u * pos.slot, base = smemAddr(sm + pos.slot * stageBytes);
             mbarExpectTx(full, txBytes);
             for (uint32_t c = 0; c < nc; ++c)
@@ -1705,9 +1752,9 @@ __global__ void __launch_bounds__(128, 1)
         const uint32_t hi = (512u >> 4) | (1u << 14) | (4u << 29);
         const uint32_t aLbo = (64u >> 4) << 16, bLbo = (kWgOutSlot >> 4) << 16;
         RingPos pos{0u, 0u};
-        uint32_t acc = 0u;
+        uint32_t t = 0u;
         bool ok = true;
-        for (uint32_t tile = blockIdx.x; tile < a.numTiles; tile += gridDim.x, pos.advance(a.stages)) {
+        for (uint32_t tile = blockIdx.x; tile < a.numTiles; tile += gridDim.x, ++t, pos.advance(a.stages)) {
             if (!mbarWaitWarp(fullBar + 8u * pos.slot, pos.phase)) {
                 ok = false;
                 break;
@@ -1715,9 +1762,10 @@ __global__ void __launch_bounds__(128, 1)
             asm volatile("tcgen05.fence::after_thread_sync;\n" ::: "memory");
             const uint32_t base = smemAddr(sm + pos.slot * stageBytes);
             const uint32_t bLo = (((base + a.cpc * kWgInSlot) & 0x3FFFFu) >> 4) | bLbo;
+            const uint32_t set = a.sets == 2u ? t & 1u : 0u, acc = t >= a.sets ? 1u : 0u;
             for (uint32_t c = 0; c < nc; ++c) {
                 const uint32_t aLo = (((base + c * kWgInSlot) & 0x3FFFFu) >> 4) | aLbo;
-                const uint32_t d = taddr + 3u * c * a.coB;
+                const uint32_t d = taddr + 3u * (set * a.cpc + c) * a.coB;
                 if (electOne()) {
 #pragma unroll
                     for (uint32_t r = 0; r < kWgTile; ++r)
@@ -1728,7 +1776,6 @@ __global__ void __launch_bounds__(128, 1)
                 }
                 __syncwarp();
             }
-            acc = 1u;
             if (electOne()) umaCommit(emptyBar + 8u * pos.slot);
             __syncwarp();
         }
@@ -1741,24 +1788,24 @@ __global__ void __launch_bounds__(128, 1)
     if (!mbarWait(doneBar, 0u)) *abortV = 1;
     asm volatile("tcgen05.fence::after_thread_sync;\n" ::: "memory");
     if (!*abortV && warp < 3u) {
+        const bool second = a.sets == 2u && blockIdx.x + gridDim.x < a.numTiles;  // the CTA's second tile
         for (uint32_t c = 0; c < nc; ++c) {
             const uint32_t ci = (chunk0 + c) * 32u + lane;
             for (uint32_t dy = 0; dy < 3u; ++dy) {
                 for (uint32_t k0 = 0; k0 < a.coB; k0 += 16u) {
-                    uint32_t rr[16];
-                    asm volatile(
-                        "tcgen05.ld.sync.aligned.32x32b.x16.b32 {%0, %1, %2, %3, %4, %5, %6, %7, %8, %9, %10, %11, "
-                        "%12, %13, %14, %15}, [%16];\n"
-                        : "=r"(rr[0]), "=r"(rr[1]), "=r"(rr[2]), "=r"(rr[3]), "=r"(rr[4]), "=r"(rr[5]), "=r"(rr[6]),
-                          "=r"(rr[7]), "=r"(rr[8]), "=r"(rr[9]), "=r"(rr[10]), "=r"(rr[11]), "=r"(rr[12]),
-                          "=r"(rr[13]), "=r"(rr[14]), "=r"(rr[15])
-                        : "r"(taddr + ((warp * 32u) << 16) + (3u * c + dy) * a.coB + k0));
-                    asm volatile("tcgen05.wait::ld.sync.aligned;\n" ::: "memory");
+                    float sum[16];
+                    wgradLoad(taddr + ((warp * 32u) << 16) + (3u * c + dy) * a.coB + k0, sum);
+                    if (second) {
+                        float other[16];
+                        wgradLoad(taddr + ((warp * 32u) << 16) + (3u * (a.cpc + c) + dy) * a.coB + k0, other);
+#pragma unroll
+                        for (uint32_t k = 0; k < 16; ++k) sum[k] += other[k];
+                    }
 #pragma unroll
                     for (uint32_t k = 0; k < 16; ++k) {
                         const uint32_t co = co0 + k0 + k;
                         if (ci < a.cin && co < a.cout)
-                            atomicAdd(a.dw + ((size_t)co * 9u + dy * 3u + warp) * a.cin + ci, __uint_as_float(rr[k]));
+                            atomicAdd(a.dw + ((size_t)co * 9u + dy * 3u + warp) * a.cin + ci, sum[k]);
                     }
                 }
             }
@@ -2876,6 +2923,9 @@ int launchWgrad(const __nv_bfloat16* in, uint32_t ldi, const __nv_bfloat16* dout
     const size_t budget = (size_t)deviceProp().sharedMemPerBlockOptin - 1024u - kWgBarBytes;
     WgradArgs a;
     a.dw = dw;
+    a.n = n;
+    a.w = w;
+    a.h = h;
     a.cin = cin;
     a.cout = cout;
     a.tilesX = (w + kWgTile - 1u) / kWgTile;
@@ -2892,12 +2942,26 @@ int launchWgrad(const __nv_bfloat16* in, uint32_t ldi, const __nv_bfloat16* dout
     a.ciGroups = (a.chunks + a.cpc - 1u) / a.cpc;
     a.cpc = (a.chunks + a.ciGroups - 1u) / a.ciGroups;
     const uint32_t groups = coBlocks * a.ciGroups;
-    const uint32_t gx = std::min(a.numTiles, std::max(1u, sms / groups));
+    // The tensor core truncates when it accumulates, so a gradient's error grows with the K steps of one sum and
+    // falls with the number of sums it is made of.  They are as many as the mma.sync kernel's (runs of up to 512
+    // pixels are not worth a split), a K step with fewer than 16 pixels counting for a third more than its pixels,
+    // and no sum takes more than kWgRunMax tiles.  Where one CTA per SM makes fewer, a CTA sums into two sets of
+    // accumulators if they fit, and then the pixels are split further, in whole rounds of CTAs.
+    const uint64_t M = (uint64_t)n * h * w;
+    const float pieces = (float)M / (float)std::max(wgradMmaChunk(M, cin, cout), 512u);
+    const uint32_t sums = std::max((uint32_t)(pieces * (1.0f + 0.3f * (float)(w % kWgTile) / (float)w)),
+                                   (a.numTiles + kWgRunMax - 1u) / kWgRunMax);
+    uint32_t gx = std::max(1u, sms / groups);
+    a.sets = sums > gx && 6u * a.cpc * a.coB <= 512u ? 2u : 1u;
+    if (sums > gx * a.sets) {
+        const uint64_t splits = (sums + a.sets - 1u) / a.sets, rounds = (splits * groups + sms - 1u) / sms;
+        gx = (uint32_t)std::max<uint64_t>(splits, rounds * sms / groups);
+    }
+    gx = std::min(gx, a.numTiles);
     // Both kernels' times in us, fitted to 260 shapes from 1 x 1 pixel to 16 x 256^2 on 16 to 512 channels (root
     // mean square errors 7 and 6 %): this one's read-out of 9 x 32 x coB sums a block and its tiles, whatever
     // part of a tile the image fills, against the other's pixels.  The choice costs 8 % or more on two of
     // them (19 and 13 %); 128 to 160 channels at 16 x 16 22.8 -> 8.5 us, 80 to 144 on 2 of 20 x 25 24.9 -> 10.4.
-    const uint64_t M = (uint64_t)n * h * w;
     const float tilesPerCta = (float)((a.numTiles + gx - 1u) / gx), rounds = (float)((gx * (uint64_t)groups + sms - 1u) / sms);
     const float here = 5.5f + rounds * (0.1f * (float)(a.cpc * a.coB) +
                                         tilesPerCta * (0.2f + (float)a.cpc * (0.8f + 0.0062f * (float)a.coB)));
@@ -2909,7 +2973,7 @@ int launchWgrad(const __nv_bfloat16* in, uint32_t ldi, const __nv_bfloat16* dout
     a.stages = 2u;
     while (a.stages < kWgStagesMax && (a.stages + 1u) * stageBytes(a.cpc) <= budget) ++a.stages;
     a.cols = 32u;
-    while (a.cols < 3u * a.cpc * a.coB) a.cols <<= 1;
+    while (a.cols < 3u * a.sets * a.cpc * a.coB) a.cols <<= 1;
     alignas(64) CUtensorMap mapIn, mapOut;
     cuuint32_t unit[4] = {1u, 1u, 1u, 1u};
     auto encode = [&](CUtensorMap* map, const __nv_bfloat16* p, uint32_t ld, uint32_t c, uint32_t edge) {
