@@ -2704,6 +2704,38 @@ int launchConvHalo(const ConvArgs& c, cudaStream_t st, __nv_bfloat16* pool = nul
     return DK_OK;
 }
 
+// Output pixels (w x h) of a per-tap tile: 128 columns of a row for the row-tap mode.
+inline uint32_t tapTileWidth(uint32_t w, bool rowTap) {
+    uint32_t tw = 1;
+    while (tw * 2u <= w && tw < 128u) tw *= 2u;
+    return rowTap ? 128u : tw;
+}
+// Estimated time in us of the kernel that takes a layer the tile kernel leaves: row-tap or per-tap up to 256
+// output channels, mma.sync above.  Fitted with convTileTime to 740 pairs of times (400 shapes of 1 x 1 to 544 x 960
+// pixels on 1 to 2,000 images, 16 to 480 channels, with and without staged stores); root mean square errors 12 %
+// (mma.sync 25) and 11 %.  A round is one tile per CTA; its loads and MMAs run beside the previous one's stores.
+float convTapTime(const ConvArgs& c, uint32_t sms, size_t optin) {
+    const uint32_t chunks = (c.cin + 63u) / 64u;
+    if (c.cout > 256u) {
+        const float blocks = (float)((c.M + 127u) / 128u) * (float)c.cout / 64.0f;
+        return 5.9f + 9.0f * (float)c.cin * (0.0095f + 1.28e-4f * blocks);
+    }
+    const bool rowTap = c.w_ >= 128u && tmaSmemBytes(c.cout, false, 2u, true) <= optin;
+    const uint32_t tw = tapTileWidth(c.w_, rowTap), th = 128u / tw;
+    const uint64_t tiles = (uint64_t)c.n * ((c.w_ + tw - 1u) / tw) * ((c.h + th - 1u) / th);
+    const bool staged = stagedStores(c) && tmaSmemBytes(c.cout, true, rowTap ? 2u : kTmaStagesMin, rowTap) <= optin;
+    const float N = (float)c.cout, fill = (float)c.M / (128.0f * (float)tiles);
+    const float mma = 9.0f * (float)chunks * (rowTap ? 0.14f + 4.2e-4f * N : 0.245f + 5.4e-4f * N);
+    return 4.1f + (float)((tiles + sms - 1u) / sms) * std::max(mma, (staged ? 0.044f : 0.107f) * N * fill);
+}
+// The same of the tile kernel: `items` work items of kT tiles, nB output channels each; `pixels` of them in all.
+float convTileTime(const ConvArgs& c, uint32_t sms, uint32_t kT, uint32_t nB, uint64_t items, uint64_t pixels,
+                   bool staged) {
+    const float N = (float)nB, fill = (float)c.M / (float)pixels;
+    const float mma = (float)((c.cin + 63u) / 64u) * (kT == 2u ? 1.9f + 0.0101f * N : 0.84f + 0.0119f * N);
+    return 3.7f + (float)((items + sms - 1u) / sms) * std::max(mma, (staged ? 0.031f : 0.084f) * N * (float)kT * fill);
+}
+
 // The 2-D halo-tile kernel's launch, or kHaloUnfit (nothing launched).
 int launchConvTile(const ConvArgs& c, cudaStream_t st) {
     const uint32_t chunks = (c.cin + 63u) / 64u;
@@ -2776,6 +2808,14 @@ int launchConvTile(const ConvArgs& c, cudaStream_t st) {
     a.tilesX = (c.w_ + kT * kTileW - 1u) / (kT * kTileW);
     a.tilesY = (c.h + kTileH - 1u) / kTileH;
     a.items = c.n * a.tilesX * a.tilesY * a.nSplit;
+    // A tile is 8 x 16 pixels of one image whatever its shape, and a pair twice that: images a few pixels wide or
+    // high go to the other kernels, which take up to 128 of their pixels in a tile (160 to 192 channels on 353 of
+    // 1 x 40: 118 us in tiles, 28 per tap; 176 to 208 on 620 of 33 x 4 210 and 163; 208 to 288 on 1,299 of 3 x 1
+    // 173, mma.sync 35).  Only where the estimates are 5 % apart: that is 69 of the 82 fitted pairs which
+    // tiles slow down by more than 3 %, and one that they speed up (by 4 %).
+    if (convTapTime(c, sms, optin) <
+        0.95f * convTileTime(c, sms, kT, a.nB, a.items, (uint64_t)c.n * a.tilesX * a.tilesY * kT * kTileW * kTileH, staged))
+        return kHaloUnfit;
     a.chunks = chunks;
     a.lastSteps = (c.cin - (chunks - 1u) * 64u + 15u) / 16u;
     a.pairs = 9u * chunks;
@@ -2832,11 +2872,8 @@ int launchConvTma(const ConvArgs& c, cudaStream_t st, bool rowTap) {
     a.coOff = c.coOff;
     a.act = c.act;
     a.accumulate = c.accumulate;
-    uint32_t tw = 1;
-    while (tw * 2u <= c.w_ && tw < 128u) tw *= 2u;
-    if (rowTap) tw = 128u;
-    a.tw = tw;
-    a.th = 128u / tw;
+    a.tw = tapTileWidth(c.w_, rowTap);
+    a.th = 128u / a.tw;
     a.tilesX = (c.w_ + a.tw - 1) / a.tw;
     a.tilesY = (c.h + a.th - 1) / a.th;
     a.numTiles = a.tilesX * a.tilesY * c.n;
