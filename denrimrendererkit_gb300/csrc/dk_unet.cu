@@ -2086,17 +2086,30 @@ __device__ __forceinline__ void st8(__nv_bfloat16* p, const float (&f)[8]) {
     *reinterpret_cast<uint4*>(p) = make_uint4(w[0], w[1], w[2], w[3]);
 }
 
-// The ReLU gradient (kRelu: dpre = dout where out > 0) and/or the bias gradient
-// (kBias: db[c] += the sum of dpre, or of dout itself without kRelu) over
-// groups of 8 channels.  A thread keeps one channel group, so its eight sums
-// stay in registers over its pixels; the block adds its partial sums in shared
-// memory and issues one atomic per channel.  Memory-bound: each operand is
-// read once, whole 64-byte runs of a pixel by neighbouring threads (32
-// channels of 2^20 pixels with both gradients: 36 us, 5.6 TB/s).  Over a
-// 16 x 256^2 training step 341 us; the separate passes with one channel per
-// thread took 236 + 719 us.
+__global__ void k_relu_backward8(const __nv_bfloat16* out, uint32_t ldo, const __nv_bfloat16* dout, uint32_t ldd,
+                                 __nv_bfloat16* dpre, uint32_t ldp, uint32_t groups, uint32_t total) {
+    for (uint32_t i = blockIdx.x * blockDim.x + threadIdx.x; i < total; i += gstride()) {
+        const uint32_t p = i / groups, k = (i - p * groups) * 8u;
+        float o[8], d[8];
+        ld8(out + (size_t)p * ldo + k, o);
+        ld8(dout + (size_t)p * ldd + k, d);
+#pragma unroll
+        for (int j = 0; j < 8; ++j) d[j] = o[j] > 0.0f ? d[j] : 0.0f;
+        st8(dpre + (size_t)p * ldp + k, d);
+    }
+}
+
+// The bias gradient (db[c] += the sum of dout) over groups of 8 channels, with
+// kRelu after the ReLU gradient (dpre = dout where out > 0, summed instead).  A
+// thread keeps one channel group, so its eight sums stay in registers over its
+// pixels; the block adds its partial sums in shared memory and issues one atomic
+// per channel.  Memory-bound: each operand is read once, whole 64-byte runs of a
+// pixel by neighbouring threads (32 channels of 2^20 pixels with both gradients:
+// 36 us, 5.6 TB/s).  Over a 16 x 256^2 training step 341 us; the separate passes
+// with one channel per thread took 236 + 719 us.  (The ReLU gradient alone keeps
+// a group per thread: small tensors 4.4 us against 6.4 in blocks like these.)
 constexpr uint32_t kRbThreads = 256u;
-template <bool kRelu, bool kBias>
+template <bool kRelu>
 __global__ void __launch_bounds__(256) k_relu_bias8(const __nv_bfloat16* out, uint32_t ldo, const __nv_bfloat16* dout,
                                                     uint32_t ldd, __nv_bfloat16* dpre, uint32_t ldp, uint32_t groups,
                                                     uint32_t M, float* db) {
@@ -2116,13 +2129,10 @@ __global__ void __launch_bounds__(256) k_relu_bias8(const __nv_bfloat16* out, ui
                 for (int j = 0; j < 8; ++j) d[j] = o[j] > 0.0f ? d[j] : 0.0f;
                 st8(dpre + (size_t)p * ldp + k, d);
             }
-            if (kBias) {
 #pragma unroll
-                for (int j = 0; j < 8; ++j) s[j] += d[j];
-            }
+            for (int j = 0; j < 8; ++j) s[j] += d[j];
         }
     }
-    if (!kBias) return;
     __shared__ float part[kRbThreads][9];
 #pragma unroll
     for (int j = 0; j < 8; ++j) part[threadIdx.x][j] = s[j];
@@ -2497,14 +2507,14 @@ inline AdamRule adamRule(float lr, float b1, float b2, float eps, uint32_t step)
 
 // k_relu_bias8 over `pixels` pixels of `c` channels: up to six resident blocks
 // per SM, at least eight pixels per thread.
-template <bool kRelu, bool kBias>
+template <bool kRelu>
 int launchReluBias(const void* out, uint32_t ldo, const void* dout, uint32_t ldd, void* dpre, uint32_t ldp, uint32_t c,
                    uint32_t pixels, float* db, void* stream) {
     if (deviceProp().multiProcessorCount == 0) ensureDevice();
     const uint32_t groups = c / 8u, perBlock = kRbThreads / groups * 8u;
     const uint32_t blocks = (uint32_t)(((uint64_t)pixels + perBlock - 1u) / perBlock);
     const uint32_t grid = std::min(blocks, (uint32_t)deviceProp().multiProcessorCount * 6u);
-    k_relu_bias8<kRelu, kBias><<<grid, kRbThreads, 0, static_cast<cudaStream_t>(stream)>>>(
+    k_relu_bias8<kRelu><<<grid, kRbThreads, 0, static_cast<cudaStream_t>(stream)>>>(
         static_cast<const __nv_bfloat16*>(out), ldo, static_cast<const __nv_bfloat16*>(dout), ldd,
         static_cast<__nv_bfloat16*>(dpre), ldp, groups, pixels, db);
     DK_CUDA(cudaGetLastError(), "relu / bias gradient launch");
@@ -3117,9 +3127,14 @@ int dk_unet_conv3x3_wgrad(const void* in, uint32_t ldi, const void* dout, uint32
 int dk_unet_relu_backward(const void* out, uint32_t ldo, const void* dout, uint32_t ldd, void* dpre, uint32_t ldp,
                           uint32_t c, uint32_t pixels, void* stream) {
     if (!out || !dout || !dpre || c % 2u) return dk::fail(DK_ERROR_INVALID_ARGUMENT, "dk_unet_relu_backward");
-    if (c / 8u <= dk::kRbThreads &&
-        dk::vec8({c, ldo, ldd, ldp}, {out, dout, dpre}, (uint64_t)pixels * (c / 8u)))
-        return dk::launchReluBias<true, false>(out, ldo, dout, ldd, dpre, ldp, c, pixels, nullptr, stream);
+    const uint64_t total8 = (uint64_t)pixels * (c / 8u);
+    if (dk::vec8({c, ldo, ldd, ldp}, {out, dout, dpre}, total8)) {
+        dk::k_relu_backward8<<<dk::gridFor(total8), 256, 0, static_cast<cudaStream_t>(stream)>>>(
+            static_cast<const bf16*>(out), ldo, static_cast<const bf16*>(dout), ldd, static_cast<bf16*>(dpre), ldp,
+            c / 8u, (uint32_t)total8);
+        DK_CUDA(cudaGetLastError(), "relu backward launch");
+        return DK_OK;
+    }
     dk::k_relu_backward<<<dk::gridFor((uint64_t)pixels * c / 2), 256, 0, static_cast<cudaStream_t>(stream)>>>(
         static_cast<const bf16*>(out), ldo, static_cast<const bf16*>(dout), ldd, static_cast<bf16*>(dpre), ldp, c,
         pixels);
@@ -3130,7 +3145,7 @@ int dk_unet_relu_backward(const void* out, uint32_t ldo, const void* dout, uint3
 int dk_unet_bias_grad(const void* dpre, uint32_t ld, uint32_t c, uint32_t pixels, float* dbias, void* stream) {
     if (!dpre || !dbias || c == 0 || c > 256u) return dk::fail(DK_ERROR_INVALID_ARGUMENT, "dk_unet_bias_grad");
     if (dk::vec8({c, ld}, {dpre}, (uint64_t)pixels * (c / 8u)))
-        return dk::launchReluBias<false, true>(nullptr, 0, dpre, ld, nullptr, 0, c, pixels, dbias, stream);
+        return dk::launchReluBias<false>(nullptr, 0, dpre, ld, nullptr, 0, c, pixels, dbias, stream);
     uint32_t lanes = 256u / c;
     uint64_t blocks = ((uint64_t)pixels + lanes * 64u - 1) / (lanes * 64u);
     int grid = (int)(blocks < 1 ? 1 : (blocks > 1024 ? 1024 : blocks));
@@ -3145,7 +3160,7 @@ int dk_unet_relu_bias_backward(const void* out, uint32_t ldo, const void* dout, 
     if (!out || !dout || !dpre || !dbias || c == 0 || c % 2u || c > 256u)
         return dk::fail(DK_ERROR_INVALID_ARGUMENT, "dk_unet_relu_bias_backward");
     if (dk::vec8({c, ldo, ldd, ldp}, {out, dout, dpre}, (uint64_t)pixels * (c / 8u)))
-        return dk::launchReluBias<true, true>(out, ldo, dout, ldd, dpre, ldp, c, pixels, dbias, stream);
+        return dk::launchReluBias<true>(out, ldo, dout, ldd, dpre, ldp, c, pixels, dbias, stream);
     const int rc = dk_unet_relu_backward(out, ldo, dout, ldd, dpre, ldp, c, pixels, stream);
     return rc != DK_OK ? rc : dk_unet_bias_grad(dpre, ldp, c, pixels, dbias, stream);
 }
