@@ -645,7 +645,7 @@ int launchWave(const DevScene& S, const Wave& W, uint32_t maxBounces, bool anyDe
         MARK(3);
         DK_CUDA(launchShadow(S, W, S.wide8 ? g.shadow8 : g.shadow, q), "shadow launch");
         DK_CUDA(launchResolve(W, g.final, q), "resolve launch");
-        launches += bounceLaunches(S);
+        launches += bounceLaunches(S, W);
     }
     MARK(0);
     if (anyDenoiser) {

@@ -654,10 +654,15 @@ __global__ void __launch_bounds__(256) k_sort_scatter(Wave W, uint32_t sel) {
 // ------------------------------------------ survivors in path order ----
 // Shading writes a flag per path; the next bounce's queue is the flagged
 // paths in increasing path order: a count per block of kLiveBlock paths, and a
-// scatter of each block's paths after those of the blocks before it, whose
-// counts (a few thousand at most) every block adds up itself.  Path order keeps
-// the extension stage's and (through the stable material sort) the shading
-// stage's path-state accesses coalesced.
+// scatter of each block's paths after those of the blocks before it.  Every
+// block adds up the counts before it itself, which saves a launch of one block
+// while the others wait; the sums grow with the square of the blocks, so waves
+// of more than kLiveDirect blocks (33.5 M paths) run that block's scan: 0.3 % of
+// a frame of 268 M paths, nothing at 34 and 134 M, and bounded at the 537 M that
+// a wave may have.  Path order keeps the extension stage's and (through the
+// stable material sort) the shading stage's path-state accesses coalesced.
+constexpr uint32_t kLiveDirect = 8192u;
+inline uint32_t liveBlocks(const Wave& W) { return (W.path_count + kLiveBlock - 1u) / kLiveBlock; }
 __device__ __forceinline__ uint32_t liveCount16(const Wave& W, uint32_t first, uint32_t n, uint32_t& bits) {
     bits = 0u;
     if (first + 16u <= n) {
@@ -682,14 +687,31 @@ __global__ void __launch_bounds__(256) k_live_count(Wave W) {
     if (threadIdx.x == 0) W.scan[blockIdx.x] = total;
 }
 
+// Exclusive scan of the block counts (one block).
+__global__ void __launch_bounds__(256) k_live_scan(Wave W, uint32_t blocks) {
+    const uint32_t per = (blocks + 255u) / 256u, begin = threadIdx.x * per, end = min(begin + per, blocks);
+    uint32_t sum = 0u, total;
+    for (uint32_t b = begin; b < end; ++b) sum += W.scan[b];
+    uint32_t before = blockExclusiveScan256(sum, total);
+    for (uint32_t b = begin; b < end; ++b) {
+        const uint32_t c = W.scan[b];
+        W.scan[b] = before;
+        before += c;
+    }
+}
+
 __global__ void __launch_bounds__(256) k_live_scatter(Wave W, uint32_t sel) {
     const uint32_t n = W.path_count;
     const uint32_t first = blockIdx.x * kLiveBlock + threadIdx.x * 16u;
     uint32_t bits = 0u, total;
     const uint32_t c = first < n ? liveCount16(W, first, n, bits) : 0u;
     uint32_t sum = 0u, before;
-    for (uint32_t b = threadIdx.x; b < blockIdx.x; b += 256u) sum += W.scan[b];
-    blockExclusiveScan256(sum, before);
+    if (gridDim.x <= kLiveDirect) {
+        for (uint32_t b = threadIdx.x; b < blockIdx.x; b += 256u) sum += W.scan[b];
+        blockExclusiveScan256(sum, before);
+    } else {
+        before = W.scan[blockIdx.x];
+    }
     uint32_t slot = before + blockExclusiveScan256(c, total);
     if (blockIdx.x == gridDim.x - 1u && threadIdx.x == 0u) W.counts[sel ^ 1u] = before + total;  // the next queue's length
     uint32_t* qNext = W.q[sel ^ 1u];
@@ -2392,13 +2414,14 @@ cudaError_t envRotation(float radians, float* sinCos, cudaStream_t st) {
 int g_sortMaterials = -1;  // -1: from DK_SORT_MATERIALS (default on)
 
 // Kernels one bounce launches (extend, shade, shadow, resolve stages).
-uint32_t bounceLaunches(const DevScene& S) {
+uint32_t bounceLaunches(const DevScene& S, const Wave& W) {
     if (g_sortMaterials < 0) {
         const char* e = getenv("DK_SORT_MATERIALS");
         g_sortMaterials = (e && e[0] == '0') ? 0 : 1;
     }
     uint32_t n = 1u + (S.volume_count ? 1u : 0u);                  // extend
     n += (g_sortMaterials ? 2u : 0u) + (S.has_subsurface && !S.volume_count && !S.wide8 ? 2u : 1u) + 2u;  // sort, (walk,) shade, survivors
+    n += liveBlocks(W) > kLiveDirect ? 1u : 0u;
     n += 1u + ((!S.all_shadow_opaque || S.volume_count) ? 1u : 0u);  // shadow
     return n + 1u;                                                   // resolve
 }
@@ -2432,9 +2455,10 @@ cudaError_t launchShade(const DevScene& S, const Wave& W, uint32_t bounce, uint3
         k_shade<false><<<grid, shadeBlock<false>(), 0, st>>>(S, W, bounce, sel, sorted);
     }
     // The survivors, in path order, are the next bounce's queue.
-    const uint32_t blocks = (W.path_count + kLiveBlock - 1u) / kLiveBlock;
+    const uint32_t blocks = liveBlocks(W);
     if (blocks) {
         k_live_count<<<blocks, 256, 0, st>>>(W);
+        if (blocks > kLiveDirect) k_live_scan<<<1, 256, 0, st>>>(W, blocks);
         k_live_scatter<<<blocks, 256, 0, st>>>(W, sel);
     }
     return cudaGetLastError();

@@ -128,7 +128,7 @@ struct Wave {
     uint2* layer_hits;      // kRecLayers per shadow-ray slot: (t bits, triangle slot) of crossed non-opaque triangles
     uint32_t* layer_count;  // per shadow-ray slot: recorded layers, bit 31 = more than kRecLayers
     uint8_t* live;     // per path: 1 when it goes on to the next bounce (written by shading)
-    uint32_t* scan;    // per block of kLiveBlock paths: live count
+    uint32_t* scan;    // per block of kLiveBlock paths: live count (in large waves, then the counts before it)
     uint32_t* qsorted; // the active queue reordered by material (the shading order)
     uint32_t* keys;    // material key of each active-queue entry
     uint32_t* bins;    // 2 x kSortBins: the keys' histogram, entries placed per key
@@ -164,7 +164,7 @@ cudaError_t launchAovPrimary(const DevScene& S, const Wave& W, int grid, cudaStr
 cudaError_t launchPreview(const DevScene& S, const DevParams& P, const Accum& A, uint32_t matCount,
                           uint32_t opaqueMask, bool interactive, cudaStream_t st);
 cudaError_t launchFinalize(const Wave& W, int grid, cudaStream_t st);
-uint32_t bounceLaunches(const DevScene& S);
+uint32_t bounceLaunches(const DevScene& S, const Wave& W);
 cudaError_t envRotation(float radians, float* sinCos /* device, 2 floats */, cudaStream_t st);
 cudaError_t launchResolveBeauty(const Accum& A, uint32_t pixels, float4* out, int grid, cudaStream_t st);
 cudaError_t buildEnvironmentTable(const float4* dPixels, uint32_t w, uint32_t h, float intensity, float maxR,
