@@ -12,7 +12,6 @@
 //             tap-flipped, transposed weights;
 //   wgrad     dW[co][tap][ci] += sum_p dOut[p][co] in[p + tap][ci]
 //             M = taps x Cin, N = Cout, K = pixels, split over CTAs.
-#include <atomic>
 #include <cstdint>
 #include <cstdlib>
 #include <initializer_list>
@@ -21,6 +20,7 @@
 #include <cuda_bf16.h>
 
 #include "dk_host.h"
+#include "dk_smem_limit.h"
 
 namespace dk {
 namespace {
@@ -2568,6 +2568,17 @@ EncodeTiledFn encodeTiled() {
     return fn;
 }
 
+// The current device's opt-in shared memory for `kernel`, once per device.
+template <typename... KArgs>
+cudaError_t raiseSmemLimit(SmemLimit& limit, void (*kernel)(KArgs...)) {
+    int device = 0;
+    if (const cudaError_t e = cudaGetDevice(&device)) return e;
+    return (cudaError_t)limit.raise(device, [&] {
+        return cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                    (int)deviceProp().sharedMemPerBlockOptin);
+    });
+}
+
 // Pipeline depth limit from the environment (a tuning knob, read at each
 // launch), clamped to [lo, hi]; hi when unset.
 uint32_t depthCap(const char* name, uint32_t lo, uint32_t hi) {
@@ -2701,12 +2712,8 @@ int launchConvHalo(const ConvArgs& c, cudaStream_t st, __nv_bfloat16* pool = nul
          {k_conv3x3_halo<true, 2, 1>, k_conv3x3_halo<true, 2, 2>, k_conv3x3_halo<true, 2, 3>,
           k_conv3x3_halo<true, 2, 4>}}};
     HaloKernel kernel = kernels[stack][chunks - 1u][last - 1u];
-    static size_t configured[2][2][4] = {};
-    if (smem > configured[stack][chunks - 1u][last - 1u]) {
-        DK_CUDA(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem),
-                "conv3x3 (halo) shared memory");
-        configured[stack][chunks - 1u][last - 1u] = smem;
-    }
+    static SmemLimit limits[2][2][4];
+    DK_CUDA(raiseSmemLimit(limits[stack][chunks - 1u][last - 1u], kernel), "conv3x3 (halo) shared memory");
     uint32_t grid = std::min(sms, a.totalRows);
     DK_CUDA(launchPdl(kernel, dim3(grid), dim3(320), smem, st, mapIn, mapW, mapOut, a), "conv3x3 (halo) launch");
     DK_CUDA(cudaGetLastError(), "conv3x3 (halo rows, TMA + tcgen05) launch");
@@ -2851,13 +2858,8 @@ int launchConvTile(const ConvArgs& c, cudaStream_t st) {
             CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_256B,
             CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
     if (r != CUDA_SUCCESS) return fail(DK_ERROR_INVALID_ARGUMENT, "weight tensor map rejected");
-    static std::atomic<bool> configured[2];  // one size for every call: threads may set it twice
-    if (!configured[pair].load()) {
-        DK_CUDA(cudaFuncSetAttribute(pair ? k_conv3x3_tile<2> : k_conv3x3_tile<1>,
-                                     cudaFuncAttributeMaxDynamicSharedMemorySize, (int)optin),
-                "conv3x3 (tiles) shared memory");
-        configured[pair].store(true);
-    }
+    static SmemLimit limits[2];
+    DK_CUDA(raiseSmemLimit(limits[pair], pair ? k_conv3x3_tile<2> : k_conv3x3_tile<1>), "conv3x3 (tiles) shared memory");
     const dim3 grid(std::min(sms, a.items));
     DK_CUDA(launchPdl(pair ? k_conv3x3_tile<2> : k_conv3x3_tile<1>, grid, dim3(352), smem, st, mapIn, mapW, a),
             "conv3x3 (tiles) launch");
@@ -2919,13 +2921,8 @@ int launchConvTma(const ConvArgs& c, cudaStream_t st, bool rowTap) {
     a.staged = staged ? 1 : 0;
     a.stages = stages;
     size_t smem = tmaSmemBytes(c.cout, staged, stages, rowTap);
-    static size_t configured[2] = {0, 0};
-    if (smem > configured[rowTap]) {
-        DK_CUDA(cudaFuncSetAttribute(rowTap ? k_conv3x3_tma<true> : k_conv3x3_tma<false>,
-                                     cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem),
-                "conv3x3 shared memory");
-        configured[rowTap] = smem;
-    }
+    static SmemLimit limits[2];
+    DK_CUDA(raiseSmemLimit(limits[rowTap], rowTap ? k_conv3x3_tma<true> : k_conv3x3_tma<false>), "conv3x3 shared memory");
     uint32_t grid = (uint32_t)deviceProp().multiProcessorCount;
     if (grid > a.numTiles) grid = a.numTiles;
     if (rowTap)
@@ -3036,13 +3033,8 @@ int launchWgrad(const __nv_bfloat16* in, uint32_t ldi, const __nv_bfloat16* dout
     if (encode(&mapOut, dout, ldd, cout, kWgTile) != CUDA_SUCCESS)
         return fail(DK_ERROR_INVALID_ARGUMENT, "gradient tensor map rejected");
     const size_t smem = a.stages * stageBytes(a.cpc) + 1024u + kWgBarBytes;
-    static std::atomic<bool> configured;  // one size for every call: threads may set it twice
-    if (!configured.load()) {
-        DK_CUDA(cudaFuncSetAttribute(k_conv3x3_wgrad, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                     (int)deviceProp().sharedMemPerBlockOptin),
-                "conv3x3 wgrad shared memory");
-        configured.store(true);
-    }
+    static SmemLimit limit;
+    DK_CUDA(raiseSmemLimit(limit, k_conv3x3_wgrad), "conv3x3 wgrad shared memory");
     k_conv3x3_wgrad<<<dim3(gx, groups), 128, smem, st>>>(mapIn, mapOut, a);
     DK_CUDA(cudaGetLastError(), "conv3x3 wgrad launch");
     return DK_OK;
@@ -3085,12 +3077,8 @@ int dk_unet_conv3x3(const void* in, uint32_t n, uint32_t h, uint32_t w, uint32_t
         uint32_t cols = 32u;
         while (cols < cout) cols <<= 1;
         size_t smem = dk::tcSmemBytes(cout);
-        static size_t configured = 0;
-        if (smem > configured) {
-            DK_CUDA(cudaFuncSetAttribute(dk::k_conv3x3_tc, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem),
-                    "conv3x3 shared memory");
-            configured = smem;
-        }
+        static dk::SmemLimit limit;
+        DK_CUDA(dk::raiseSmemLimit(limit, dk::k_conv3x3_tc), "conv3x3 shared memory");
         dk::k_conv3x3_tc<<<(uint32_t)((M + dk::kTcRows - 1) / dk::kTcRows), 128, smem, st>>>(a, cols);
         DK_CUDA(cudaGetLastError(), "conv3x3 (tcgen05) launch");
         return DK_OK;
