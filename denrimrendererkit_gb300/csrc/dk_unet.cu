@@ -886,7 +886,7 @@ __global__ void __launch_bounds__(352, 1)
     uint64_t* bars = reinterpret_cast<uint64_t*>(sEpi + (a.staged ? tileStageBytes(a.nB) : 0u));
     const uint32_t wFull = smemAddr(bars), wEmpty = wFull + 8u * kTileWStagesMax, aFull = wEmpty + 8u * kTileWStagesMax;
     const uint32_t aEmpty = aFull + 16u, accFull = aEmpty + 16u, accEmpty = accFull + 16u;
-    uint32_t* table = reinterpret_cast<uint32_t*>(bars + kTileBars);  // per (tap, chunk): A offset | steps << 16 | tap << 20 | chunk << 24
+    uint32_t* table = reinterpret_cast<uint32_t*>(bars + kTileBars);  // the (tap, chunk) order of the weight boxes: tap | chunk << 8
     uint32_t* tslot = table + 9u * kTileChunksMax;
     int* abortFlag = reinterpret_cast<int*>(tslot + 1);
     const uint32_t tid = threadIdx.x, lane = tid & 31u, warp = __shfl_sync(0xffffffffu, tid >> 5, 0);
@@ -924,8 +924,7 @@ __global__ void __launch_bounds__(352, 1)
             tap = tid / a.chunks;
             c = tid - tap * a.chunks;
         }
-        const uint32_t off = c * (kChunk >> 4) + ((tap / 3u) * kPitch + tap % 3u) * 8u;
-        table[tid] = off | ((c + 1u < a.chunks ? 4u : a.lastSteps) << 16) | (tap << 20) | (c << 24);
+        table[tid] = tap | (c << 8);
     }
     __syncthreads();
     asm volatile("tcgen05.fence::after_thread_sync;\n" ::: "memory");
@@ -952,8 +951,8 @@ __global__ void __launch_bounds__(352, 1)
 #pragma unroll
                     for (uint32_t j = 0; j < kTilePairs; ++j) {
                         const uint32_t e = table[s * kTilePairs + j];
-                        tmaLoad3(smemAddr(sW + pos.slot * wBytes + j * wBox), &mapW, (int)((e >> 24) * 64u),
-                                 (int)((e >> 20) & 15u), co0, full);
+                        tmaLoad3(smemAddr(sW + pos.slot * wBytes + j * wBox), &mapW, (int)((e >> 8) * 64u),
+                                 (int)(e & 255u), co0, full);
                     }
                 }
             }
@@ -2409,7 +2408,7 @@ struct AdamTable {
     uint32_t groups;
 };
 __global__ void __launch_bounds__(256) k_adam_groups(const __grid_constant__ AdamTable t, AdamRule rule) {
-    __shared__ __nv_bfloat16 tile[32][36];  // [ci][co], rows of 72 bytes
+    __shared__ __align__(8) __nv_bfloat16 tile[32][36];  // [ci][co], rows of 72 bytes, read in 8-byte pieces
     uint32_t lo = 0, hi = t.groups - 1u;
     while (lo < hi) {
         const uint32_t mid = (lo + hi + 1u) >> 1;
