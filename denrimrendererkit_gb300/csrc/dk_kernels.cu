@@ -1365,12 +1365,9 @@ __device__ __forceinline__ float divBy(float a, float b, float y) {
     return __fmaf_rn(__fmaf_rn(-b, q, a), y, q);
 }
 
-// The same for a stored distance, which may be as large as FP32 goes: a quotient beyond its range leaves
-// divBy's corrections without a number, and takes the division.
-__device__ __forceinline__ float divDistance(float a, float b, float y) {
-    const float q = divBy(a, b, y);
-    return isfinite(q) ? q : ex::div(a, b);
-}
+// The same for a finite distance a >= 0, which may be as large as FP32 goes: where the quotient leaves its
+// range the corrections give no number, and it is infinite.
+__device__ __forceinline__ float divDistance(float a, float b, float y) { return fminf(divBy(a, b, y), INFINITY); }
 
 // The volume's constants of a ray's entry (ddaBegin), computed once per block.
 struct MarchVolume {
