@@ -1999,7 +1999,7 @@ __device__ __forceinline__ void storePreview(const Accum& A, size_t pix, float4 
     A.count[pix] = 1u;
 }
 
-// One thread per pixel, a warp per 8 x 4 pixels.  The kernel is bound by
+// One thread per pixel.  The kernel is bound by
 // instruction fetch: some 400 KB of code, of which every warp runs a large
 // part once, so warps at different places evict each other's instructions (a
 // version without barriers spent 31 of 36 cycles between a warp's issues
@@ -2013,22 +2013,36 @@ __device__ __forceinline__ void storePreview(const Accum& A, size_t pix, float4 
 // probes bounded by their radius; 2.7 with the environment lookup called;
 // 0.78 with the phases.  Blocks x minimum residency 128 x 4 / 256 x 2 / 512 x 1 /
 // 512 x 2 / 1024 x 1: 1.22 / 0.99 / 1.03 / 0.78 / 0.82 ms.
-#ifndef DK_PREVIEW_BLOCK
-#define DK_PREVIEW_BLOCK 512
-#endif
-#ifndef DK_PREVIEW_MIN_BLOCKS
-#define DK_PREVIEW_MIN_BLOCKS 2
-#endif
-template <bool kInteractive>
-__global__ void __launch_bounds__(DK_PREVIEW_BLOCK, DK_PREVIEW_MIN_BLOCKS)
+// Frames that do not fill the SMs with such blocks, and volume walks, whose
+// lanes differ too much to wait for each other, lose by it: they run in blocks
+// of 128 threads, or of one warp (launchPreview), with 128 registers or more.
+// A warp has 8 x 4 pixels, in blocks of one warp 32 in a row, which spread a
+// surface's expensive pixels over more warps.
+// The interactive kernels stay within 128 registers: with more, a product is
+// fused differently and the last bits of a frame change.
+constexpr uint32_t kPreviewLarge = 512u, kPreviewMid = 128u, kPreviewSmall = 32u;
+template <bool kInteractive, uint32_t kBlock>
+constexpr uint32_t previewResidency() {
+    return kBlock == kPreviewLarge ? 2u : kInteractive || kBlock == kPreviewMid ? 512u / kBlock : 1u;
+}
+template <bool kInteractive, uint32_t kBlock>
+__global__ void __launch_bounds__(kBlock, previewResidency<kInteractive, kBlock>())
     k_preview(const __grid_constant__ DevScene S, const __grid_constant__ DevParams P, Accum A, MatTable mt,
               uint32_t opaqueMask) {
     const size_t plane = (size_t)P.width * P.height;
     __shared__ float3 axisEnv[6];
     if (kInteractive) loadAxisEnvironment(S, axisEnv);
-    const uint32_t lane = laneId(), warp = (blockIdx.x * DK_PREVIEW_BLOCK + threadIdx.x) >> 5;
-    const uint32_t tilesX = (P.tile_w + 7u) / 8u;
-    const uint32_t lx = (warp % tilesX) * 8u + (lane & 7u), ly = (warp / tilesX) * 4u + (lane >> 3);
+    uint32_t lx, ly;
+    if constexpr (kBlock == kPreviewSmall) {
+        const uint32_t i = blockIdx.x * kBlock + threadIdx.x;
+        lx = i % P.tile_w;
+        ly = i / P.tile_w;
+    } else {
+        const uint32_t lane = laneId(), warp = (blockIdx.x * kBlock + threadIdx.x) >> 5;
+        const uint32_t tilesX = (P.tile_w + 7u) / 8u;
+        lx = (warp % tilesX) * 8u + (lane & 7u);
+        ly = (warp / tilesX) * 4u + (lane >> 3);
+    }
     const bool valid = lx < P.tile_w && ly < P.tile_h;
     // Threads outside the tile, and later those whose ray missed, run the block's
     // phases on a neighbour's pixel or hit and store nothing of them.
@@ -2482,13 +2496,22 @@ cudaError_t launchAovPrimary(const DevScene& S, const Wave& W, int grid, cudaStr
 cudaError_t launchPreview(const DevScene& S, const DevParams& P, const Accum& A, uint32_t matCount,
                           uint32_t opaqueMask, bool interactive, cudaStream_t st) {
     const MatTable mt{0u, matCount};
-    const uint64_t warps = (uint64_t)((P.tile_w + 7u) / 8u) * ((P.tile_h + 3u) / 4u);
-    const uint32_t grid = (uint32_t)((warps * 32u + DK_PREVIEW_BLOCK - 1u) / DK_PREVIEW_BLOCK);
-    if (!grid) return cudaSuccess;
-    if (interactive)
-        k_preview<true><<<grid, DK_PREVIEW_BLOCK, 0, st>>>(S, P, A, mt, opaqueMask);
-    else
-        k_preview<false><<<grid, DK_PREVIEW_BLOCK, 0, st>>>(S, P, A, mt, opaqueMask);
+    const uint64_t pixels = (uint64_t)P.tile_w * P.tile_h;
+    if (!pixels) return cudaSuccess;
+    // us a frame, blocks of 32 / 128 / 512 threads (a general loop of 128 before them all), interactive quality:
+    // material scene 200 x 150 173 / 177 / 223 (269), 400 x 300 282 / 208 / 232 (605), 640 x 360 450 / 302 / 247;
+    // 82,000 triangles 64 x 64 631 / 707 / 972 (658), 400 x 300 1015 / 967 / 1214, 640 x 360 1614 / 1333 / 1188;
+    // 768^3 volume 200 x 150 831 / 1095 / 1717 (882), 1280 x 720 2449 / 1856 / 2754.  Preview quality likewise.
+    const uint64_t small = S.volume_count ? 150000u : 40000u;
+    const uint32_t block = pixels < small ? kPreviewSmall
+                           : S.volume_count || pixels < 200000u ? kPreviewMid : kPreviewLarge;
+    const uint64_t warps = block == kPreviewSmall ? (pixels + 31u) / 32u
+                                                  : (uint64_t)((P.tile_w + 7u) / 8u) * ((P.tile_h + 3u) / 4u);
+    const uint32_t grid = (uint32_t)((warps * 32u + block - 1u) / block);
+    auto kernel = block == kPreviewLarge ? (interactive ? k_preview<true, kPreviewLarge> : k_preview<false, kPreviewLarge>)
+                  : block == kPreviewMid ? (interactive ? k_preview<true, kPreviewMid> : k_preview<false, kPreviewMid>)
+                                         : (interactive ? k_preview<true, kPreviewSmall> : k_preview<false, kPreviewSmall>);
+    kernel<<<grid, block, 0, st>>>(S, P, A, mt, opaqueMask);
     return cudaGetLastError();
 }
 cudaError_t launchFinalize(const Wave& W, int grid, cudaStream_t st) {
