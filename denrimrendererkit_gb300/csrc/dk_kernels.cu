@@ -784,12 +784,16 @@ __global__ void __launch_bounds__(128) k_subsurface_walk(DevScene S, Wave W, uin
         }
         if (__all_sync(0xffffffffu, i == kNoWork && exhausted)) break;
         // Advance the rays until as many lanes wait (for their event or for a new
-        // path) as run: events are long code, worth sharing.
+        // path) as run, and to the last one once no new paths are left: events are
+        // long code, worth sharing (the material scene, 1024 x 1024 x 1 spp, whose
+        // paths are all fetched at once: 3.82 -> 3.73 ms a frame with the second).
         bool running = i != kNoWork;
+        const bool last = __any_sync(0xffffffffu, exhausted);
         for (;;) {
             int count;
             const bool nodes = majorityStep(running, st.node, count);
-            if (__popc(__ballot_sync(0xffffffffu, !running && !(i == kNoWork && exhausted))) >= count) break;
+            const int waiting = __popc(__ballot_sync(0xffffffffu, !running && !(i == kNoWork && exhausted)));
+            if (last ? count == 0 : waiting >= count) break;
             const bool leaf = (st.node & kLeafBit) != 0u;
             if (!running || nodes == leaf) continue;
             running = leaf ? closestTriStep(S, st, stackNode, stackT) : closestNodeStep(S, st, stackNode, stackT);
