@@ -2034,8 +2034,6 @@ __global__ void __launch_bounds__(kBlock, previewResidency<kInteractive, kBlock>
     k_preview(const __grid_constant__ DevScene S, const __grid_constant__ DevParams P, Accum A, MatTable mt,
               uint32_t opaqueMask) {
     const size_t plane = (size_t)P.width * P.height;
-    __shared__ float3 axisEnv[6];
-    if (kInteractive) loadAxisEnvironment(S, axisEnv);
     uint32_t lx, ly;
     if constexpr (kBlock == kPreviewSmall) {
         const uint32_t i = blockIdx.x * kBlock + threadIdx.x;
@@ -2079,6 +2077,8 @@ __global__ void __launch_bounds__(kBlock, previewResidency<kInteractive, kBlock>
     }
     if (firstHit == 0xffffffffu) return;
     if (!hit) rec = sharedHit;
+    __shared__ float3 axisEnv[6];
+    if (kInteractive) loadAxisEnvironment(S, axisEnv);
 
     Hit h = makeHitAny(S, ray, rec);
     Material m = materialForHit(S, mt, h);
