@@ -42,7 +42,7 @@ def build(force: bool = False, verbose: bool = False) -> str:
     # reference's arithmetic operation by operation, like the oracle.
     flags = [*ARCH, "-lineinfo", "-O3", "-std=c++17", "-Xcompiler", "-fPIC", "-Xcompiler", "-pthread",
              "-Xcompiler", "-ffp-contract=off", "--expt-relaxed-constexpr"]
-    # Tuning knobs, e.g. DK_NVCC_DEFINES="DK_SHADE_MIN_BLOCKS=6 DK_LAYERS_MIN_BLOCKS=4".
+    # Tuning knobs, e.g. DK_NVCC_DEFINES="DK_SHADE_WARPS=24 DK_LAYERS_MIN_BLOCKS=5".
     flags += [f"-D{d}" for d in os.environ.get("DK_NVCC_DEFINES", "").split()]
 
     def compile_one(src: str) -> str:
