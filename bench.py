@@ -436,7 +436,7 @@ def run_gb300(args, rank, world, local):
                 "frac": achieved / peak, "peak_source": f"{kind} (MEASURED_PEAKS.json hbm_gbs)" if kind == "measured"
                 else "fallback 6.8 TB/s", "traffic": traffic,
                 "units": "achieved and traffic are per step (one frame, all launches of the stage); traffic = "
-                         "DRAM read+write bytes scaled from a small-case ncu capture (profiles/<stage>_spheres_large.md)",
+                         "DRAM read+write bytes scaled from a small-case ncu capture of the stage",
                 "algorithmic_bytes_per_step": {k: float(v) for k, v in per_frame.items()},
                 "kernel_ms_per_step": kernel_ms, "slowest_stage": max(kernel_ms, key=kernel_ms.get),
                 "per_path": {k: float(v) / paths for k, v in counters.items() if k != "paths"}}
@@ -559,7 +559,7 @@ def sdf_measure(args, flush, steps=3, warmup=2):
                          "(the reference's layouts), counted by the oracle on every 16th pixel in x and y, scaled",
                 "note": "a lower bound of the memory side only: the 92 MB of FP16 samples stay in L2 and the pass "
                         "is bound by instruction issue and dependent-load latency (ncu, small case: 1.1 TB/s "
-                        "of L2, 55 % issue-active at bounce 0; profiles/k_volume_march_sdf_spheres.md)"}
+                        "of L2, 55 % issue-active at bounce 0)"}
     return {"workload": "sdf-spheres 768^3, 8^3 bricks (26.8 K kept, 3 %), 1024x1024 x 16 spp, 8 bounces",
             "value": out["fp16"]["mpaths_s"], "unit": METRIC, "fp16": out["fp16"], "fp32": out["fp32"],
             "fp16_vs_fp32": out["fp16_vs_fp32"], "roofline": roof,

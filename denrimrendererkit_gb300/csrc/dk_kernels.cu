@@ -529,8 +529,8 @@ __global__ void __launch_bounds__(128) k_extend(DevScene S, Wave W, uint32_t sel
 // change any result: every path carries its own RNG state and pixel samples
 // are accumulated in sample order.
 // Keys: 0 a miss, 1 + material ID (at most kSortBins - 3), kSortBins - 2 a
-// material with a subsurface weight (shaded by the kernel that carries the
-// subsurface random walk), kSortBins - 1 a distance-volume hit.
+// material with a subsurface weight (where k_subsurface_walk begins),
+// kSortBins - 1 a distance-volume hit.
 constexpr uint32_t kSubsurfaceKey = kSortBins - 2u;
 __device__ __forceinline__ uint32_t shadeKey(const DevScene& S, const Wave& W, uint32_t p) {
     uint32_t tri = __float_as_uint(W.hit[p].y);
@@ -726,9 +726,9 @@ __global__ void __launch_bounds__(256) k_live_scatter(Wave W, uint32_t sel) {
 // continueSubsurfaceRandomWalk (PathTrace.metal:3525-3621) for the paths whose
 // material has a subsurface weight, ahead of the shading kernel: up to eight
 // rays inside the surface per path.  Persistent threads with per-lane refill,
-// like k_extend: a lane advances its ray a bounded number of visits, and when
-// the ray is done scatters, leaves or fetches the next path while its
-// neighbours go on.  Inside the shading kernel the same walks kept 5.8 of a
+// like k_extend: a warp advances its rays by majority steps, and a lane whose
+// ray is done scatters, leaves or fetches the next path with the others that
+// wait.  Inside the shading kernel the same walks kept 5.8 of a
 // warp's 32 lanes busy and took 102 of the 159 ms of a 20-job serving mix whose
 // largest image has such a material; with this kernel the mix takes 67 ms.
 // The outcome goes to the path's NEE slots, which shading reads before it

@@ -445,7 +445,8 @@ __global__ void __launch_bounds__(128, 1) k_conv3x3_tc(ConvArgs a, uint32_t tmem
 size_t tcSmemBytes(uint32_t cout) { return (size_t)kTcStages * (kTcRows * 128u + cout * 128u) + 1024u + 64u; }
 
 // ------------------------------------------- tcgen05 + TMA, persistent ----
-// The production convolution.  Persistent CTAs (one per SM) walk output
+// The convolution of the layers that neither the halo-row nor the tile kernel
+// below takes.  Persistent CTAs (one per SM) walk output
 // tiles of 128 pixels (th image rows x tw columns, tw a power of two <= 128)
 // with three warp roles:
 //   warp 0     TMA producer: per (tap, 64-channel chunk) one 4-D box of the
@@ -1616,14 +1617,18 @@ size_t haloSmemBytes(uint32_t cout, uint32_t chunks, bool staged, uint32_t ring,
 // input block and one {32 channels, 16, 16} per output block, zero filled
 // outside the image, then 16 K steps x 3 vertical taps of straight-line MMAs
 // per input block.  The sums stay in tensor memory over all of a CTA's tiles
-// (at most a few hundred K steps, like a chunk of a split-K sum) and are added
-// to dW once, 32 consecutive input channels per warp instruction.
+// (at most 64 to a set of accumulators, 1,024 K steps; launchWgrad) and are
+// added to dW once, 32 consecutive input channels per warp instruction.
 // Bound: shared-memory operand reads at 32 output channels (4 KB of A per MMA),
-// a fixed ~20 us of set-up and read-out at the deep levels.  Measured over the
-// 19 layers of a 16 x 256^2 training step: 689 us; an mma.sync kernel that read
-// every input pixel once per tap took 4218 us.  Error against 64 bits on those
-// gradients: 2e-7 to 1.2e-5 (tensor-core sums truncate, so it grows with a
-// CTA's K steps), below the former kernel's on every layer.
+// and 10 to 20 us of set-up and read-out, which small problems avoid
+// (k_conv3x3_wgrad_mma).  Measured over the 19 layers of a 16 x 256^2 training
+// step: 694 us, two of the layers on mma.sync; all of them there took 4218 us.
+// The tensor core truncates, so the error against 64 bits grows with the K steps
+// of a sum: 1.8e-7 to 1.2e-5 on those gradients and 2.2e-5 for 96 to 32 channels,
+// 1.8e-7 to 2.7e-5 on mma.sync, no layer above it there.
+// An infinite or NaN activation in the last column or row of an image that ends
+// inside a tile reaches all nine taps' sums of its channel, through its products
+// with the zero fill; elsewhere the taps whose pixels are in the image.
 struct WgradArgs {
     float* dw;  // [cout][9][cin], accumulated
     uint32_t cin, cout, tilesX, tilesY, numTiles;
@@ -2520,9 +2525,11 @@ int launchReluBias(const void* out, uint32_t ldo, const void* dout, uint32_t ldd
     return DK_OK;
 }
 
-// 3: halo-row TMA + tcgen05 convolution where the layer fits it, else the
-// per-tap one (default); 2: the per-tap persistent TMA + tcgen05 convolution;
-// 1: the cp.async + tcgen05 one; 0: the mma.sync one.
+// 3 (default): the halo-row TMA + tcgen05 convolution where the layer fits it,
+// else the tile kernel where it is the faster one (launchConvTile), else the
+// row-tap or per-tap one, or mma.sync above 256 output channels; 2: the per-tap
+// persistent TMA + tcgen05 convolution; 1: the cp.async + tcgen05 one; 0: the
+// mma.sync one.
 int g_convPath = 3;
 
 // Launch with programmatic stream serialization (see pdlWait); DK_PDL=0 launches
@@ -2954,11 +2961,10 @@ int launchWgradMma(const __nv_bfloat16* in, uint32_t ldi, const __nv_bfloat16* d
 // The weight gradient's launch: input blocks per CTA from the accumulator
 // columns (3 x coB per block of 32 channels) and two pipeline stages of shared
 // memory, fewer where the pixel tiles alone would leave SMs idle, two at most.
-// The tensor core truncates when it adds to an accumulator, so a gradient's low
-// digits depend on how many partial sums it is made of: with two blocks as many
-// as the kernel before this one took (76 against 68 for 96 to 32 channels), and
-// gradients that agree with its to 1e-5.  Three there, in 152 sums, took 27 us
-// less of a training step's 2.3 ms and differed by up to 3e-5.
+// With three, 96 to 32 channels on 16 x 256^2 take 106 us instead of 133, up to
+// 1 % of a training step, in twice as many sums: 9.0e-6 from 64 bits instead of
+// 2.2e-5 (mma.sync 2.7e-5), and up to 3e-5 from the gradients that both the
+// mma.sync kernel and this one have given so far.  Two keep those.
 int launchWgrad(const __nv_bfloat16* in, uint32_t ldi, const __nv_bfloat16* dout, uint32_t ldd, uint32_t n, uint32_t h,
                 uint32_t w, uint32_t cin, uint32_t cout, float* dw, cudaStream_t st) {
     if (deviceProp().multiProcessorCount == 0) ensureDevice();

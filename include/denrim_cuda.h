@@ -612,15 +612,18 @@ int dk_unet_adam_groups(const dk_unet_adam_group* groups, uint32_t group_count, 
                         float eps, uint32_t step, void* stream);
 int dk_unet_weights_to_bf16(const float* weights, uint32_t count, void* wbf16, void* wflip, uint32_t cout,
                             uint32_t cin, void* stream);
-/* Selects the convolution kernel (Cout <= 256 for the tcgen05 ones): 3
- * (default) the halo-row TMA + tcgen05 kernel for images at least 128 pixels
- * wide whose weights and input rows fit one CTA's shared memory, else 2;
- * 2 persistent per-tap TMA + tcgen05 with warp roles, 1 cp.async + tcgen05,
- * 0 mma.sync; the alternatives are kept for comparison. */
+/* Selects the convolution kernel: 3 (default) the halo-row TMA + tcgen05 kernel
+ * for images at least 128 pixels wide whose weights and input rows fit one CTA's
+ * shared memory, else the 2-D halo-tile kernel (any Cout) where an estimate of
+ * both finds it faster, else 2 with rows of 128 pixels where the image is as
+ * wide; 2 persistent per-tap TMA + tcgen05 with warp roles, 1 cp.async +
+ * tcgen05 (both Cout <= 256, else 0), 0 mma.sync; the alternatives are kept for
+ * comparison. */
 int dk_unet_set_conv_path(int path);
 /* Reads and clears the denoiser kernels' error flag (non-zero: a bounded wait
  * for the tensor cores or a copy timed out and the affected tiles were not
- * written; 1, 2, 3 name the cp.async, per-tap TMA and halo-row kernels). */
+ * written; 1 to 5 name the cp.async, per-tap TMA, halo-row, weight-gradient and
+ * tile kernels). */
 int dk_unet_error(int* out_error);
 
 /* ------------------------------------------------------------------------- */
