@@ -2993,13 +2993,13 @@ int launchWgrad(const __nv_bfloat16* in, uint32_t ldi, const __nv_bfloat16* dout
     const uint32_t groups = coBlocks * a.ciGroups;
     // The tensor core truncates when it accumulates, so a gradient's error grows with the K steps of one sum and
     // falls with the number of sums it is made of.  They are as many as the mma.sync kernel's (runs of up to 512
-    // pixels are not worth a split), a K step with fewer than 16 pixels counting for a third more than its pixels,
-    // and no sum takes more than kWgRunMax tiles.  Where one CTA per SM makes fewer, a CTA sums into two sets of
+    // pixels are not worth a split), a K step with fewer than 16 pixels counting for a third more than its pixels or
+    // as a whole one, and no sum takes more than kWgRunMax tiles.  Where one CTA per SM makes fewer, a CTA sums into two sets of
     // accumulators if they fit, and then the pixels are split further, in whole rounds of CTAs.
     const uint64_t M = (uint64_t)n * h * w;
     const float pieces = (float)M / (float)std::max(wgradMmaChunk(M, cin, cout), 512u);
-    const uint32_t sums = std::max((uint32_t)(pieces * (1.0f + 0.3f * (float)(w % kWgTile) / (float)w)),
-                                   (a.numTiles + kWgRunMax - 1u) / kWgRunMax);
+    const float ragged = std::min(1.0f + 0.3f * (float)(w % kWgTile) / (float)w, (float)(a.tilesX * kWgTile) / (float)w);
+    const uint32_t sums = std::max((uint32_t)(pieces * ragged), (a.numTiles + kWgRunMax - 1u) / kWgRunMax);
     uint32_t gx = std::max(1u, sms / groups);
     a.sets = sums > gx && 6u * a.cpc * a.coB <= 512u ? 2u : 1u;
     if (sums > gx * a.sets) {
