@@ -54,8 +54,9 @@ def relu_time(lib, c, pixels):
 
 
 def test_a_small_tensor_costs_a_launch(lib):
-    # 2.4 MB, 0.35 us of memory time: one wave of blocks, each thread one load deep, like a single pixel
-    assert relu_time(lib, 96, 4096) <= 1.4 * relu_time(lib, 96, 1)
+    # 2.4 MB, 0.35 us of memory time: one wave of blocks, each thread one load deep, like a single pixel; eight
+    # pixels a thread in two rounds of loads took twice as long
+    assert relu_time(lib, 96, 4096) <= 1.65 * relu_time(lib, 96, 1)
 
 
 def test_many_channels_go_at_the_rate_of_few(lib):
