@@ -2381,8 +2381,10 @@ struct AdamRule {
     float lr, b1, b2, eps, c1, c2;
 };
 __device__ __forceinline__ float adamStep(const AdamRule& r, float w, float g, float& m, float& v) {
-    m = r.b1 * m + (1.0f - r.b1) * g;
-    v = r.b2 * v + (1.0f - r.b2) * g * g;
+    // The new term is fused, the decayed one rounded, in both entry points: left to the compiler it was the other way
+    // round in one build, which changes the last bit of every third m and every fourth v.
+    m = __fmaf_rn(1.0f - r.b1, g, r.b1 * m);
+    v = __fmaf_rn((1.0f - r.b2) * g, g, r.b2 * v);
     return w - r.lr * (m / r.c1) / (sqrtf(v / r.c2) + r.eps);
 }
 __global__ void k_adam(float* wts, const float* grad, float* m, float* v, uint32_t count, AdamRule rule,
